@@ -268,6 +268,23 @@ def test_gemm_simt_fp32(M, N, K):
     assert torch.equal(alone[0], ops().gemm_nt_simt(a, w)[M - 1])
 
 
+@pytest.mark.parametrize("N,K,pad", [(64, 256, 0), (65, 512, 0), (130, 777, 0), (63, 1000, 3), (100, 2051, 1), (1024, 2048, 4), (40000, 300, 0)])
+def test_gemm_float32_tiles_and_parts(N, K, pad):
+    """The 32-bit product at the edges of its row tiles (4, 8, 16, 32, 64) and of the parts of k, rows that begin on 16-byte
+    addresses and rows that do not; every row the same bits however many rows the call has.  A sum's error is at most
+    (the additions that a term passes through) units of 2^-24 of the sum of the terms' sizes: half a part, the parts, two."""
+    parts = min(8, max(1, K // 256))
+    steps = -(-K // parts) // 2 + 32 + parts + 2
+    w = rnd((N, K + pad), torch.float32, 7)[:, :K]
+    a = rnd((130, K + pad), torch.float32, 6)[:, :K]
+    bias = rnd((N,), torch.float32, 8)
+    whole = ops().gemm_nt_simt(a, w, bias)
+    limit = steps * 2.0 ** -24 * (abs(f64(a)) @ abs(f64(w)).T + abs(f64(bias)))
+    assert (abs(f64(whole) - (f64(a) @ f64(w).T + f64(bias))) <= limit).all()
+    for M in (1, 3, 4, 5, 8, 9, 16, 17, 32, 33, 63, 64, 65, 129):
+        assert torch.equal(ops().gemm_nt_simt(a[130 - M:], w, bias), whole[130 - M:]), M
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,K", [(1, 53, 72), (37, 64, 16), (130, 136, 104), (64, 384, 96), (8, 4096, 4096)])
 def test_gemm_bf16(M, N, K, out_dtype):

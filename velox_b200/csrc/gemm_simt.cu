@@ -1,11 +1,12 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]): the plain matrix product.
 //
 // Multiply-adds on the CUDA cores in float32, no tensor cores, no reduced
-// precision mode: this is the matrix product of the 32-bit path, and the
-// reference against which the tensor-core products are checked.  Every output
-// element is the sum over k in ascending order, so a row's result does not
-// depend on how many rows the call has.  Any M, N, K.
+// precision mode.  float32 operands, the 32-bit path's, go to the kernel in
+// gemm_f32.cu; the kernel here takes bfloat16 ones and is the reference against
+// which the tensor-core products are checked.  The order of a sum is fixed by K alone
+// (here: ascending k), so a row's result does not depend on how many rows the call has.  Any M, N, K.
 #include "common.cuh"
+#include "gemm_f32.cuh"
 
 #define GS_BM 64
 #define GS_BN 64
@@ -83,8 +84,8 @@ extern "C" int vx_gemm_nt_simt_batched(const void* A, const void* W, const float
     dim3 grid((N + GS_BN - 1) / GS_BN, (M + GS_BM - 1) / GS_BM, batch);
     if (grid.y > 65535 || batch > 65535) return VX_ERR_LIMIT;
     if (in_dtype == VX_F32 && out_dtype == VX_F32)
-        VX_LAUNCH_K(VX_K_GEMM, (gemm_nt_simt_kernel<float, float>), grid, 256, 0, stream, (const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, sa, sw, sc);
-    else if (in_dtype == VX_BF16 && out_dtype == VX_BF16)
+        return vx_gemm_f32((const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
+    if (in_dtype == VX_BF16 && out_dtype == VX_BF16)
         VX_LAUNCH_K(VX_K_GEMM, (gemm_nt_simt_kernel<bf16, bf16>), grid, 256, 0, stream, (const bf16*)A, (const bf16*)W, bias, (bf16*)C, M, N, K, lda, ldw, ldc, sa, sw, sc);
     else if (in_dtype == VX_BF16 && out_dtype == VX_F32)
         VX_LAUNCH_K(VX_K_GEMM, (gemm_nt_simt_kernel<bf16, float>), grid, 256, 0, stream, (const bf16*)A, (const bf16*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, sa, sw, sc);

@@ -950,7 +950,8 @@ def paged_prefill_attention_tc(q: torch.Tensor, q_row_stride: int, k_pool, v_poo
 
 
 def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """a [M,K] times w [N,K] transposed, float32 multiply-adds on the CUDA cores."""
+    """a [M,K] times w [N,K] transposed, float32 multiply-adds on the CUDA cores.  `w` is a weight: not
+    something the kernel launched just before this one writes (its first tiles are fetched before the wait for that kernel)."""
     _dev(a, w, bias)
     _need(a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1], "gemm: a [M,K], w [N,K]")
     _need(a.stride(1) == 1 and w.stride(1) == 1 and a.dtype == w.dtype, "gemm: rows contiguous, one element type")
@@ -970,8 +971,8 @@ GEMM_HEADS_FEW_ROWS = 8   # rows up to which the products per head take the kern
 
 def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """One product per head: out[:, h, :] = a[:, h, :] w[h]^T with a [M, H, K], w [H, N, K] (contiguous), out [M, H, N];
-    `a` and `out` may be views into wider rows (their last dimension contiguous).  float32 multiply-adds (in float32, every
-    sum over k in ascending order whatever the number of rows; bfloat16 steps of up to 8 rows take a kernel of their own)."""
+    `a` and `out` may be views into wider rows (their last dimension contiguous).  float32 multiply-adds (in float32, the
+    order of a sum is fixed by K alone, whatever the number of rows; bfloat16 steps of up to 8 rows take a kernel of their own)."""
     _dev(a, w, out)
     _need(a.dim() == 3 and w.dim() == 3 and out.dim() == 3 and w.is_contiguous() and a.shape[1] == w.shape[0]
           and a.shape[2] == w.shape[2] and out.shape == (a.shape[0], w.shape[0], w.shape[1]), "gemm_heads: a [M,H,K], w [H,N,K], out [M,H,N]")

@@ -3,8 +3,8 @@
 
 The one place where a matrix product is chosen:
   float32   the engine's own multiply-add kernel on the CUDA cores: true 32-bit,
-            every output element summed over k in ascending order, so a row's
-            result does not depend on the rows beside it.
+            every output element summed over k in an order that K alone fixes, so a
+            row's result does not depend on the rows beside it.
   bfloat16  the tensor-core product (see `matmul`).
 """
 from __future__ import annotations
