@@ -33,8 +33,22 @@
 #define ATT_WARPS 4
 #define ATT_MAX_D 256
 
-template <typename T>
-__global__ void paged_attention_generic_kernel(
+// Four neighbouring elements with one load (16 bytes of float32, 8 of bfloat16).
+__device__ __forceinline__ float4 att_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 att_load4(const bf16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.x));
+    const float2 b = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162&>(u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// FOUR: the sizes of keys and values, the stride of a value row and the pools' addresses are multiples of four elements.  What
+// bounds this kernel is the latency of its loads: a lane fetches a key four elements at a time, eight loads ahead, into
+// four partial sums, and a value row comes as four neighbouring channels a lane, eight keys ahead (one element at a time
+// and one key at a time: 160 us for 96 prompt tokens beside 3 decoded ones on 100 to 400 keys, 16 heads of 128, float32; now 85).
+// Which form runs follows from the layer's sizes, so a position's sums have one order.
+template <typename T, bool FOUR>
+__global__ void __launch_bounds__(ATT_WARPS * 32) paged_attention_generic_kernel(
     const T* __restrict__ q, int q_row_stride, const T* __restrict__ k_pool,
     const T* __restrict__ v_pool, const int* __restrict__ block_table, int max_blocks,
     const int* __restrict__ seq_of_token, const int* __restrict__ positions, T* __restrict__ out,
@@ -43,7 +57,7 @@ __global__ void paged_attention_generic_kernel(
     int chunk) {
     pdl_wait();
     pdl_trigger();
-    __shared__ float q_s[ATT_MAX_D];
+    __shared__ __align__(16) float q_s[ATT_MAX_D];
     __shared__ float acc_s[ATT_WARPS][ATT_MAX_D];
     __shared__ float m_s[ATT_WARPS], l_s[ATT_WARPS];
 
@@ -82,7 +96,20 @@ __global__ void paged_attention_generic_kernel(
             const T* kp = k_pool + base * D;
             if (v_share > 1) base = ((size_t)page * (Hk / v_share) + hk / v_share) * S + (j % S);
             float dot = 0.f;
-            for (int d = 0; d < D; ++d) dot += q_s[d] * to_f32(kp[d]);
+            if (FOUR) {
+                float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+                for (int d = 0; d < D; d += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(q_s + d), b = att_load4(kp + d);
+                    sum.x = fmaf(a.x, b.x, sum.x);
+                    sum.y = fmaf(a.y, b.y, sum.y);
+                    sum.z = fmaf(a.z, b.z, sum.z);
+                    sum.w = fmaf(a.w, b.w, sum.w);
+                }
+                dot = (sum.x + sum.y) + (sum.z + sum.w);
+            } else {
+                for (int d = 0; d < D; ++d) dot += q_s[d] * to_f32(kp[d]);
+            }
             s = dot * scale;
             if (softcap > 0.f) s = softcap * tanhf(s / softcap);
             s -= slope * (float)(kv_len - 1 - j);
@@ -94,14 +121,32 @@ __global__ void paged_attention_generic_kernel(
 #pragma unroll
         for (int i = 0; i < NR; ++i) acc[i] *= alpha;
         const int nvalid = min(32, nkeys - c * 32);
-        for (int jj = 0; jj < nvalid; ++jj) {
-            const float pj = __shfl_sync(0xffffffffu, p, jj);
-            const size_t bj = __shfl_sync(0xffffffffu, (unsigned long long)base, jj);
-            const T* vp = v_pool + bj * v_stride;
+        if (FOUR) {
+#pragma unroll 8
+            for (int jj = 0; jj < nvalid; ++jj) {
+                const float pj = __shfl_sync(0xffffffffu, p, jj);
+                const size_t bj = __shfl_sync(0xffffffffu, (unsigned long long)base, jj);
+                const T* vp = v_pool + bj * v_stride + lane * 4;
 #pragma unroll
-            for (int i = 0; i < NR; ++i) {
-                const int d = lane + 32 * i;
-                if (d < Dv) acc[i] += pj * to_f32(vp[d]);
+                for (int r = 0; r < NR / 4; ++r) {
+                    if (lane * 4 + 128 * r >= Dv) break;
+                    const float4 v = att_load4(vp + 128 * r);
+                    acc[4 * r] = fmaf(pj, v.x, acc[4 * r]);
+                    acc[4 * r + 1] = fmaf(pj, v.y, acc[4 * r + 1]);
+                    acc[4 * r + 2] = fmaf(pj, v.z, acc[4 * r + 2]);
+                    acc[4 * r + 3] = fmaf(pj, v.w, acc[4 * r + 3]);
+                }
+            }
+        } else {
+            for (int jj = 0; jj < nvalid; ++jj) {
+                const float pj = __shfl_sync(0xffffffffu, p, jj);
+                const size_t bj = __shfl_sync(0xffffffffu, (unsigned long long)base, jj);
+                const T* vp = v_pool + bj * v_stride;
+#pragma unroll
+                for (int i = 0; i < NR; ++i) {
+                    const int d = lane + 32 * i;
+                    if (d < Dv) acc[i] += pj * to_f32(vp[d]);
+                }
             }
         }
         m = m_new;
@@ -110,7 +155,7 @@ __global__ void paged_attention_generic_kernel(
     if (lane == 0) { m_s[warp] = m; l_s[warp] = l; }
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
-        const int d = lane + 32 * i;
+        const int d = FOUR ? lane * 4 + 128 * (i >> 2) + (i & 3) : lane + 32 * i;
         if (d < Dv) acc_s[warp][d] = acc[i];
     }
     __syncthreads();
@@ -163,14 +208,20 @@ extern "C" int vx_paged_attention_generic_chunk(const void* q, int q_row_stride,
         return VX_ERR_SHAPE;
     if (window < 0 || keep_first < 0 || bias_exp < 0.f || chunk < 0 || (chunk && keep_first)) return VX_ERR_SHAPE;
     dim3 grid(tokens, H);
-    if (dtype == VX_F32)
-        VX_LAUNCH_K(VX_K_ATTENTION, (paged_attention_generic_kernel<float>), grid, ATT_WARPS * 32, 0, stream, (const float*)q, q_row_stride, (const float*)k_pool, (const float*)v_pool, block_table,
-            max_blocks, seq_of_token, positions, (float*)out, out_row_stride, scale, window, H, Hk, D, S, Dv, keep_first, bias_exp, sinks, gate_col, softcap, v_stride, v_share, out_f32, chunk);
-    else if (dtype == VX_BF16)
-        VX_LAUNCH_K(VX_K_ATTENTION, (paged_attention_generic_kernel<bf16>), grid, ATT_WARPS * 32, 0, stream, (const bf16*)q, q_row_stride, (const bf16*)k_pool, (const bf16*)v_pool, block_table,
-            max_blocks, seq_of_token, positions, (bf16*)out, out_row_stride, scale, window, H, Hk, D, S, Dv, keep_first, bias_exp, sinks, gate_col, softcap, v_stride, v_share, out_f32, chunk);
-    else
-        return VX_ERR_DTYPE;
+    if (dtype != VX_F32 && dtype != VX_BF16) return VX_ERR_DTYPE;
+    const bool four = !((D | Dv | v_stride) & 3) && !((((uintptr_t)k_pool) | ((uintptr_t)v_pool)) & (dtype == VX_F32 ? 15 : 7));
+#define ATT_GO(T, F)                                                                                                                 \
+    VX_LAUNCH_K(VX_K_ATTENTION, (paged_attention_generic_kernel<T, F>), grid, ATT_WARPS * 32, 0, stream, (const T*)q, q_row_stride,  \
+                (const T*)k_pool, (const T*)v_pool, block_table, max_blocks, seq_of_token, positions, (T*)out, out_row_stride, scale, \
+                window, H, Hk, D, S, Dv, keep_first, bias_exp, sinks, gate_col, softcap, v_stride, v_share, out_f32, chunk)
+    if (dtype == VX_F32) {
+        if (four) ATT_GO(float, true);
+        else ATT_GO(float, false);
+    } else {
+        if (four) ATT_GO(bf16, true);
+        else ATT_GO(bf16, false);
+    }
+#undef ATT_GO
     VX_LAUNCH_CHECK();
     return VX_OK;
 }
