@@ -421,6 +421,34 @@ def test_decode_attention_gives_the_same_bits_in_every_block_shape():
         assert torch.equal(part[:n], full[:n]), n
 
 
+@pytest.mark.parametrize("D,H,Hk,window,S", [(128, 8, 2, 0, 16), (128, 24, 2, 0, 32), (64, 6, 6, 300, 16), (64, 32, 2, 0, 48)])
+def test_decode_attention_forms_agree(D, H, Hk, window, S):
+    """A block or a warp per piece: the same bits, at lengths around the edges of a tile (16 keys), a sub-piece (32), the
+    ring (64) and a piece (256), with one and two tiles of 8 query heads."""
+    lens = [1, 16, 17, 32, 33, 64, 65, 96, 97, 224, 255, 256, 257, 289, 513, 800]
+    q, kp, vp, bt, sot, pos, want = paged_case(torch.bfloat16, [(n - 1, 1) for n in lens], H, Hk, D, S, window, seed=17)
+    run = lambda shape: ops().paged_decode_attention(q, H * D, kp, vp, bt, sot, pos, 1 / math.sqrt(D), window, H, Hk, D, len(lens),
+                                                     max(lens), shape=shape)
+    first = run(0)
+    close(first, want, torch.bfloat16)
+    for shape in (1, 8):
+        assert torch.equal(run(shape), first), shape
+
+
+def test_decode_attention_shows_a_score_that_is_no_number():
+    """A query that is not a number gives an output that is none, whatever the number of keys; its neighbours keep theirs."""
+    H, Hk, D, S = 8, 2, 128, 16
+    lens = [1, 33, 257, 700]
+    q, kp, vp, bt, sot, pos, _ = paged_case(torch.bfloat16, [(n - 1, 1) for n in lens], H, Hk, D, S, 0, seed=18)
+    good = ops().paged_decode_attention(q, H * D, kp, vp, bt, sot, pos, 0.1, 0, H, Hk, D, 4, 700)
+    q2 = q.clone()
+    q2.view(4, H, D)[:, 3, 5] = float("nan")
+    got = ops().paged_decode_attention(q2, H * D, kp, vp, bt, sot, pos, 0.1, 0, H, Hk, D, 4, 700).view(4, H, D)
+    assert torch.isnan(got[:, 3]).all()
+    rest = [h for h in range(H) if h != 3]
+    assert torch.equal(got[:, rest], good.view(4, H, D)[:, rest])
+
+
 def test_decode_attention_refuses_what_it_cannot_do():
     from velox_b200.csrc.ops import KernelError
     q, kp, vp, bt, sot, pos, _ = paged_case(torch.bfloat16, [(9, 1)], 4, 2, 48, 16, 0, seed=14)

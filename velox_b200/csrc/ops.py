@@ -96,6 +96,7 @@ def _declare(lib) -> None:
         "vx_paged_prefill_attention_tc_ext": [P, I, I, P, P, I, P, I, P, P, P, P, I, F, I, I, I, I, I, I, I, P, I, P, P, I, P],
         "vx_paged_prefill_attention": [P, I, P, P, P, I, P, P, P, P, I, F, I, I, I, I, I, I, I, P],
         "vx_paged_decode_attention": [P, I, P, P, P, I, P, P, P, P, I, P, I, F, I, I, I, I, I, I, I, I, P],
+        "vx_paged_decode_attention_shape": [P, I, P, P, P, I, P, P, P, P, I, P, I, F, I, I, I, I, I, I, I, I, I, P],
         "vx_sample": [P, I, I, I, P, P, P, P, P],
         "vx_qk_norm_rope_kv_pairs": [P, I, P, P, F, P, I, P, P, P, P, I, I, I, I, I, I, I, I, P],
         "vx_paged_attention_generic_cap": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, P],
@@ -845,13 +846,13 @@ def paged_decode_attention(q: torch.Tensor, q_row_stride: int, k_pool, v_pool, b
                            seq_of_token, positions, scale: float, window: int, num_heads: int, num_kv_heads: int,
                            head_dim: int, requests: int, max_kv: int, token_rows=None,
                            out: Optional[torch.Tensor] = None, out_rows: Optional[int] = None,
-                           single_tokens: bool = True) -> torch.Tensor:
+                           single_tokens: bool = True, shape: int = 0) -> torch.Tensor:
     """Attention of one query token per entry over its request's pages (bfloat16), the
     key range split over blocks of DECODE_CHUNK_TILES * 16 keys.  `max_kv` bounds
     every entry's number of keys (it sizes the grid and the scratch).  `token_rows`
     picks the entries' rows; `single_tokens=False` says that some of them are tokens of
     one request's portion (the kernel then waits for the step's cache writes before it
-    reads any key)."""
+    reads any key).  `shape` names the kernel's form (for measurements and tests; 0: the sizes choose)."""
     _dev(q, k_pool, v_pool, block_table, seq_of_token, positions, token_rows)
     _need(q.dtype == torch.bfloat16 and k_pool.dtype == torch.bfloat16 and v_pool.dtype == torch.bfloat16,
           "paged_decode_attention: bfloat16 only")
@@ -865,11 +866,11 @@ def paged_decode_attention(q: torch.Tensor, q_row_stride: int, k_pool, v_pool, b
     scratch = None
     if max_splits > 1:
         scratch = workspace(q.device, requests * num_heads * max_splits * (head_dim + 2))
-    _check(library().vx_paged_decode_attention(
+    _check(library().vx_paged_decode_attention_shape(
         _ptr(q), q_row_stride, _ptr(k_pool), _ptr(v_pool), _ptr(block_table), block_table.shape[1],
         _ptr(token_rows), _ptr(seq_of_token), _ptr(positions), _ptr(scratch), max_splits, _ptr(out),
         num_heads * head_dim, float(scale), int(window), requests, num_heads, num_kv_heads, head_dim,
-        k_pool.shape[2], DECODE_CHUNK_TILES, 1 if single_tokens else 0, _stream()), "paged_decode_attention")
+        k_pool.shape[2], DECODE_CHUNK_TILES, 1 if single_tokens else 0, int(shape), _stream()), "paged_decode_attention")
     return out
 
 
