@@ -1,6 +1,6 @@
 // Token sampling from float32 logits: greedy, temperature, temperature + top-p.
 //
-// One block per row.  For row r with temperature T, nucleus mass P and a
+// A cluster of one to eight blocks per row, as many as the rows leave SMs for.  For row r with temperature T, nucleus mass P and a
 // uniform number u in [0,1) that the host drew for this (request, step):
 //   T <= 1e-7:  the argmax, the lowest index winning ties.
 //   otherwise:  e_i = 2^((x_i - max) log2(e) / T);  with 0 < P < 1 only the most
@@ -9,7 +9,10 @@
 //               float t whose mass {e >= t} still reaches P times the whole;  the token
 //               is the first index, in index order, whose cumulative kept mass
 //               exceeds u times the kept total.
-// Every pass over the row reads it with consecutive lanes on consecutive elements.
+// Each block reads its part of the row once, all loads in flight together, and keeps it in shared memory (where it fits) when it
+// is needed again; maxima, histograms and masses are put together through the cluster's shared memory, where every block
+// reads all eight and comes to the same conclusion by itself.  One block per row had one SM pull the whole row from L2 five
+// times: 20 rows of 151,936 took 91 us by nucleus, 8 greedy rows SAMP_OLD us; now SAMP_NEW and SAMP_NEW2.
 // The threshold t is found ten bits a pass: a histogram, over the next ten bits of
 // the patterns of e (positive floats order like their patterns), of the mass in each
 // bin, as exact integers so that the order of the additions does not matter, then a
@@ -18,12 +21,15 @@
 // bit, one pass a bit, took 1.1 ms a row at a vocabulary of 151,936.)
 // The same logits and u give the same token on every run.
 #include "common.cuh"
+#include <cooperative_groups.h>
 #include <limits.h>
+
+namespace cg = cooperative_groups;
 
 #define SAMPLE_THREADS 1024
 #define SAMPLE_WARPS (SAMPLE_THREADS / 32)
 #define SAMPLE_BINS 1024
-#define SAMPLE_GROUPS 256  // groups of 32 elements per warp: rows of up to 2^18 elements
+#define SAMPLE_GROUPS 256  // groups of 32 elements per stretch: rows of up to 2^18 elements
 static_assert(SAMPLE_BINS == SAMPLE_THREADS, "the scan below gives every thread one bin");
 
 __device__ __forceinline__ float sample_ex2(float x) {
@@ -32,17 +38,15 @@ __device__ __forceinline__ float sample_ex2(float x) {
     return y;
 }
 
-// f(index, value) for every element of the row, each thread its share in ascending
-// index order.  Sixteen elements a thread are asked for before the first is used
-// (four 16-byte loads when the row allows it): one SM has to pull the whole row, and
-// with one load in flight per thread a pass over 151,936 logits took 43 us.
+// f(index, value) for elements [i0, i1) of the row, each thread its share in ascending index order (i0 a multiple of 4).
+// Sixteen elements a thread are asked for before the first is used (four 16-byte loads when the row allows it).
 template <typename F>
-__device__ __forceinline__ void row_for_each(const float* __restrict__ x, int V, F f) {
+__device__ __forceinline__ void row_for_each(const float* __restrict__ x, int i0, int i1, F f) {
     const int tid = threadIdx.x;
     if ((((uintptr_t)x) & 15) == 0) {
-        const int n4 = V >> 2;
+        const int n4 = i1 >> 2;
         const float4* x4 = reinterpret_cast<const float4*>(x);
-        for (int j0 = tid; j0 < n4; j0 += SAMPLE_THREADS * 4) {
+        for (int j0 = (i0 >> 2) + tid; j0 < n4; j0 += SAMPLE_THREADS * 4) {
             float4 v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -60,19 +64,19 @@ __device__ __forceinline__ void row_for_each(const float* __restrict__ x, int V,
                 }
             }
         }
-        for (int i = (n4 << 2) + tid; i < V; i += SAMPLE_THREADS) f(i, x[i]);
+        for (int i = max(n4 << 2, i0) + tid; i < i1; i += SAMPLE_THREADS) f(i, x[i]);
     } else {
-        for (int i0 = tid; i0 < V; i0 += SAMPLE_THREADS * 4) {
+        for (int j0 = i0 + tid; j0 < i1; j0 += SAMPLE_THREADS * 4) {
             float v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int i = i0 + u * SAMPLE_THREADS;
-                if (i < V) v[u] = x[i];
+                const int i = j0 + u * SAMPLE_THREADS;
+                if (i < i1) v[u] = x[i];
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int i = i0 + u * SAMPLE_THREADS;
-                if (i < V) f(i, v[u]);
+                const int i = j0 + u * SAMPLE_THREADS;
+                if (i < i1) f(i, v[u]);
             }
         }
     }
@@ -122,31 +126,65 @@ __device__ __forceinline__ int block_min_int(int v, int* si) {
     return v;
 }
 
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// BLOCKS: blocks of a row's cluster, each with 32 / BLOCKS stretches that are dealt to as many warps as there are blocks.
+// KEPT: the block keeps its part of the row in shared memory; otherwise later passes read it from memory again.
+template <int BLOCKS, typename T>
+__device__ __forceinline__ T* sample_at(cg::cluster_group& cluster, T* p, int block) {
+    return BLOCKS > 1 ? cluster.map_shared_rank(p, block) : p;
+}
+
+template <int BLOCKS, bool KEPT>
+__global__ void __cluster_dims__(BLOCKS, 1, 1) __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
               const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
     pdl_wait();
     pdl_trigger();
+    constexpr int STRETCHES = SAMPLE_WARPS / BLOCKS, BUFFERS = BLOCKS > 1 ? 2 : 1;
+    extern __shared__ float slice_s[];
     __shared__ float sv[32];
     __shared__ int si[32];
-    __shared__ unsigned hist_lo[SAMPLE_BINS], hist_hi[SAMPLE_BINS];
+    __shared__ unsigned hist_lo[BUFFERS][SAMPLE_BINS], hist_hi[BUFFERS][SAMPLE_BINS];
     __shared__ unsigned long long warp_total[SAMPLE_WARPS];
     __shared__ unsigned long long above_s;
     __shared__ int first_s;
-    __shared__ float warp_mass[SAMPLE_WARPS];
-    __shared__ float group_mass[SAMPLE_WARPS][SAMPLE_GROUPS];
-    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ float stretch_mass[STRETCHES];
+    __shared__ float group_mass[STRETCHES][SAMPLE_GROUPS];
+    __shared__ float best_of[BLOCKS];
+    __shared__ int best_i_of[BLOCKS], cand_of[BLOCKS], last_of[BLOCKS];
+    cg::cluster_group cluster = cg::this_cluster();
+    // (a row of one block: plain barriers, its own shared memory)
+    auto sync = [&]() { if (BLOCKS > 1) cluster.sync(); else __syncthreads(); };
+    const int rank = BLOCKS > 1 ? (int)cluster.block_rank() : 0;
+    const int r = blockIdx.x / BLOCKS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* x = logits + (size_t)r * ld;
+    // The row is cut into 32 stretches of `groups` groups of 32 elements; a block has four of them.
+    const int groups = ((V + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) >> 5;   // at most SAMPLE_GROUPS
+    const int b0 = min(rank * STRETCHES * groups * 32, V), b1 = min((rank + 1) * STRETCHES * groups * 32, V);
 
+    const float temp = temperature ? temperature[r] : 0.f;
+    const bool greedy = !(temp > 1e-7f);
     float best = -INFINITY;
     int best_i = INT_MAX;
-    row_for_each(x, V, [&](int i, float v) {
+    row_for_each(x, b0, b1, [&](int i, float v) {
         if (v > best) { best = v; best_i = i; }  // ascending i: the first maximum stays
+        if (KEPT && !greedy) slice_s[i - b0] = v;
     });
+    const float* slice = KEPT ? slice_s : x + b0;   // the block's part of the row
     block_argmax(best, best_i, sv, si);
-    const float temp = temperature ? temperature[r] : 0.f;
-    if (!(temp > 1e-7f)) {
-        if (tid == 0) out[r] = best_i;
+    if (BLOCKS > 1) {
+        if (tid < BLOCKS) {   // every block gets every block's
+            sample_at<BLOCKS>(cluster, best_of, tid)[rank] = best;
+            sample_at<BLOCKS>(cluster, best_i_of, tid)[rank] = best_i;
+        }
+        sync();
+        best = best_of[0];
+        best_i = best_i_of[0];
+#pragma unroll
+        for (int b = 1; b < BLOCKS; ++b)   // (ascending index order)
+            if (best_of[b] > best || (best_of[b] == best && best_i_of[b] < best_i)) { best = best_of[b]; best_i = best_i_of[b]; }
+    }
+    if (greedy) {   // (nobody reaches into another block's shared memory any more)
+        if (rank == 0 && tid == 0) out[r] = best_i;
         return;
     }
     const float k = 1.4426950408889634f / temp;  // e_i = 2^((x_i - max) k)
@@ -158,29 +196,42 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
         unsigned prefix = 0u;             // the bits of the threshold's pattern found so far
         unsigned long long above = 0ull;  // mass of the patterns above the bins still in question
         unsigned long long target = 0ull;
-        for (int shift = 20; shift >= 0; shift -= 10) {
-            hist_lo[tid] = 0u;
-            hist_hi[tid] = 0u;
+        int buf = 0;
+        for (int shift = 20; shift >= 0; shift -= 10, buf ^= BUFFERS - 1) {
+            // (a histogram is cleared two passes after it was read; the cluster barrier in between orders the two)
+            hist_lo[buf][tid] = 0u;
+            hist_hi[buf][tid] = 0u;
             if (tid == 0) first_s = SAMPLE_THREADS;
             __syncthreads();
             // All elements of a bin have the same exponent, so a bin's mass is the sum of
             // their 24-bit mantissas times a power of two; the mantissas' low and high 12
             // bits are summed apart, each sum below 2^30 (64-bit atomics in shared memory
-            // are a compare-and-swap loop: the same pass took 70 us with them, 18 us so).
-            row_for_each(x, V, [&](int, float v) {
+            // are a compare-and-swap loop).
+            auto count = [&](int, float v) {
                 const unsigned pat = __float_as_uint(sample_ex2((v - xmax) * k));
                 if (pat != 0u && (pat >> (shift + 10)) == prefix) {
                     const unsigned bin = (pat >> shift) & (SAMPLE_BINS - 1);
                     const unsigned m = (pat & 0x7FFFFFu) | 0x800000u;
-                    atomicAdd(&hist_lo[bin], m & 0xFFFu);
-                    atomicAdd(&hist_hi[bin], m >> 12);
+                    atomicAdd(&hist_lo[buf][bin], m & 0xFFFu);
+                    atomicAdd(&hist_hi[buf][bin], m >> 12);
                 }
-            });
-            __syncthreads();
+            };
+            if (KEPT) {
+                for (int i = tid; i < b1 - b0; i += SAMPLE_THREADS) count(i, slice[i]);
+            } else {
+                row_for_each(x, b0, b1, count);
+            }
+            sync();
             // thread t looks at bin 1023 - t: its mass in fixed point (2^40 for 1.0) ...
             const unsigned bin_of_thread = SAMPLE_BINS - 1 - tid;
             const int exponent = (int)(((((prefix << 10) | bin_of_thread) << shift) >> 23) & 0xFFu);
-            unsigned long long s = ((unsigned long long)hist_hi[bin_of_thread] << 12) + hist_lo[bin_of_thread];
+            unsigned lo = 0u, hi = 0u;
+#pragma unroll
+            for (int b = 0; b < BLOCKS; ++b) {
+                lo += sample_at<BLOCKS>(cluster, hist_lo[buf], b)[bin_of_thread];
+                hi += sample_at<BLOCKS>(cluster, hist_hi[buf], b)[bin_of_thread];
+            }
+            unsigned long long s = ((unsigned long long)hi << 12) + lo;
             s = exponent >= 110 ? s << (exponent - 110) : (110 - exponent < 64 ? s >> (110 - exponent) : 0ull);
             // ... and with it the mass of all bins above it
 #pragma unroll
@@ -211,48 +262,52 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
         threshold = __uint_as_float(prefix);
     }
 
-    // Kept mass, then the token.  The warps' stretches of the row follow each other in index
-    // order; a stretch is walked in groups of 32 consecutive elements, one a lane, and the
-    // kept mass of every group is noted, so that the walk for the token only has to look
-    // at the groups' masses and then at one group.
-    const int groups = ((V + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) >> 5;   // per warp; at most SAMPLE_GROUPS
-    const int w0 = min(warp * groups * 32, V), w1 = min(w0 + groups * 32, V);
-    float* gm = group_mass[warp];
+    // Kept mass, then the token.  The stretches of the row follow each other in index order; a stretch is walked in groups of
+    // 32 consecutive elements, one a lane, and the kept mass of every group is noted, so that the walk for the token only
+    // has to look at the groups' masses and then at one group.
+    const int mine_s = warp / BLOCKS;   // the warp's stretch of the block's
+    const int w0 = mine_s * groups * 32;       // (counted from b0)
+    float* gm = group_mass[mine_s];
     int last_kept = -1;
-    for (int g0 = 0; g0 < groups; g0 += 4) {
+    __syncthreads();   // (the slice is whole)
+    for (int g0 = warp % BLOCKS; g0 < groups; g0 += 4 * BLOCKS) {
         float xv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int i = w0 + (g0 + u) * 32 + lane;
-            xv[u] = (g0 + u < groups && i < w1) ? x[i] : -INFINITY;
+            const int g = g0 + u * BLOCKS, i = w0 + g * 32 + lane;
+            xv[u] = g < groups && b0 + i < b1 ? slice[i] : -INFINITY;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            if (g0 + u >= groups) break;
+            const int g = g0 + u * BLOCKS;
+            if (g >= groups) break;
             float e = sample_ex2((xv[u] - xmax) * k);   // (nothing there: 2^-inf = 0)
             if (!(e >= threshold) || xv[u] == -INFINITY) e = 0.f;
             const unsigned kept = __ballot_sync(0xffffffffu, e > 0.f);
-            if (kept) last_kept = w0 + (g0 + u) * 32 + 31 - __clz(kept);
+            if (kept) last_kept = b0 + w0 + g * 32 + 31 - __clz(kept);
             const float incl = warp_scan(e, lane);
-            if (lane == 31) gm[g0 + u] = incl;
+            if (lane == 31) gm[g] = incl;
         }
     }
-    __syncwarp();
+    const int last_neg = block_min_int(last_kept >= 0 ? -last_kept : INT_MAX, si);   // (its barriers make the masses visible)
+    const bool leads = warp % BLOCKS == 0;   // one warp of every stretch goes on
     float mine = 0.f;   // the groups' masses added up in group order
-    for (int c = 0; c < groups; c += 32) mine += __shfl_sync(0xffffffffu, warp_scan(c + lane < groups ? gm[c + lane] : 0.f, lane), 31);
-    __syncthreads();
-    if (lane == 0) warp_mass[warp] = mine;
-    __syncthreads();
+    if (leads) {
+        for (int c = 0; c < groups; c += 32) mine += __shfl_sync(0xffffffffu, warp_scan(c + lane < groups ? gm[c + lane] : 0.f, lane), 31);
+        if (lane == 0) stretch_mass[mine_s] = mine;
+    }
+    sync();
     float excl = 0.f, total = 0.f;
-    for (int w = 0; w < SAMPLE_WARPS; ++w) {  // in warp order, the same in every thread
-        if (w == warp) excl = total;
-        total += warp_mass[w];
+    const int stretch = rank * STRETCHES + mine_s;
+    for (int w = 0; w < SAMPLE_WARPS; ++w) {  // in index order, the same in every thread
+        if (w == stretch) excl = total;
+        total += sample_at<BLOCKS>(cluster, stretch_mass, w / STRETCHES)[w % STRETCHES];
     }
     const float target = uniform[r] * total;
 
     int cand = INT_MAX;
-    if (excl + mine > target) {
-        // the token lies in this warp's stretch or before it: the first group whose mass crosses ...
+    if (leads && excl + mine > target) {
+        // the token lies in this stretch or before it: the first group whose mass crosses ...
         float run = excl;
         int group = -1;
         for (int c = 0; c < groups && group < 0; c += 32) {
@@ -271,21 +326,51 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
             // ... and in it the first kept element with which the mass crosses
             const int i = w0 + group * 32 + lane;
             float e = 0.f;
-            if (i < w1) {
-                e = sample_ex2((x[i] - xmax) * k);
+            if (b0 + i < b1) {
+                e = sample_ex2((slice[i] - xmax) * k);
                 if (!(e >= threshold)) e = 0.f;
             }
             const float incl = warp_scan(e, lane);
             const unsigned hit = __ballot_sync(0xffffffffu, e > 0.f && run + incl > target);
-            if (hit) cand = w0 + group * 32 + __ffs(hit) - 1;
+            if (hit) cand = b0 + w0 + group * 32 + __ffs(hit) - 1;
         }
     }
     cand = block_min_int(cand, si);
-    if (cand == INT_MAX) {  // rounding left nobody above the target: the last kept token
-        const int neg = block_min_int(last_kept >= 0 ? -last_kept : INT_MAX, si);
-        cand = neg == INT_MAX ? best_i : -neg;
+    if (tid == 0) {
+        sample_at<BLOCKS>(cluster, cand_of, 0)[rank] = cand;
+        sample_at<BLOCKS>(cluster, last_of, 0)[rank] = last_neg;
     }
-    if (tid == 0) out[r] = cand;
+    sync();
+    if (rank != 0 || tid != 0) return;
+    int neg = last_of[0];
+    cand = cand_of[0];
+    for (int b = 1; b < BLOCKS; ++b) {
+        cand = min(cand, cand_of[b]);
+        neg = min(neg, last_of[b]);
+    }
+    // rounding left nobody above the target: the last kept token
+    out[r] = cand != INT_MAX ? cand : (neg == INT_MAX ? best_i : -neg);
+}
+
+#define SAMPLE_PART_MAX (160 * 1024)   // most bytes of a row that a block keeps
+#define SAMPLE_PART_MIN 12288          // fewest elements worth a block: below, the cluster's barriers cost more than the pass (301 elements: 9.8 us in one block, 18 in eight)
+static int sample_sm_count() {
+    static int sms[VX_MAX_DEVICES];
+    return vx_sm_count(sms);
+}
+// All forms at the first call on a device: a later call may come from inside a stream capture.
+static int configure_sample() {
+    static bool configured[VX_MAX_DEVICES];
+    const int dev = vx_current_device();
+    if (dev < 0) return VX_ERR_LIMIT;
+    if (configured[dev]) return VX_OK;
+    cudaError_t e = cudaFuncSetAttribute(sample_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
+    if (e != cudaSuccess) return (int)e;
+    configured[dev] = true;
+    return VX_OK;
 }
 
 extern "C" int vx_sample(const float* logits, int ld, int rows, int vocab, const float* temperature,
@@ -294,7 +379,29 @@ extern "C" int vx_sample(const float* logits, int ld, int rows, int vocab, const
     if (vocab <= 0 || ld < vocab) return VX_ERR_SHAPE;
     if (vocab > (1 << 18)) return VX_ERR_LIMIT;  // the fixed-point mass of a row has to fit 64 bits
     if (temperature && !uniform) return VX_ERR_SHAPE;
-    VX_LAUNCH_K(VX_K_SAMPLE, (sample_kernel), rows, SAMPLE_THREADS, 0, stream, logits, ld, vocab, temperature, top_p, uniform, out);
+    // As many blocks a row as the rows leave SMs for (a block fills an SM's registers; clusters beyond one round cost more
+    // than their blocks save: 64 rows greedy 6.7 us with one block each, 16 with eight), and the row's parts in shared memory where they fit.
+    const int sms = sample_sm_count();
+    int blocks = 8ll * rows <= sms ? 8 : 4ll * rows <= sms ? 4 : 2ll * rows <= sms ? 2 : 1;
+    while (blocks > 1 && vocab / blocks < SAMPLE_PART_MIN) blocks /= 2;
+    const size_t groups = ((vocab + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) >> 5;   // (as in the kernel)
+    const size_t part = temperature ? SAMPLE_WARPS / blocks * groups * 32 * sizeof(float) : 0;
+#define SAMPLE_GO(BLOCKS, KEPT)                                                                                       \
+    VX_LAUNCH_K(VX_K_SAMPLE, (sample_kernel<BLOCKS, KEPT>), rows * BLOCKS, SAMPLE_THREADS, KEPT ? part : 0, stream, logits, ld, vocab, \
+                temperature, top_p, uniform, out)
+    const int rc = configure_sample();
+    if (rc != VX_OK) return rc;
+    if (part <= SAMPLE_PART_MAX) {
+        if (blocks == 8) SAMPLE_GO(8, true);
+        else if (blocks == 4) SAMPLE_GO(4, true);
+        else if (blocks == 2) SAMPLE_GO(2, true);
+        else SAMPLE_GO(1, true);
+    } else {   // (never with eight blocks: 2^18 / 8 elements fit)
+        if (blocks == 4) SAMPLE_GO(4, false);
+        else if (blocks == 2) SAMPLE_GO(2, false);
+        else SAMPLE_GO(1, false);
+    }
+#undef SAMPLE_GO
     VX_LAUNCH_CHECK();
     return VX_OK;
 }
