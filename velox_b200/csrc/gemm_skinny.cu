@@ -7,7 +7,7 @@
 // with a gated epilogue, 8 gate rows and their 8 up rows) and the whole of K; its
 // warps take the 32-wide k chunks in turn (chunk c goes to warp c mod the number of warps), each
 // thread loading 16 contiguous bytes of two W rows per chunk straight from global
-// memory into registers, four chunks in flight, with no shared memory on the way:
+// memory into registers, a batch of chunks in flight, with no shared memory on the way:
 // every byte of W is used exactly once.  The first chunks are asked for before the
 // wait on earlier kernels (programmatic dependent launch): weights depend on
 // nothing, so they stream while the previous kernel finishes.  x is read through
@@ -45,7 +45,9 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], unsigned a0, unsig
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <bool GATED, bool SEG, typename TOut, int SK_WARPS, int SK_UNROLL, int MIN_BLOCKS>
+// TAIL: a warp's chunks need not be whole batches of SK_UNROLL.  (The loop that allows for it is up to 10 % slower where they
+// are: 24576 x 4096 gated, 8 rows, 32.0 and 35.5 us.)
+template <bool GATED, bool SEG, typename TOut, int SK_WARPS, int SK_UNROLL, int MIN_BLOCKS, bool TAIL>
 __global__ void __launch_bounds__(SK_WARPS * 32, MIN_BLOCKS)
 gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, const float* __restrict__ bias,
                    TOut* __restrict__ out, int M, int N, int K, int ldx, int ldw, int ldo, int act, int R, int seg_rows,
@@ -88,44 +90,90 @@ gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, const
     const int nchunks = K >> 5;
     int c = warp;
     uint4 a[SK_UNROLL], b[SK_UNROLL];
-    bool loaded = false;
-    if (c + (SK_UNROLL - 1) * SK_WARPS < nchunks) {
-#pragma unroll
-        for (int u = 0; u < SK_UNROLL; ++u) {
-            const int k = (c + u * SK_WARPS) << 5;
-            a[u] = va ? ld_stream16(wa + k) : zero4;
-            b[u] = vb ? ld_stream16(wb + k) : zero4;
-        }
-        loaded = true;
-    }
-    pdl_wait();
-    pdl_trigger();
-    for (; c + (SK_UNROLL - 1) * SK_WARPS < nchunks; c += SK_UNROLL * SK_WARPS) {
-        if (!loaded) {
+    if (!TAIL) {
+        bool loaded = false;
+        if (c + (SK_UNROLL - 1) * SK_WARPS < nchunks) {
 #pragma unroll
             for (int u = 0; u < SK_UNROLL; ++u) {
                 const int k = (c + u * SK_WARPS) << 5;
                 a[u] = va ? ld_stream16(wa + k) : zero4;
                 b[u] = vb ? ld_stream16(wb + k) : zero4;
             }
+            loaded = true;
         }
-        loaded = false;
-        uint4 xv[SK_UNROLL];
+        pdl_wait();
+        pdl_trigger();
+        for (; c + (SK_UNROLL - 1) * SK_WARPS < nchunks; c += SK_UNROLL * SK_WARPS) {
+            if (!loaded) {
 #pragma unroll
-        for (int u = 0; u < SK_UNROLL; ++u)
-            xv[u] = xok ? *reinterpret_cast<const uint4*>(xr + ((c + u * SK_WARPS) << 5)) : make_uint4(0, 0, 0, 0);
+                for (int u = 0; u < SK_UNROLL; ++u) {
+                    const int k = (c + u * SK_WARPS) << 5;
+                    a[u] = va ? ld_stream16(wa + k) : zero4;
+                    b[u] = vb ? ld_stream16(wb + k) : zero4;
+                }
+            }
+            loaded = false;
+            uint4 xv[SK_UNROLL];
 #pragma unroll
-        for (int u = 0; u < SK_UNROLL; ++u) {
-            mma_bf16_16816(acc, a[u].x, b[u].x, a[u].y, b[u].y, xv[u].x, xv[u].y);
-            mma_bf16_16816(acc, a[u].z, b[u].z, a[u].w, b[u].w, xv[u].z, xv[u].w);
+            for (int u = 0; u < SK_UNROLL; ++u)
+                xv[u] = xok ? *reinterpret_cast<const uint4*>(xr + ((c + u * SK_WARPS) << 5)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < SK_UNROLL; ++u) {
+                mma_bf16_16816(acc, a[u].x, b[u].x, a[u].y, b[u].y, xv[u].x, xv[u].y);
+                mma_bf16_16816(acc, a[u].z, b[u].z, a[u].w, b[u].w, xv[u].z, xv[u].w);
+            }
         }
-    }
-    for (; c < nchunks; c += SK_WARPS) {
-        const int k = c << 5;
-        const uint4 ta = va ? ld_stream16(wa + k) : zero4, tb = vb ? ld_stream16(wb + k) : zero4;
-        const uint4 xv = xok ? *reinterpret_cast<const uint4*>(xr + k) : make_uint4(0, 0, 0, 0);
-        mma_bf16_16816(acc, ta.x, tb.x, ta.y, tb.y, xv.x, xv.y);
-        mma_bf16_16816(acc, ta.z, tb.z, ta.w, tb.w, xv.z, xv.w);
+    } else {
+        // The warp's chunks come in batches of SK_UNROLL, whole ones and then what is left: all loads of a batch are on their
+        // way before the first is used (which chunks there are is the same for the whole warp).
+        auto ask = [&]() {
+            if (c + (SK_UNROLL - 1) * SK_WARPS < nchunks) {
+#pragma unroll
+                for (int u = 0; u < SK_UNROLL; ++u) {
+                    const int k = (c + u * SK_WARPS) << 5;
+                    a[u] = va ? ld_stream16(wa + k) : zero4;
+                    b[u] = vb ? ld_stream16(wb + k) : zero4;
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < SK_UNROLL - 1; ++u) {
+                    const int k = (c + u * SK_WARPS) << 5;
+                    if (c + u * SK_WARPS < nchunks) {
+                        a[u] = va ? ld_stream16(wa + k) : zero4;
+                        b[u] = vb ? ld_stream16(wb + k) : zero4;
+                    }
+                }
+            }
+        };
+        ask();
+        pdl_wait();
+        pdl_trigger();
+        for (; c + (SK_UNROLL - 1) * SK_WARPS < nchunks;) {
+            uint4 xv[SK_UNROLL];
+#pragma unroll
+            for (int u = 0; u < SK_UNROLL; ++u)
+                xv[u] = xok ? *reinterpret_cast<const uint4*>(xr + ((c + u * SK_WARPS) << 5)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < SK_UNROLL; ++u) {
+                mma_bf16_16816(acc, a[u].x, b[u].x, a[u].y, b[u].y, xv[u].x, xv[u].y);
+                mma_bf16_16816(acc, a[u].z, b[u].z, a[u].w, b[u].w, xv[u].z, xv[u].w);
+            }
+            c += SK_UNROLL * SK_WARPS;
+            ask();
+        }
+        if (c < nchunks) {
+            uint4 xv[SK_UNROLL];
+#pragma unroll
+            for (int u = 0; u < SK_UNROLL - 1; ++u)
+                if (c + u * SK_WARPS < nchunks)
+                    xv[u] = xok ? *reinterpret_cast<const uint4*>(xr + ((c + u * SK_WARPS) << 5)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < SK_UNROLL - 1; ++u)
+                if (c + u * SK_WARPS < nchunks) {
+                    mma_bf16_16816(acc, a[u].x, b[u].x, a[u].y, b[u].y, xv[u].x, xv[u].y);
+                    mma_bf16_16816(acc, a[u].z, b[u].z, a[u].w, b[u].w, xv[u].z, xv[u].w);
+                }
+        }
     }
     // thread holds out^T[row g (c0,c1) and g+8 (c2,c3)][x rows 2t, 2t+1]
     red[warp][g][2 * t] = acc[0];
@@ -168,6 +216,7 @@ gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, const
 //   5: 16, 2, 4
 //   6: 8, 8, 3
 //   7: 4, 8, 4
+//   8: 5, 8, 3
 // Measured on a B200 (M = 8, microseconds, back to back under programmatic
 // launch, variants 1/2/3/7): 4096x4096 9.2/7.4/7.0/7.6; 4096x12288 24/19/16.8/18.7;
 // 6144x4096 11.4/11.4/10.3/9.6; 24576x4096 gated 44/45/33.6/35.4; 151936x4096
@@ -179,11 +228,19 @@ static int sm_count() {
     return vx_sm_count(sms);
 }
 
+// What decides beside the number of tiles is whether K's chunks are whole batches for the warps: a batch that is not whole
+// costs a trip to memory like any other.  (Until variants were chosen by it, the chunks that were left were loaded one at a
+// time.)  Microseconds, 1 / 8 rows, chosen now and before: 151936 x 1024 float32 out (7) 44.4 / 45.5, 88.5 / 91.7; 151936 x
+// 2560 (8) 111 / 119, 140 / 145; 19456 x 2560 gated (8) 17.2 / 18.8, 21.5 / 22.1; 6144 x 2560 (8) 6.2 / 6.7, 7.2 / 7.4;
+// 4096 x 1024 (3) 2.6 / 2.7, 3.7 / 3.8; 2560 x 9728 (3) 10.4 / 10.8, 11.8 / 12.5; 2048 x 3072 (3) 3.9 / 4.4, 5.1 / 5.6.
 static int pick_variant(int N, int K) {
     const int sms = sm_count();
-    const int tiles = (N + 15) / 16;
-    if (tiles <= 2 * sms || tiles >= 8 * sms) return 3;
-    return 7;
+    const int tiles = (N + 15) / 16, chunks = K / 32;
+    if (tiles <= 2 * sms) return 3;
+    if (tiles >= 8 * sms && chunks % 64 == 0) return 3;
+    if (chunks % 40 == 0) return 8;
+    if (tiles < 8 * sms || chunks % 32 == 0) return 7;
+    return 3;
 }
 
 template <bool GATED, bool SEG, typename TOut>
@@ -198,8 +255,8 @@ static int launch_skinny(const bf16* x, const bf16* W, const float* bias, TOut* 
     const int units = GATED ? N / 2 : N, tile = GATED ? 8 : 16;
     int R = tile;
     long long room = 0;
-    if (variant >= 1 && variant <= 7 && balance) {
-        static const int per_sm[8] = {0, 4, 2, 2, 1, 4, 3, 4};
+    if (variant >= 1 && variant <= 8 && balance) {
+        static const int per_sm[9] = {0, 4, 2, 2, 1, 4, 3, 4, 3};
         const long long slots = (long long)sm_count() * per_sm[variant];
         const long long tiles = (units + tile - 1) / tile;
         const long long waves = (tiles + slots - 1) / slots;
@@ -215,19 +272,24 @@ static int launch_skinny(const bf16* x, const bf16* W, const float* bias, TOut* 
             if (blocks <= room || R >= tile) break;
         }
     }
-#define SK_GO(WARPS, UNROLL, MINB)                                                                                  \
-    VX_LAUNCH_K(VX_K_GEMM, (gemm_skinny_kernel<GATED, SEG, TOut, WARPS, UNROLL, MINB>), blocks, WARPS * 32, 0, stream, x, W, \
+#define SK_GO(WARPS, UNROLL, MINB, TAIL)                                                                            \
+    VX_LAUNCH_K(VX_K_GEMM, (gemm_skinny_kernel<GATED, SEG, TOut, WARPS, UNROLL, MINB, TAIL>), blocks, WARPS * 32, 0, stream, x, W, \
                 bias, out, M, N, K, ldx, ldw, ldo, act, R, seg_rows, seg_stride, segments)
+#define SK_BOTH(WARPS, UNROLL, MINB)                            \
+    if (K % (32 * WARPS * UNROLL)) SK_GO(WARPS, UNROLL, MINB, true); \
+    else SK_GO(WARPS, UNROLL, MINB, false)
     switch (variant) {
-        case 1: SK_GO(8, 4, 4); break;
-        case 2: SK_GO(16, 4, 2); break;
-        case 3: SK_GO(8, 8, 2); break;
-        case 4: SK_GO(16, 8, 1); break;
-        case 5: SK_GO(16, 2, 4); break;
-        case 6: SK_GO(8, 8, 3); break;
-        case 7: SK_GO(4, 8, 4); break;
+        case 1: SK_GO(8, 4, 4, true); break;
+        case 2: SK_GO(16, 4, 2, true); break;
+        case 3: SK_BOTH(8, 8, 2); break;
+        case 4: SK_GO(16, 8, 1, true); break;
+        case 5: SK_GO(16, 2, 4, true); break;
+        case 6: SK_GO(8, 8, 3, true); break;
+        case 7: SK_BOTH(4, 8, 4); break;
+        case 8: SK_BOTH(5, 8, 3); break;
         default: return VX_ERR_SHAPE;
     }
+#undef SK_BOTH
 #undef SK_GO
     VX_LAUNCH_CHECK();
     return VX_OK;
@@ -235,7 +297,7 @@ static int launch_skinny(const bf16* x, const bf16* W, const float* bias, TOut* 
 
 // gated: 0 plain (no activation, or with `act` >= 0 through vx_gemm_skinny_act that one); 1: W rows come in tiles of 16 = 8 gate rows then their 8 up
 // rows, and out is [M, N/2] = act(gate) * up.  out_dtype: VX_BF16 or VX_F32.
-// variant: 0 lets the sizes choose (pick_variant); 1..5 name one, for tuning.
+// variant: 0 lets the sizes choose (pick_variant); 1..8 name one, for tuning.
 extern "C" int vx_gemm_skinny_act(const void* x, const void* W, const float* bias, void* out, int M, int N, int K,
                                   int ldx, int ldw, int ldo, int gated, int act, int out_dtype, int variant,
                                   cudaStream_t stream) {
