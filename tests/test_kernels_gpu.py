@@ -737,3 +737,96 @@ def test_prefill_attention_tc_in_runs_finds_one_far_key(far):
     scale = np.abs(value).max()
     assert np.abs(want[-1, :D] - value).max() < 0.03 * scale, "the far key does not decide the plain answer: the case lost its point"
     assert np.abs(f64(out)[-1, :D] - value).max() < 0.04 * scale
+
+
+# ----------------------------------------------------------------------------
+class _NoCalls:
+    """A call module that leaves everything to the wrappers in Python."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 40, 130])
+def test_call_module_agrees_with_the_wrappers(rows, monkeypatch):
+    """The operations that go through the call module give the bits that their Python wrappers give, and count as launches."""
+    o = ops()
+    H, Hk, D, S, E = 8, 2, 128, 16, 256
+    g = torch.Generator(device=DEV)
+    g.manual_seed(rows)
+    rnd = lambda *shape: torch.randn(shape, generator=g, device=DEV)
+    res, delta, w = rnd(rows, E), rnd(rows, E).bfloat16(), rnd(E)
+    wq, wg = rnd((H + 2 * Hk) * D, E).bfloat16(), rnd(512, E).bfloat16()
+    qw, kw, inv = rnd(D), rnd(D), torch.rand(D // 2, device=DEV)
+    pos = torch.arange(rows, dtype=torch.int32, device=DEV)
+    pages = -(-rows // S) + 1
+    bt = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1)
+    cu = torch.tensor([0, rows], dtype=torch.int32, device=DEV)
+    zero = torch.zeros(1, dtype=torch.int32, device=DEV)
+    some = torch.tensor([rows - 1, 0], dtype=torch.int32, device=DEV)
+
+    def all_of_them():
+        r = res.clone()
+        kp, vp = torch.zeros(pages, Hk, S, D, device=DEV).bfloat16(), torch.zeros(pages, Hk, S, D, device=DEV).bfloat16()
+        n0 = o.launch_count()
+        h = o.add_rmsnorm(r, delta, w, 1e-6, torch.bfloat16)
+        out = [r, h, o.add_rmsnorm(r, None, w, 1e-6, torch.float32), o.add_rmsnorm(r, delta, w, 1e-6, torch.bfloat16, rows=some)]
+        qkv = o.gemm_bf16(h, wq)
+        out += [o.gemm_bf16(h, wq, out_dtype=torch.float32), qkv.clone()]
+        o.qk_norm_rope_kv(qkv, qw, kw, 1e-6, inv, D, pos, pos, kp, vp, H, Hk, D)
+        out += [qkv, kp, vp]
+        seq = torch.zeros(rows, dtype=torch.int32, device=DEV)
+        out.append(o.paged_decode_attention(qkv, qkv.shape[1], kp, vp, bt, seq, pos, 0.1, 0, H, Hk, D, rows, rows, single_tokens=False))
+        out.append(o.paged_prefill_attention_tc(qkv, qkv.shape[1], kp, vp, bt, cu, zero, 0.1, 0, H, Hk, D, 1, rows, rows, max_kv=rows))
+        out += [o.gemm_tcgen05(h, wg, gated_activation="silu"), o.gemm_tcgen05(h, wg, pair=True),
+                o.gemm_tcgen05(h, wg, activation="relu"), o.gated_act(o.gemm_bf16(h, wg, out_dtype=torch.float32), "silu", 8, torch.bfloat16)]
+        o.check_device_errors()
+        return out, o.launch_count() - n0
+
+    o._full_precision_sums()
+    fast, n_fast = all_of_them()
+    monkeypatch.setattr(o, "_CALLS", _NoCalls())
+    slow, n_slow = all_of_them()
+    assert n_fast == n_slow
+    for i, (x, y) in enumerate(zip(fast, slow)):
+        assert x.dtype == y.dtype and torch.equal(x, y), i
+
+
+def test_call_module_leaves_refusals_to_the_wrappers():
+    """What a wrapper refuses is refused with its message, whether or not the call module looked at it first."""
+    from velox_b200.csrc.ops import KernelError
+    o = ops()
+    x, w = torch.zeros(4, 64, device=DEV), torch.ones(64, device=DEV)
+    with pytest.raises(KernelError, match="weight has 32 elements"):
+        o.add_rmsnorm(x, None, w[:32], 1e-6, torch.bfloat16)
+    with pytest.raises(KernelError, match="delta must match"):
+        o.add_rmsnorm(x, x.bfloat16()[:2], w, 1e-6, torch.bfloat16)
+    with pytest.raises(KernelError, match="CUDA tensors"):
+        o.add_rmsnorm(x.cpu(), None, w.cpu(), 1e-6, torch.bfloat16)
+    with pytest.raises(KernelError, match="norm weight size"):
+        o.qk_norm_rope_kv(x.bfloat16(), w[:8], None, 1e-6, None, 0, torch.zeros(4, dtype=torch.int32, device=DEV), None, None, None, 2, 1, 16)
+    with pytest.raises(KernelError, match="bfloat16 operands"):
+        o.gemm_bf16(x, x)
+    with pytest.raises(KernelError, match="K a multiple of 8"):
+        o.gemm_tcgen05(x.bfloat16()[:, :60], x.bfloat16()[:, :60])
+    with pytest.raises(KernelError, match="even width"):
+        o.gated_act(x[:, :63].contiguous(), "silu")
+
+
+@pytest.mark.parametrize("K", [32, 96, 288, 1024, 1280, 2080, 2560])
+@pytest.mark.parametrize("variant", [0, 3, 7, 8])
+def test_skinny_product_with_batches_that_are_not_whole(K, variant):
+    """K that gives a warp no whole batch of chunks, whole ones only, or whole ones and a rest, by every number of warps
+    that the sizes choose.  A sum's error is at most K roundings of 2^-24 of the sum of the products' magnitudes."""
+    N, M = 272, 5
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(M, K, generator=g).bfloat16(), torch.randn(N, K, generator=g).bfloat16()
+    out = ops().gemm_skinny(a.to(DEV), w.to(DEV), None, torch.float32, variant=variant).cpu().double()
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert ((out - want).abs() <= K * 2.0 ** -24 * size).all()
+    gated = ops().gemm_skinny(a.to(DEV), w.to(DEV), None, torch.float32, gated_activation="relu", variant=variant).cpu().double()
+    t = want.view(M, N // 16, 2, 8)
+    ref = (t[:, :, 0].clamp(min=0) * t[:, :, 1]).reshape(M, -1)
+    s = size.view(M, N // 16, 2, 8)
+    bound = (K + 2) * 2.0 ** -24 * 2 * (s[:, :, 0] * s[:, :, 1]).reshape(M, -1)
+    assert ((gated - ref).abs() <= bound).all()

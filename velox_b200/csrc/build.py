@@ -1,9 +1,9 @@
 """Compiles the CUDA sources beside this file into one shared library for sm_100a,
-and the host sources under `host/` (C++, no CUDA) into a second one.
+the host sources under `host/` (C++, no CUDA) into a second one, and the Python module under `calls/`.
 
 `nvcc` is called directly, one object per source file in parallel, then one link;
-no Python or torch header is included by the sources, so a full build takes well
-under a minute.  The library is built in `_build/` beside the sources when that
+no Python or torch header is included by the CUDA and host sources, so a full build takes about
+a minute.  The library is built in `_build/` beside the sources when that
 folder can be written, else under the system's temporary folder.  A build is
 skipped when the library is newer than every source.  Progress lines go to
 stderr.
@@ -188,6 +188,63 @@ def build_host(force: bool = False, verbose: bool = True) -> str:
             fcntl.flock(lock, fcntl.LOCK_UN)
 
 
+CALLS_LIB_NAME = "velox_b200_calls.so"
+CALLS_DIR = os.path.join(HERE, "calls")
+
+
+def build_calls(force: bool = False, verbose: bool = True) -> str:
+    """Build the Python module of the operations that an eager step calls most (C++ with Python's and torch's headers) if
+    it is out of date; returns its path.  It is rebuilt for another Python or torch."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    out_dir = build_dir()
+    lib = os.path.join(out_dir, CALLS_LIB_NAME)
+    srcs = sorted(glob.glob(os.path.join(CALLS_DIR, "*.cpp")))
+    if not srcs:
+        raise BuildError("no .cpp sources in %s" % CALLS_DIR)
+    made_for = os.path.join(out_dir, CALLS_LIB_NAME + ".for")
+    want = "python %s torch %s" % (sys.version.split()[0], torch.__version__)
+
+    def current() -> bool:
+        if force or _stale(lib, srcs + [os.path.abspath(__file__)]) or not os.path.isfile(made_for):
+            return False
+        with open(made_for) as f:
+            return f.read() == want
+
+    if current():
+        return lib
+    with open(os.path.join(out_dir, ".lock_calls"), "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if current():
+                return lib
+            t0 = time.time()
+            if verbose:
+                _say("compiling the call module into %s" % out_dir)
+            cuda = os.path.join(os.path.dirname(os.path.dirname(find_nvcc())), "include")
+            inc = [sysconfig.get_paths()["include"], *include_paths(), cuda]
+            tmp = lib + ".tmp%d" % os.getpid()
+            cmd = [find_cxx(), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+                   "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+            cmd += [x for d in dict.fromkeys(inc) for x in ("-I", d)] + srcs + ["-o", tmp]
+            cmd += ["-L" + d for d in library_paths()] + ["-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+            p = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+            if p.returncode != 0:
+                raise BuildError("the call module failed to compile:\n%s\n%s" % (" ".join(cmd), p.stdout))
+            os.replace(tmp, lib)
+            with open(made_for, "w") as f:
+                f.write(want)
+            if verbose:
+                _say("built %s in %.0f s" % (lib, time.time() - t0))
+            return lib
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+
+
 if __name__ == "__main__":
     build(force="--force" in sys.argv, ptxas_info="--ptxas" in sys.argv)
     build_host(force="--force" in sys.argv)
+    build_calls(force="--force" in sys.argv)

@@ -52,6 +52,37 @@ def library():
     return _LIB
 
 
+_CALLS = None
+
+
+def _calls():
+    """The module of the operations that are called most (`calls/calls.cpp`); built first if needed."""
+    global _CALLS
+    if _CALLS is None:
+        library()
+        import importlib.machinery
+        import importlib.util
+        path = _build.build_calls()
+        loader = importlib.machinery.ExtensionFileLoader("velox_b200_calls", path)
+        try:
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("velox_b200_calls", loader))
+            loader.exec_module(module)
+            module.bind(_LIB._name)
+        except (ImportError, OSError) as e:
+            raise KernelError("the call module %s could not be loaded: %s" % (path, e))
+        _CALLS = module
+    return _CALLS
+
+
+def _called(out, what: str):
+    """What an operation of the call module gave (not None): its result, its launch counted."""
+    global _LAUNCHES
+    if out.__class__ is int:
+        return _check(out, what)
+    _LAUNCHES += 1
+    return out
+
+
 def set_pdl(enabled: bool) -> None:
     """Programmatic dependent launch on or off for kernels launched from now on
     (on by default; VELOX_B200_PDL=0 in the environment starts with it off)."""
@@ -248,6 +279,9 @@ def add_rmsnorm(residual: torch.Tensor, delta: Optional[torch.Tensor], weight: t
     Without `rows` the sum is written back into `residual` (if there is a delta
     and `update_residual`).  With `rows` (int32 indices) only those rows are
     read, and the sums go to `residual_out` if given."""
+    out = (_CALLS or _calls()).add_rmsnorm(residual, delta, weight, eps, out_dtype, rows, residual_out, update_residual)
+    if out is not None:
+        return _called(out, "add_rmsnorm")
     _dev(residual, delta, weight, rows)
     _need(residual.dtype == torch.float32 and residual.is_contiguous(), "add_rmsnorm: float32 contiguous residual")
     _need(weight.dtype == torch.float32, "add_rmsnorm: float32 weight")
@@ -287,6 +321,10 @@ def gated_act(gate_up: torch.Tensor, activation: str, block: int = 0,
     """act(gate) * up.  block == 0: rows are [all gates | all ups]; block > 0: rows
     are tiles of `block` gates followed by their `block` ups.  float32 input may give a
     bfloat16 result (`out_dtype`)."""
+    if activation in ACTIVATIONS:
+        out = (_CALLS or _calls()).gated_act(gate_up, ACTIVATIONS[activation], int(block), out_dtype or gate_up.dtype)
+        if out is not None:
+            return _called(out, "gated_act")
     _dev(gate_up)
     _need(gate_up.is_contiguous() and gate_up.shape[-1] % 2 == 0, "gated_act: contiguous rows of even width")
     _need(activation in ACTIVATIONS, "gated_act: activation %r is not one of %s" % (activation, sorted(ACTIVATIONS)))
@@ -308,6 +346,11 @@ def qk_norm_rope_kv(qkv: torch.Tensor, q_weight, k_weight, eps: float, inv_freq,
     `magnitude`.  Without a slot mapping a row may hold queries only (`num_kv_heads` 0)."""
     v_head_dim = int(v_head_dim) or head_dim
     num_v_heads = int(num_v_heads) or num_kv_heads
+    done = (_CALLS or _calls()).qk_norm_rope_kv(qkv, q_weight, k_weight, eps, inv_freq, rot_dim, positions, slot_mapping, k_pool, v_pool,
+                                                num_heads, num_kv_heads, head_dim, v_head_dim, 1 if interleaved else 0, num_v_heads,
+                                                magnitude)
+    if done is not None:
+        return _called(done, "qk_norm_rope_kv")
     _dev(qkv, q_weight, k_weight, inv_freq, positions, slot_mapping, k_pool, v_pool)
     _need(qkv.is_contiguous() and positions.dtype == torch.int32, "qk_norm_rope_kv: contiguous qkv, int32 positions")
     page_size = 1
@@ -830,7 +873,7 @@ def workspace(device, nfloats: int, which: str = "decode") -> torch.Tensor:
     graph's own."""
     if torch.cuda.is_current_stream_capturing():
         return torch.empty(max(nfloats, 1), dtype=torch.float32, device=device)
-    key = (str(device), which)
+    key = (device, which)
     buf = _WORKSPACE.get(key)
     if buf is None or buf.numel() < nfloats:
         buf = torch.empty(max(nfloats, 1 << 16), dtype=torch.float32, device=device)
@@ -853,6 +896,18 @@ def paged_decode_attention(q: torch.Tensor, q_row_stride: int, k_pool, v_pool, b
     picks the entries' rows; `single_tokens=False` says that some of them are tokens of
     one request's portion (the kernel then waits for the step's cache writes before it
     reads any key).  `shape` names the kernel's form (for measurements and tests; 0: the sizes choose)."""
+    _dev(q)
+    keys = max_kv if window <= 0 else min(max_kv, window + 15)
+    max_splits = max(1, -(-(-(-keys // 16) + (1 if window > 0 else 0)) // DECODE_CHUNK_TILES))
+    scratch = None
+    if max_splits > 1:
+        scratch = workspace(q.device, requests * num_heads * max_splits * (head_dim + 2))
+    done = (_CALLS or _calls()).decode_attention(
+        q, q_row_stride, k_pool, v_pool, block_table, seq_of_token, positions, scale, window, num_heads, num_kv_heads, head_dim, requests,
+        token_rows, out, out_rows if out_rows is not None else requests, scratch, max_splits, DECODE_CHUNK_TILES,
+        1 if single_tokens else 0, shape)
+    if done is not None:
+        return _called(done, "paged_decode_attention")
     _dev(q, k_pool, v_pool, block_table, seq_of_token, positions, token_rows)
     _need(q.dtype == torch.bfloat16 and k_pool.dtype == torch.bfloat16 and v_pool.dtype == torch.bfloat16,
           "paged_decode_attention: bfloat16 only")
@@ -861,11 +916,6 @@ def paged_decode_attention(q: torch.Tensor, q_row_stride: int, k_pool, v_pool, b
     if out is None:
         out = torch.empty((out_rows if out_rows is not None else requests, num_heads * head_dim),
                           dtype=q.dtype, device=q.device)
-    keys = max_kv if window <= 0 else min(max_kv, window + 15)
-    max_splits = max(1, -(-(-(-keys // 16) + (1 if window > 0 else 0)) // DECODE_CHUNK_TILES))
-    scratch = None
-    if max_splits > 1:
-        scratch = workspace(q.device, requests * num_heads * max_splits * (head_dim + 2))
     _check(library().vx_paged_decode_attention_shape(
         _ptr(q), q_row_stride, _ptr(k_pool), _ptr(v_pool), _ptr(block_table), block_table.shape[1],
         _ptr(token_rows), _ptr(seq_of_token), _ptr(positions), _ptr(scratch), max_splits, _ptr(out),
@@ -919,6 +969,23 @@ def paged_prefill_attention_tc(q: torch.Tensor, q_row_stride: int, k_pool, v_poo
     runs of key tiles that several blocks share; 0: never.  `halves`: the probabilities go to the
     tensor core as two bfloat16 halves (32-bit softmax weights in effect; half as many products again);
     with it `sinks` and `gate_col` as in `paged_attention_generic`."""
+    _dev(q)
+    # runs of key tiles: up to a quarter of the longest request's key tiles, 16 at most; only a step whose
+    # portions are short can have a request that is cut (a long portion has query tiles enough)
+    max_splits, scratch = 1, None
+    toks_per_tile = (128 // (num_heads // num_kv_heads)) & ~7   # (as pt_toks_per_tile in the kernel)
+    sms = _sm_count(q.device)
+    if max_kv >= 8 * 128 and 2 * -(-max_new // (2 * toks_per_tile)) * num_kv_heads <= sms:   # (a block takes two query tiles)
+        max_splits = max(1, min(PREFILL_MAX_SPLITS, -(-max_kv // 128) // 4, sms // num_kv_heads))
+        scratch = workspace(q.device, tokens * num_heads * max_splits * (head_dim + 2), which="prefill")
+    if not halves and sinks is None and gate_col < 0:
+        done = (_CALLS or _calls()).prefill_attention(q, q_row_stride, k_pool, v_pool, block_table, cu_seqlens, kv_offsets, scale, window,
+                                                      num_heads, num_kv_heads, head_dim, requests, max_new, tokens, seq_list, out,
+                                                      scratch, max_splits, _error_word(q.device))
+        if done is not None:
+            done = _called(done, "paged_prefill_attention_tc")
+            note_bounded_wait()
+            return done
     _dev(q, k_pool, v_pool, block_table, cu_seqlens, kv_offsets, seq_list, out, sinks)
     _need(halves or (sinks is None and gate_col < 0), "paged_prefill_attention_tc: a sink and a gate go with halves=True")
     _check_sinks_gate("paged_prefill_attention_tc", sinks, gate_col, num_heads, q_row_stride)
@@ -929,14 +996,6 @@ def paged_prefill_attention_tc(q: torch.Tensor, q_row_stride: int, k_pool, v_poo
     _need(k_pool.is_contiguous() and v_pool.is_contiguous(), "paged_prefill_attention_tc: contiguous pools")
     if out is None:
         out = torch.empty((tokens, num_heads * head_dim), dtype=q.dtype, device=q.device)
-    # runs of key tiles: up to a quarter of the longest request's key tiles, 16 at most; only a step whose
-    # portions are short can have a request that is cut (a long portion has query tiles enough)
-    max_splits, scratch = 1, None
-    toks_per_tile = (128 // (num_heads // num_kv_heads)) & ~7   # (as pt_toks_per_tile in the kernel)
-    sms = _sm_count(q.device)
-    if max_kv >= 8 * 128 and 2 * -(-max_new // (2 * toks_per_tile)) * num_kv_heads <= sms:   # (a block takes two query tiles)
-        max_splits = max(1, min(PREFILL_MAX_SPLITS, -(-max_kv // 128) // 4, sms // num_kv_heads))
-        scratch = workspace(q.device, tokens * num_heads * max_splits * (head_dim + 2), which="prefill")
     args = (_ptr(q), q_row_stride, tokens, _ptr(k_pool), _ptr(v_pool), k_pool.shape[0], _ptr(block_table),
             block_table.shape[1], _ptr(cu_seqlens), _ptr(kv_offsets), _ptr(seq_list), _ptr(out), num_heads * head_dim, float(scale),
             int(window), requests, int(max_new), num_heads, num_kv_heads, head_dim, k_pool.shape[2],
@@ -1523,10 +1582,10 @@ _SM_COUNTS = {}
 
 
 def _sm_count(device) -> int:
-    key = str(device)
-    if key not in _SM_COUNTS:
-        _SM_COUNTS[key] = torch.cuda.get_device_properties(device).multi_processor_count
-    return _SM_COUNTS[key]
+    count = _SM_COUNTS.get(device)
+    if count is None:
+        count = _SM_COUNTS[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    return count
 
 
 _ERROR_WORDS = {}
@@ -1534,10 +1593,10 @@ _ERROR_WORDS = {}
 
 def _error_word(device) -> torch.Tensor:
     """The device int that kernels with bounded waits report into."""
-    key = str(device)
-    if key not in _ERROR_WORDS:
-        _ERROR_WORDS[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _ERROR_WORDS[key]
+    word = _ERROR_WORDS.get(device)
+    if word is None:
+        word = _ERROR_WORDS[device] = torch.zeros(1, dtype=torch.int32, device=device)
+    return word
 
 
 _BOUNDED_WAIT_LAUNCHES = 0   # launches of kernels with bounded waits, ever
@@ -1583,6 +1642,10 @@ def check_device_errors() -> None:
 
 
 def tcgen05_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
+    if a.is_cuda:
+        yes = (_CALLS or _calls()).tcgen05_supported(a, w)
+        if yes is not None:
+            return yes
     return (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.shape[1] % 8 == 0 and w.shape[0] % 16 == 0
             and a.stride(1) == 1 and w.stride(1) == 1 and a.stride(0) % 8 == 0 and w.stride(0) % 8 == 0
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
@@ -1629,6 +1692,13 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
     code, act = _epilogue("gemm_tcgen05", gated_activation, activation)
     _need(activation is None or activation in TCGEN05_ACTIVATIONS, "gemm_tcgen05: a plain activation is one of %s" % (TCGEN05_ACTIVATIONS,))
     _need(not (pair and activation), "gemm_tcgen05: a plain activation on tiles of single blocks")
+    if gated_activation is None or gated_activation in ACTIVATIONS:
+        out = (_CALLS or _calls()).gemm_tcgen05(a, w, bias, code, ACTIVATIONS.get(gated_activation, 0) if pair else act, 1 if wide else 0,
+                                                1 if pair else 0, _error_word(a.device))
+        if out is not None:
+            out = _called(out, "gemm_tcgen05_pair" if pair else "gemm_tcgen05")
+            note_bounded_wait()
+            return out
     _need(a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1], "gemm_tcgen05: a [M,K], w [N,K]")
     _need(tcgen05_supported(a, w), "gemm_tcgen05: bfloat16, K a multiple of 8, N a multiple of 16, 16-byte aligned rows")
     m, k = a.shape
@@ -1722,6 +1792,11 @@ def _full_precision_sums() -> None:
 
 def gemm_bf16(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """a [M,K] times w [N,K] transposed on the tensor cores, float32 accumulation."""
+    if bias is None and _MATMUL_SET:
+        few = a.shape[0] <= SKINNY_MAX_ROWS
+        out = (_CALLS or _calls()).gemm_bf16(a, w, out_dtype or torch.bfloat16)
+        if out is not None:
+            return _called(out, "gemm_skinny") if few and skinny_supported(a.shape[0], a.shape[1], a, w) else out
     _dev(a, w, bias)
     _need(a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16, "gemm_bf16: bfloat16 operands")
     out_dtype = out_dtype or torch.bfloat16

@@ -12,6 +12,7 @@ layers.
 from __future__ import annotations
 
 import ctypes
+import itertools
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
@@ -107,7 +108,7 @@ def build_step_arrays(entries: Sequence[StepEntry], cache, vocab_size: Optional[
         rids = cache.handles(e.request_id for e in entries)
     except KeyError as e:
         raise KeyError("request %r holds no cache; add it first" % (e.args[0],))
-    tokens = np.fromiter((t for e in entries for t in e.tokens), np.int64, total)
+    tokens = np.fromiter(itertools.chain.from_iterable(e.tokens for e in entries), np.int64, total)
     if vocab_size is not None and total and (tokens.min() < 0 or tokens.max() >= vocab_size):
         bad = next(e.request_id for e in entries if any(not 0 <= int(t) < vocab_size for t in e.tokens))
         raise ValueError("request %r: token id outside [0, %d)" % (bad, vocab_size))
