@@ -123,6 +123,14 @@ gemm_skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, const
                 mma_bf16_16816(acc, a[u].z, b[u].z, a[u].w, b[u].w, xv[u].z, xv[u].w);
             }
         }
+        // (never run: without it the compiler gives the loop above two registers less and 3 % less speed)
+        for (; c < nchunks; c += SK_WARPS) {
+            const int k = c << 5;
+            const uint4 ta = va ? ld_stream16(wa + k) : zero4, tb = vb ? ld_stream16(wb + k) : zero4;
+            const uint4 xv = xok ? *reinterpret_cast<const uint4*>(xr + k) : make_uint4(0, 0, 0, 0);
+            mma_bf16_16816(acc, ta.x, tb.x, ta.y, tb.y, xv.x, xv.y);
+            mma_bf16_16816(acc, ta.z, tb.z, ta.w, tb.w, xv.z, xv.w);
+        }
     } else {
         // The warp's chunks come in batches of SK_UNROLL, whole ones and then what is left: all loads of a batch are on their
         // way before the first is used (which chunks there are is the same for the whole warp).
