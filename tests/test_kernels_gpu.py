@@ -830,3 +830,26 @@ def test_skinny_product_with_batches_that_are_not_whole(K, variant):
     s = size.view(M, N // 16, 2, 8)
     bound = (K + 2) * 2.0 ** -24 * 2 * (s[:, :, 0] * s[:, :, 1]).reshape(M, -1)
     assert ((gated - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("columns", [16, 48, 128, 144, 176, 208, 240, 256])
+@pytest.mark.parametrize("M,N,K", [(1, 16, 8), (130, 464, 200), (300, 1040, 320)])
+def test_gemm_tcgen05_tiles_of_any_width(M, N, K, columns):
+    """Tiles whose last 32 columns are half a tile's, tiles wider than the matrix, several tiles a block: the sums that tiles
+    of 256 columns give, bit for bit (every sum is formed over k in the same order), gated, plain with a bias and activated."""
+    g = torch.Generator().manual_seed(M + columns)
+    a, w = torch.randn(M, K, generator=g).bfloat16().to(DEV), torch.randn(N, K, generator=g).bfloat16().to(DEV)
+    bias = torch.randn(N, generator=g).to(DEV)
+    for more in (dict(gated_activation="silu"), dict(bias=bias), dict(activation="relu2")):
+        wide = ops().gemm_tcgen05(a, w, **more)
+        assert torch.equal(ops().gemm_tcgen05(a, w, columns=columns, **more), wide), more
+    ops().check_device_errors()
+
+
+def test_tcgen05_tile_fills_rounds():
+    """The choice of tiles stays within what the kernels take."""
+    for m in (1, 128, 129, 312, 777, 2048, 40000):
+        for n in (16, 512, 6144, 19456, 34816):
+            for k in (64, 2048, 2560, 9728):
+                pair, columns = ops().tcgen05_tile(m, n, k, torch.device(DEV))
+                assert pair == (columns == 0) and columns % 16 == 0 and columns <= 256

@@ -2,17 +2,17 @@
 // cores: tcgen05.mma with the accumulator in tensor memory, operands brought into
 // shared memory by TMA.
 //
-// Blocks are persistent (one per SM); each takes 128 x BN tiles of C (BN = 128 or
-// 256) in turn and has six warps, which work on different tiles at once: while the
+// Blocks are persistent (one per SM); each takes 128 x bn tiles of C (bn at most BN = 128 or
+// 256, chosen so that the tiles fill rounds of the SMs) in turn and has six warps, which work on different tiles at once: while the
 // epilogue warps write tile i from one half of the tensor memory, the tensor core
 // already accumulates tile i + 1 in the other half, fed by a ring of stages that
 // runs on across tiles:
 //   warp 0   producer: one thread waits for a free stage and issues two tiled TMA
 //            loads (cp.async.bulk.tensor.2d, 128-byte swizzle): a 128 x 64 tile of A
-//            and a BN x 64 tile of W, completion counted on the stage's "full"
+//            and a bn x 64 tile of W, completion counted on the stage's "full"
 //            mbarrier;
 //   warp 1   allocates 2 x BN columns of tensor memory; one thread waits for a full
-//            stage, issues four tcgen05.mma (M 128, N BN, K 16 each) whose operands
+//            stage, issues four tcgen05.mma (M 128, N bn, K 16 each) whose operands
 //            are shared-memory descriptors of the swizzled tiles, and commits them to
 //            the stage's "empty" mbarrier, so the stage is free when the tensor core
 //            has read it; after a tile's last k block it commits to that
@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(TC_THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const float* __restrict__ bias, bf16* __restrict__ C, int M, int N, int K, int ldc, int act,
                     int* __restrict__ error, const int* __restrict__ row_tiles, const int* __restrict__ n_row_tiles,
-                    const float* __restrict__ row_scale, const int* __restrict__ src_of_row, float limit, float slope) {
+                    const float* __restrict__ row_scale, const int* __restrict__ src_of_row, float limit, float slope, int bn) {
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_s;
@@ -65,7 +65,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // Tiles are numbered with the row tile running fastest, so that blocks working
     // at the same time share a tile of W and walk over the rows of A (which stays
     // in L2): W is read from memory once.  Block b takes tiles b, b + grid, ...
-    const int mtiles = row_tiles ? n_row_tiles[0] : (M + TC_BM - 1) / TC_BM, ntiles = (N + BN - 1) / BN;
+    const int mtiles = row_tiles ? n_row_tiles[0] : (M + TC_BM - 1) / TC_BM, ntiles = (N + bn - 1) / bn;
     const int total_tiles = mtiles * ntiles;
     const int my_tiles = (total_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
@@ -99,7 +99,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
                 const int rt = tile % mtiles;
                 const int m0 = row_tiles ? row_tiles[3 * rt + 1] : rt * TC_BM;
-                const int n0 = (tile / mtiles) * BN + (row_tiles ? row_tiles[3 * rt] * N : 0);   // (row of W)
+                const int n0 = (tile / mtiles) * bn + (row_tiles ? row_tiles[3 * rt] * N : 0);   // (row of W)
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (it >= STAGES &&
@@ -109,7 +109,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         break;
                     }
                     const unsigned bar = tc_smem_u32(&full_bar[s]);
-                    tc_mbar_expect_tx(bar, STAGE_BYTES);
+                    tc_mbar_expect_tx(bar, A_BYTES + (unsigned)bn * (TC_BK * 2));
                     unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
                     tc_tma_load_2d(tc_smem_u32(st), &map_a, kb * TC_BK, m0, bar);
                     tc_tma_load_2d(tc_smem_u32(st + A_BYTES), &map_w, kb * TC_BK, n0, bar);
@@ -119,8 +119,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else if (warp == 1) {
         // ---- tensor core: tile ti accumulates into buffer ti & 1 ----
         if (lane == 0) {
-            // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = BN, M = 128
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) |
+            // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = bn, M = 128
+            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) |
                                    ((unsigned)(TC_BM >> 4) << 24);
             int it = 0;
             for (int ti = 0; ti < my_tiles && !failed; ++ti) {
@@ -162,7 +162,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int buf = ti & 1;
             const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
             const int rt = tile % mtiles;
-            const int m0 = row_tiles ? row_tiles[3 * rt + 1] : rt * TC_BM, n0 = (tile / mtiles) * BN;
+            const int m0 = row_tiles ? row_tiles[3 * rt + 1] : rt * TC_BM, n0 = (tile / mtiles) * bn;
+            const int n_end = min(N, n0 + bn);   // (columns past it hold zeros, or what an earlier tile left)
             // (a grouped tile stores only its own rows: those after them belong to the next group)
             const int row = (row_tiles && quarter * 32 + lane >= row_tiles[3 * rt + 2]) ? M : m0 + quarter * 32 + lane;
             const float rs = EPI != TC_PLAIN && row_scale && row < M ? row_scale[src_of_row[row]] : 1.f;
@@ -173,8 +174,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned tmem_acc = tmem_base + (unsigned)(buf * BN) + ((unsigned)(quarter * 32) << 16);
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                if (n0 + c0 >= N) break;   // (uniform) columns past N hold zeros
+            for (int c0 = 0; c0 < bn; c0 += 32) {
+                if (n0 + c0 >= n_end) break;   // (uniform)
                 unsigned r[32];
                 tc_ld32(tmem_acc + (unsigned)c0, r);
                 if (row >= M) continue;
@@ -186,7 +187,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     bf16* dst = C + (size_t)row * ldc + n0 + c0;
 #pragma unroll
                     for (int j = 0; j < 32; j += 8) {
-                        if (n0 + c0 + j >= N) break;
+                        if (n0 + c0 + j >= n_end) break;
                         float v[8];
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
@@ -207,7 +208,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     bf16* dst = C + (size_t)row * ldc + ((n0 + c0) >> 1);
 #pragma unroll
                     for (int t = 0; t < 2; ++t) {   // two tiles of 8 gates + 8 ups
-                        if (n0 + c0 + t * 16 >= N) break;
+                        if (n0 + c0 + t * 16 >= n_end) break;
                         uint4 pk;
                         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
@@ -242,17 +243,17 @@ template <int BN, int STAGES, int EPI>
 static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mw, const float* bias, bf16* C, int M, int N, int K,
                      int ldc, int act, int* error, cudaStream_t stream, const int* row_tiles = nullptr,
                      const int* n_row_tiles = nullptr, int max_row_tiles = 0, const float* row_scale = nullptr,
-                     const int* src_of_row = nullptr, float limit = 0.f, float slope = 0.f) {
+                     const int* src_of_row = nullptr, float limit = 0.f, float slope = 0.f, int bn = BN) {
     const size_t smem = (size_t)STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024;
     static bool configured[VX_MAX_DEVICES];
     if (int rc = vx_configure_smem(gemm_tcgen05_kernel<BN, STAGES, EPI>, smem, configured)) return rc;
     // persistent: one block per SM (its shared memory fills one), fewer if there are fewer tiles
     static int sm_counts[VX_MAX_DEVICES];
     const int sms = vx_sm_count(sm_counts);
-    const int tiles = (row_tiles ? max_row_tiles : (M + TC_BM - 1) / TC_BM) * ((N + BN - 1) / BN);
+    const int tiles = (row_tiles ? max_row_tiles : (M + TC_BM - 1) / TC_BM) * ((N + bn - 1) / bn);
     dim3 grid(tiles < sms ? tiles : sms);
     VX_LAUNCH_K(VX_K_GEMM, (gemm_tcgen05_kernel<BN, STAGES, EPI>), grid, TC_THREADS, smem, stream, ma, mw, bias, C, M,
-                N, K, ldc, act, error, row_tiles, n_row_tiles, row_scale, src_of_row, limit, slope);
+                N, K, ldc, act, error, row_tiles, n_row_tiles, row_scale, src_of_row, limit, slope, bn);
     VX_LAUNCH_CHECK();
     return VX_OK;
 }
@@ -260,7 +261,8 @@ static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mw, const float* 
 // gated: 0 plain, C is [M, N]; 1: W's rows come in tiles of 8 gate rows followed by
 // their 8 up rows and C is [M, N/2] = act(gate) * up; 2: C is [M, N] = act(.), relu or its square.  `error` is a device int that
 // a block sets (TC_ERR_*) if one of its bounded waits runs out; the caller zeroes it
-// and reads it when it wants to know.  `wide` picks 128 x 256 tiles (else 128 x 128).
+// and reads it when it wants to know.  `wide` picks 128 x 256 tiles (0: 128 x 128; 16 to 256, a multiple of 16: tiles of as many
+// columns).
 extern "C" int vx_gemm_tcgen05(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int lda,
                                int ldw, int ldc, int gated, int act, int wide, int* error, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return VX_OK;
@@ -270,11 +272,12 @@ extern "C" int vx_gemm_tcgen05(const void* A, const void* W, const float* bias, 
     if (gated < 0 || gated > TC_ACT || (gated && (act < 0 || act > VX_ACT_LAST)) || (gated == TC_GATED && bias)) return VX_ERR_SHAPE;
     if (gated == TC_ACT && !tc_cheap_act(act)) return VX_ERR_SHAPE;
     if (ldc < (gated == TC_GATED ? N / 2 : N)) return VX_ERR_SHAPE;
+    if (wide < 0 || wide > 256 || (wide > 1 && (wide & 15))) return VX_ERR_SHAPE;
     CUtensorMap ma, mw;
-    const int bn = wide ? 256 : 128;
+    const int bn = wide > 1 ? wide : (wide ? 256 : 128);
     if (!tc_make_map(&ma, A, M, K, lda, TC_BM) || !tc_make_map(&mw, W, N, K, ldw, bn)) return VX_ERR_DRIVER;
     bf16* c = (bf16*)C;
-#define TC_GO(BN_, ST_, E_) tc_launch<BN_, ST_, E_>(ma, mw, bias, c, M, N, K, ldc, act, error, stream)
+#define TC_GO(BN_, ST_, E_) tc_launch<BN_, ST_, E_>(ma, mw, bias, c, M, N, K, ldc, act, error, stream, nullptr, nullptr, 0, nullptr, nullptr, 0.f, 0.f, bn)
     if (wide) return gated == TC_GATED ? TC_GO(256, 4, TC_GATED) : (gated == TC_ACT ? TC_GO(256, 4, TC_ACT) : TC_GO(256, 4, TC_PLAIN));
     return gated == TC_GATED ? TC_GO(128, 6, TC_GATED) : (gated == TC_ACT ? TC_GO(128, 6, TC_ACT) : TC_GO(128, 6, TC_PLAIN));
 #undef TC_GO

@@ -1651,6 +1651,24 @@ def tcgen05_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def tcgen05_tile(m: int, n: int, k: int, device) -> Tuple[bool, int]:
+    """(pair, columns) of the tiles for an [m, n] product of depth k: 256 x 256 by pairs of blocks, or 128 x columns by single
+    ones.  What counts are the rounds of the GPU's SMs, padding included, so narrower tiles win where they fill the last round.
+    A round of narrower tiles takes 1/2 + columns / 512 of one of 256 columns (a block also brings the 128 rows of A: measured
+    0.83 to 0.93 at 176, 0.91 at 208), a round of pairs 0.93 of it, but 1.02 up to k = 2,048, where a pair's start counts.
+    Gated products, us, chosen and before (256 columns or pairs): 777 x 6144 x 1024 (160 columns) 21.4, 28.9; 200 x 6144 x 1024 (128)
+    12.9, 17.7; 777 x 12288 x 2048 (208) 43.7, 47.1; 312 x 19456 x 2560 (208) 40.8, 44.3; 200 x 19456 x 2560 (144) 36.2, 41.5; from about 900
+    rows at these widths on pairs stay ahead (900 x 24576 x 4096: 157, 162 with 224 columns)."""
+    sms = _sm_count(device)
+    rows = -(-m // 128)
+    best, columns = (0.93 if k > 2048 else 1.02) * -(-(-(-m // 256) * -(-n // 256)) // max(1, sms // 2)), 0
+    for c in range(256, 127, -16):
+        cost = -(-(rows * -(-n // c)) // sms) * (0.5 + c / 512)
+        if cost < best:
+            best, columns = cost, c
+    return columns == 0, columns
+
+
 def tcgen05_pair_better(m: int, n: int, device) -> bool:
     """Whether 256 x 256 tiles by pairs of blocks beat 128 x 256 tiles by single blocks for
     an [m, n] result: both kinds of block spend the same time on a tile (a pair a little
@@ -1681,19 +1699,21 @@ def tcgen05_fills(m: int, n: int, device) -> bool:
 
 
 def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: Optional[str] = None,
-                 wide: bool = True, pair: bool = False, activation: Optional[str] = None) -> torch.Tensor:
+                 wide: bool = True, pair: bool = False, activation: Optional[str] = None, columns: int = 0) -> torch.Tensor:
     """a [M,K] times w [N,K] transposed on the tcgen05 tensor cores (bfloat16 in and
     out, float32 accumulation in tensor memory, operands by TMA).  With
     `gated_activation`, w's rows come in tiles of 8 gate rows followed by their 8 up
     rows and the result is act(gate) * up, [M, N/2].  `wide`: 128 x 256 tiles, else
     128 x 128; `pair`: 256 x 256 tiles, each formed by a pair of blocks.  With `activation` the result is act(.) of the
-    float32 sums (single blocks only; one of `TCGEN05_ACTIVATIONS`)."""
+    float32 sums (single blocks only; one of `TCGEN05_ACTIVATIONS`).  `columns` (a multiple of 16, at most 256): tiles of
+    128 rows and so many columns."""
     _dev(a, w, bias)
     code, act = _epilogue("gemm_tcgen05", gated_activation, activation)
     _need(activation is None or activation in TCGEN05_ACTIVATIONS, "gemm_tcgen05: a plain activation is one of %s" % (TCGEN05_ACTIVATIONS,))
+    _need(not columns or (16 <= columns <= 256 and columns % 16 == 0 and not pair), "gemm_tcgen05: tiles of 16 to 256 columns by single blocks")
     _need(not (pair and activation), "gemm_tcgen05: a plain activation on tiles of single blocks")
     if gated_activation is None or gated_activation in ACTIVATIONS:
-        out = (_CALLS or _calls()).gemm_tcgen05(a, w, bias, code, ACTIVATIONS.get(gated_activation, 0) if pair else act, 1 if wide else 0,
+        out = (_CALLS or _calls()).gemm_tcgen05(a, w, bias, code, ACTIVATIONS.get(gated_activation, 0) if pair else act, columns or (1 if wide else 0),
                                                 1 if pair else 0, _error_word(a.device))
         if out is not None:
             out = _called(out, "gemm_tcgen05_pair" if pair else "gemm_tcgen05")
@@ -1716,7 +1736,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
                                               _ptr(_error_word(a.device)), _stream()), "gemm_tcgen05_pair")
     else:
         _check(library().vx_gemm_tcgen05(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0), w.stride(0), cols,
-                                         code, act, 1 if wide else 0, _ptr(_error_word(a.device)), _stream()), "gemm_tcgen05")
+                                         code, act, columns or (1 if wide else 0), _ptr(_error_word(a.device)), _stream()), "gemm_tcgen05")
     note_bounded_wait()
     return out
 

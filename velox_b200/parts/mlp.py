@@ -64,8 +64,8 @@ class GatedMLP(FeedForward):
         elif fused and h.shape[0] >= FUSED_TCGEN05_MIN_ROWS and ops.tcgen05_supported(h, w):
             # a prompt portion: tcgen05 product with the same epilogue (measured no slower than
             # the library product followed by the activation kernel from 128 rows, faster from 512)
-            a = ops.gemm_tcgen05(h, w, None, gated_activation=self.activation,
-                                 pair=ops.tcgen05_pair_better(h.shape[0], w.shape[0], h.device))
+            pair, columns = ops.tcgen05_tile(h.shape[0], w.shape[0], h.shape[1], h.device)
+            a = ops.gemm_tcgen05(h, w, None, gated_activation=self.activation, pair=pair, columns=columns)
         elif h.dtype == torch.bfloat16:
             # the library product hands over its float32 sums: gate and up are not rounded
             # before the activation, as in the fused kernels
