@@ -411,3 +411,34 @@ def test_bounded_logits_and_products_per_head():
         ops.gemm_heads(dev(a, dtype)[:, :, :12], dev(w, dtype), out[:, :, :20])
         close(out[:, :, :20], np.einsum("mhk,hnk->mhn", a[:, :, :12], w), 2 * TOL[dtype])
         assert torch.isnan(out[:, :, 20:]).all()
+
+
+@pytest.mark.parametrize("C,R,H,window", [(512, 64, 16, 0), (256, 48, 40, 0), (128, 16, 3, 100), (64, 64, 17, 33)])
+@pytest.mark.parametrize("max_kv", [0, 640])
+def test_latent_attention_on_the_tensor_cores(C, R, H, window, max_kv):
+    """bfloat16 rows of the sizes that go to the tensor-core kernel, with and without runs: lengths around a tile's edges
+    (32 rows), widths of an odd number of 16 elements, heads that do not fill a block, a window.  The result is rounded
+    to bfloat16 (2^-9); weights in two bfloat16 halves (2^-17), float32 sums and the scores' rounding
+    (2^-24 of sums up to 40 times the score) are well below: 2^-8 of a row's largest value."""
+    from velox_b200.csrc import ops
+    lens, S = [1, 31, 32, 33, 64, 65, 270, 600], 16
+    g = torch.Generator().manual_seed(C + H)
+    blocks = -(-max(lens) // S)
+    pool = torch.full((len(lens) * blocks, 1, S, C + R), float("nan")).bfloat16()
+    table = torch.randperm(len(lens) * blocks, generator=g).view(len(lens), blocks).int()
+    qa = (0.3 * torch.randn(len(lens), H, C + R, generator=g)).bfloat16()
+    want = torch.empty(len(lens), H, C, dtype=torch.float64)
+    for i, n in enumerate(lens):
+        rows = torch.randn(n, C + R, generator=g).bfloat16()
+        for j in range(n):
+            pool[table[i, j // S], 0, j % S] = rows[j]
+        s = qa[i].double() @ rows.double().T * 0.1
+        if window:
+            s[:, :max(0, n - window)] = -float("inf")
+        want[i] = s.softmax(-1) @ rows[:, :C].double()
+    t = lambda x: x.to(DEV)
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32)
+    got = ops.latent_attention(t(qa), t(pool), t(table), t(torch.arange(len(lens), dtype=torch.int32)), t(pos), 0.1, H, C, R,
+                               max_kv=max_kv, window=window).cpu().double()
+    err = (got - want).abs().amax(-1) / want.abs().amax(-1)
+    assert torch.isfinite(got).all() and err.max() <= 2.0 ** -8, err.max()

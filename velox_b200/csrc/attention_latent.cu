@@ -12,7 +12,9 @@
 // row again read once for the four heads.  With `runs` > 1 a token's tiles are dealt to the runs in contiguous stretches,
 // every run writes (maximum, sum, accumulator) to a scratch buffer, and a join kernel adds them in run order.  Scores,
 // weights and sums are float32; the order of every sum depends on the token's own position and on `runs` alone.
+// bfloat16 rows of sizes that suit it go to a kernel on the tensor cores instead (latent_attention_mma_kernel).
 #include "common.cuh"
+#include "mma_helpers.cuh"
 
 #define AL_WARPS 4
 #define AL_HW 4                       // heads of a warp
@@ -239,6 +241,220 @@ latent_attention_kernel(const T* __restrict__ qa, const T* __restrict__ pool, co
     }
 }
 
+// The same for bfloat16 rows with C 64, 128, 256 or 512 and W a multiple of 16, by mma.sync.m16n8k16 (bf16 in, float32 out): a
+// block's sixteen heads are the 16 rows, keys (for the scores) or channels (for the sums) the columns.  Rows stay bfloat16 in
+// shared memory (cp.async, two tiles in flight); a warp forms the scores of 8 of a tile's 32 keys for all heads, every warp takes
+// the softmax of all of them (the same operations in the same order), and adds up a quarter of the channels.  The weights go to
+// the tensor cores in two bfloat16 parts, w = hi + lo up to 2^-17 of w, far below the result's own rounding; sums are float32.
+// A decode step's blocks have a tile or two each, and what bounds them is the length of the chain from one to the next: the
+// kernel above takes 17 us a tile (144 steps of five shared-memory reads a score, then 32 rows one after another).
+// LAT_FIG
+template <int NT>   // n-tiles of 8 channels a warp: C / 32
+__global__ void __launch_bounds__(AL_WARPS * 32)
+latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict__ pool, const int* __restrict__ block_table,
+                            int max_blocks, const int* __restrict__ seq_of_token, const int* __restrict__ positions,
+                            bf16* __restrict__ out, float* __restrict__ scratch, float scale, int H, int R, int S, int runs, int window) {
+    extern __shared__ __align__(16) float al_smem[];
+    constexpr int C = 32 * NT;
+    const int W = C + R, ld = W + 8;   // (rows 16 (mod 32) bytes apart modulo 128: ldmatrix hits distinct banks)
+    bf16* q_s = reinterpret_cast<bf16*>(al_smem);           // [16][ld]
+    bf16* k_s = q_s + AL_HEADS * ld;                        // [2][AL_TILE][ld]
+    float* s_s = reinterpret_cast<float*>(k_s + 2 * AL_TILE * ld);   // [16][AL_TILE + 4]
+    constexpr int SLD = AL_TILE + 4;
+    const int t = blockIdx.x, h0 = blockIdx.y * AL_HEADS, run = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+    pdl_wait();
+    pdl_trigger();
+    const int kv_len = positions[t] + 1;
+    const int* bt = block_table + (size_t)seq_of_token[t] * max_blocks;
+    const int start = (window > 0 && kv_len > window) ? kv_len - window : 0;
+    const int first_tile = start / AL_TILE;
+    const int tiles = (kv_len + AL_TILE - 1) / AL_TILE;
+    const int per_run = (tiles - first_tile + runs - 1) / runs;
+    const int tile0 = first_tile + run * per_run, tile1 = min(tiles, tile0 + per_run);
+
+    auto copy_row = [&](bf16* dst, const bf16* src) {   // null: zeros
+        for (int d = lane * 8; d < W; d += 256) {
+            const unsigned to = (unsigned)__cvta_generic_to_shared(dst + d);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(src ? src + d : qa), "r"(src ? 16 : 0));
+        }
+    };
+    auto ask = [&](int tile) {
+        if (tile < tile1) {
+            const int j = tile * AL_TILE + lane;
+            // (lane r: where row r of the tile lies, -1: before the window or past the last; 2^31 rows are 2 TB)
+            const int row = j < kv_len && j >= start ? bt[j / S] * S + j % S : -1;
+            bf16* dst = k_s + (size_t)(tile & 1) * AL_TILE * ld;
+#pragma unroll
+            for (int i = 0; i < AL_TILE / AL_WARPS; ++i) {
+                const int r = warp + i * AL_WARPS, from = __shfl_sync(0xffffffffu, row, r);
+                copy_row(dst + r * ld, from >= 0 ? pool + (size_t)from * W : nullptr);
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < AL_HEADS / AL_WARPS; ++i) {
+        const int hh = warp + i * AL_WARPS;
+        copy_row(q_s + hh * ld, h0 + hh < H ? qa + ((size_t)t * H + h0 + hh) * W : nullptr);
+    }
+    ask(tile0);
+    ask(tile0 + 1);
+
+    float acc[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};   // heads g and g + 8; the sums are this thread's share of a quad's
+    const int mi = lane >> 3;
+    const bf16* qa_at = q_s + (((mi & 1) << 3) + (lane & 7)) * ld + ((mi >> 1) << 3);   // A operand
+
+    for (int tile = tile0; tile < tile1; ++tile) {
+        cp_async_wait<1>();
+        __syncthreads();
+        const bf16* kt = k_s + (size_t)(tile & 1) * AL_TILE * ld;
+        // scores of keys 8 warp .. + 7: two steps of 16 elements a turn, in two sums
+        {
+            const bf16* k_at = kt + (warp * 8 + (lane & 7)) * ld + (mi << 3);
+            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+            int d = 0;
+#pragma unroll 2
+            for (; d + 32 <= W; d += 32) {
+                unsigned a[4], b[4];
+                ldmatrix_x4(b[0], b[1], b[2], b[3], k_at + d);
+                ldmatrix_x4(a[0], a[1], a[2], a[3], qa_at + d);
+                mma_bf16(s0, a, b[0], b[1]);
+                ldmatrix_x4(a[0], a[1], a[2], a[3], qa_at + d + 16);
+                mma_bf16(s1, a, b[2], b[3]);
+            }
+            if (d < W) {   // (16 elements are left; the second half of the load repeats the first and is unused)
+                unsigned a[4], b[4];
+                ldmatrix_x4(b[0], b[1], b[2], b[3], kt + (warp * 8 + (lane & 7)) * ld + ((mi & 1) << 3) + d);
+                ldmatrix_x4(a[0], a[1], a[2], a[3], qa_at + d);
+                mma_bf16(s0, a, b[0], b[1]);
+            }
+            const int key = tile * AL_TILE + warp * 8 + c2;
+            float* dst = s_s + g * SLD + warp * 8 + c2;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const bool seen = key + j < kv_len && key + j >= start;
+                dst[j] = seen ? (s0[j] + s1[j]) * scale : -INFINITY;
+                dst[8 * SLD + j] = seen ? (s0[j + 2] + s1[j + 2]) * scale : -INFINITY;
+            }
+        }
+        __syncthreads();
+        // weights of all 32 keys, as A operands of two steps of 16 keys: [step][A register] two keys each
+        unsigned hi[2][4], lo[2][4];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const float* row = s_s + (g + 8 * half) * SLD + c2;
+            float p[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 x = *reinterpret_cast<const float2*>(row + 8 * i);
+                p[2 * i] = x.x;
+                p[2 * i + 1] = x.y;
+            }
+            float mx = p[0];
+#pragma unroll
+            for (int i = 1; i < 8; ++i) mx = fmaxf(mx, p[i]);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float m_new = fmaxf(m[half], mx), less = m_new == -INFINITY ? 0.f : m_new;
+            const float alpha = expf(m[half] - less);   // m = -inf before the first tile: 0
+            m[half] = m_new;
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                p[i] = expf(p[i] - less);
+                sum += p[i];
+            }
+            l[half] = l[half] * alpha + sum;
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                acc[i][2 * half] *= alpha;
+                acc[i][2 * half + 1] *= alpha;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
+                const float2 back = __bfloat1622float2(h);
+                hi[i >> 1][(i & 1) * 2 + half] = *reinterpret_cast<const unsigned*>(&h);
+                lo[i >> 1][(i & 1) * 2 + half] = pack_bf16(p[2 * i] - back.x, p[2 * i + 1] - back.y);
+            }
+        }
+        // sums over the keys for channels 8 NT warp ..
+        const bf16* v_at = kt + (((mi & 1) << 3) + (lane & 7)) * ld + warp * 8 * NT + ((mi >> 1) << 3);
+#pragma unroll
+        for (int step = 0; step < 2; ++step)
+#pragma unroll
+            for (int i = 0; i < NT; i += 2) {
+                unsigned b[4];
+                ldmatrix_x4_trans(b[0], b[1], b[2], b[3], v_at + step * 16 * ld + i * 8);
+                mma_bf16(acc[i], hi[step], b[0], b[1]);
+                mma_bf16(acc[i + 1], hi[step], b[2], b[3]);
+                mma_bf16(acc[i], lo[step], b[0], b[1]);
+                mma_bf16(acc[i + 1], lo[step], b[2], b[3]);
+            }
+        __syncthreads();   // (the tile's place and the scores may be overwritten)
+        ask(tile + 2);
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        l[half] += __shfl_xor_sync(0xffffffffu, l[half], 1);
+        l[half] += __shfl_xor_sync(0xffffffffu, l[half], 2);
+        const int h = h0 + g + 8 * half;
+        if (h >= H) continue;
+        const int d0 = warp * 8 * NT + c2;
+        if (runs == 1) {
+            const float inv = 1.f / l[half];   // (a token always sees itself: l > 0)
+            bf16* dst = out + ((size_t)t * H + h) * C + d0;
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+                *reinterpret_cast<__nv_bfloat162*>(dst + 8 * i) = __floats2bfloat162_rn(acc[i][2 * half] * inv, acc[i][2 * half + 1] * inv);
+            continue;
+        }
+        float* dst = scratch + (((size_t)t * H + h) * runs + run) * (C + 2);
+        if (warp == 0 && (lane & 3) == 0) *reinterpret_cast<float2*>(dst) = make_float2(m[half], l[half]);
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+            *reinterpret_cast<float2*>(dst + 2 + d0 + 8 * i) = make_float2(acc[i][2 * half], acc[i][2 * half + 1]);
+    }
+}
+
+// What the kernel above takes: sizes, and 16-byte rows (8-byte pairs of the scratch, 4-byte pairs of the result).
+static bool latent_mma_takes(const void* qa, const void* pool, const void* out, const float* scratch, int C, int R) {
+    return (C == 64 || C == 128 || C == 256 || C == 512) && (C + R) % 16 == 0 &&
+           (((uintptr_t)qa | (uintptr_t)pool) & 15) == 0 && ((uintptr_t)out & 3) == 0 && ((uintptr_t)scratch & 7) == 0;
+}
+static int launch_latent_mma(const bf16* qa, const bf16* pool, const int* block_table, int max_blocks, const int* seq_of_token,
+                             const int* positions, bf16* out, float* scratch, float scale, int tokens, int H, int C, int R, int S,
+                             int runs, int window, cudaStream_t stream) {
+    const auto bytes = [](int W) {
+        return sizeof(bf16) * (size_t)(AL_HEADS + 2 * AL_TILE) * (W + 8) + sizeof(float) * AL_HEADS * (AL_TILE + 4);
+    };
+    static bool configured[4][VX_MAX_DEVICES];
+    dim3 grid(tokens, (H + AL_HEADS - 1) / AL_HEADS, runs);
+#define AL_GO(NT, SLOT)                                                                                               \
+    do {                                                                                                              \
+        if (int rc = vx_configure_smem(latent_attention_mma_kernel<NT>, bytes(1024), configured[SLOT])) return rc;     \
+        VX_LAUNCH_K(VX_K_ATTENTION, (latent_attention_mma_kernel<NT>), grid, AL_WARPS * 32, bytes(C + R), stream, qa, pool, \
+                    block_table, max_blocks, seq_of_token, positions, out, scratch, scale, H, R, S, runs, window);     \
+    } while (0)
+    if (C == 64) AL_GO(2, 0);
+    else if (C == 128) AL_GO(4, 1);
+    else if (C == 256) AL_GO(8, 2);
+    else AL_GO(16, 3);
+#undef AL_GO
+    VX_LAUNCH_CHECK();
+    return VX_OK;
+}
+// (float32 rows stay with the kernel above)
+static int launch_latent_mma(const float*, const float*, const int*, int, const int*, const int*, float*, float*, float, int, int, int, int,
+                             int, int, int, cudaStream_t) {
+    return VX_ERR_DTYPE;
+}
+
 // One block per (token, head): the runs' parts added in run order.  Every run's weight exp(m_r - M) / L is formed once, in
 // shared memory (runs <= AL_MAX_RUNS); a channel's sum then has all its reads in flight together.
 #define AL_MAX_RUNS 1024
@@ -286,7 +502,11 @@ static int launch_latent_attention(const T* qa, const T* pool, const int* block_
         VX_LAUNCH_K(VX_K_ATTENTION, (latent_attention_kernel<T, NR4>), grid, AL_WARPS * 32, smem, stream, qa, pool,    \
                     block_table, max_blocks, seq_of_token, positions, out, scratch, scale, H, C, R, S, runs, window);  \
     } while (0)
-    if (C <= 128) AL_GO(1, 0);
+    if (sizeof(T) == 2 && latent_mma_takes(qa, pool, out, scratch, C, R)) {
+        const int rc = launch_latent_mma(qa, pool, block_table, max_blocks, seq_of_token, positions, out, scratch, scale, tokens, H, C, R,
+                                         S, runs, window, stream);
+        if (rc != VX_OK) return rc;
+    } else if (C <= 128) AL_GO(1, 0);
     else if (C <= 256) AL_GO(2, 1);
     else if (C <= 512) AL_GO(4, 2);
     else AL_GO(8, 3);
