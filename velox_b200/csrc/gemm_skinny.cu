@@ -12,7 +12,7 @@
 // wait on earlier kernels (programmatic dependent launch): weights depend on
 // nothing, so they stream while the previous kernel finishes.  x is read through
 // L1/L2 (every block reads all of it).  The k order inside a tile is permuted the
-// same way for both operands, which a dot product does not notice.  The 8 warps'
+// same way for both operands, which a dot product does not notice.  The warps'
 // partial tiles are added in shared memory in warp order, so the result is the
 // same on every run and a row's result does not depend on the rows beside it.
 //

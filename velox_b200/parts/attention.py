@@ -301,7 +301,7 @@ class PagedAttention(Mixer):
             out, seqs, n = None, None, ctx.n_seqs
             if ctx.n_single and ops.decode_attention_supported(qkv.dtype, D, page, H // Hk):
                 # A mixed step: the tokens of requests that bring one token, or a few, go to the
-                # decode kernel (a warp per 256 keys), not into a query tile of their own; the
+                # decode kernel (pieces of 256 keys), not into a query tile of their own; the
                 # kernels write disjoint rows.  A decoded token's result is then the same bits
                 # whether or not prompt portions ride in its step.
                 out = torch.empty((qkv.shape[0], H * D), dtype=qkv.dtype, device=qkv.device)
