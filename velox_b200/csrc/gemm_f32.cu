@@ -166,13 +166,13 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     cluster.sync();   // (a block's sums are read until here)
 }
 
-// k's parts and their length (a multiple of 32): 256 k a part at least, eight parts at most.  The last part is not empty:
-// (parts - 1) * length < K, as length < K / parts + 32 and K >= 256 parts.
+// k's parts and their length (a multiple of 32), eight parts at most: of 256 k at least from 1,024 on, of 64 below, where the
+// chains of a sum would else be as long as there (narrow models, whose errors nothing averages out).  No part is empty.
 static void gf_parts(int K, int* parts, int* len) {
-    int p = K / 256;
+    int p = K / (K >= 1024 ? 256 : 64);
     p = p < 1 ? 1 : (p > GF32_MAX_PARTS ? GF32_MAX_PARTS : p);
-    *parts = p;
     *len = ((K + p - 1) / p + GF32_BK - 1) / GF32_BK * GF32_BK;
+    *parts = (K + *len - 1) / *len;
 }
 
 struct GfCall {
