@@ -333,6 +333,39 @@ def test_sample_temperature_and_top_p(vocab):
     assert ops().sample(x, t(temps), t(tops), t(us)).tolist() == got
 
 
+@pytest.mark.parametrize("vocab", [25000, 60001, 151936, 262144])
+def test_sample_gives_the_same_token_in_every_form(vocab):
+    """On 148 SMs 1 and 12 rows are drawn by eight blocks a row, 20 by four, 40 by two and 80 by one (fewer where the vocabulary is
+    small), with the row's parts kept in shared memory or, where they don't fit, read again.  Every form adds in the same order, so a
+    row's token is the same in all of them, bit for bit, and each form is held against float64.  60,001: rows that begin on no 16-byte
+    address.  Ties of the maximum lie in different blocks' parts."""
+    from velox_b200.sampling.rng import uniform
+    rows = 80
+    x = torch.randn(rows, vocab, generator=torch.Generator().manual_seed(vocab)) * 2.0
+    for r in range(0, rows, 4):
+        x[r, [vocab // 3 + r, vocab - 1 - r]] = 20.0   # (the first wins)
+    temps = [(0.0, 0.8, 1.0, 1.3)[r % 4] for r in range(rows)]
+    tops = [(1.0, 0.9, 0.5, 0.0, 0.999)[r % 5] for r in range(rows)]
+    us = [uniform(7, 0, r) for r in range(rows)]
+    x, t = x.to(DEV), lambda v: torch.tensor(v, dtype=torch.float32, device=DEV)
+    draw = lambda n: ops().sample(x[:n], t(temps[:n]), t(tops[:n]), t(us[:n])).tolist()
+    got = draw(rows)
+    for n in (1, 12, 20, 40):
+        assert draw(n) == got[:n], n
+        assert ops().sample(x[:n]).tolist() == [P.greedy(v) for v in f64(x[:n])], n
+    assert ops().sample(x).tolist() == [P.greedy(v) for v in f64(x)]
+    assert all(got[r] == vocab // 3 + r for r in range(0, rows, 4))
+    for r in range(1, 40):
+        if temps[r] == 0.0:
+            continue
+        p = P.probabilities(f64(x[r]), temps[r], tops[r])
+        want = P.sample_from(p, us[r])
+        if got[r] != want:   # only where u falls on a boundary of the cumulative distribution (as above)
+            c = np.cumsum(p)
+            lo, hi = sorted((got[r], want))
+            assert p[got[r]] > 0 and abs(c[lo] - us[r]) < 1e-5 * max(1, hi - lo), (r, got[r], want)
+
+
 def test_sample_top_p_keeps_only_the_nucleus():
     x = torch.full((1, 300), -5.0, device=DEV)
     x[0, [10, 20, 30]] = torch.tensor([3.0, 2.0, 1.0], device=DEV)

@@ -138,6 +138,8 @@ template <int BLOCKS, bool KEPT>
 __global__ void __cluster_dims__(BLOCKS, 1, 1) __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
               const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+    cg::cluster_group cluster = cg::this_cluster();
+    if (BLOCKS > 1) cluster.barrier_arrive();   // (here this block's shared memory exists: waited for before the first store into another's)
     pdl_wait();
     pdl_trigger();
     constexpr int STRETCHES = SAMPLE_WARPS / BLOCKS, BUFFERS = BLOCKS > 1 ? 2 : 1;
@@ -152,13 +154,12 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
     __shared__ float group_mass[STRETCHES][SAMPLE_GROUPS];
     __shared__ float best_of[BLOCKS];
     __shared__ int best_i_of[BLOCKS], cand_of[BLOCKS], last_of[BLOCKS];
-    cg::cluster_group cluster = cg::this_cluster();
     // (a row of one block: plain barriers, its own shared memory)
     auto sync = [&]() { if (BLOCKS > 1) cluster.sync(); else __syncthreads(); };
     const int rank = BLOCKS > 1 ? (int)cluster.block_rank() : 0;
     const int r = blockIdx.x / BLOCKS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* x = logits + (size_t)r * ld;
-    // The row is cut into 32 stretches of `groups` groups of 32 elements; a block has four of them.
+    // The row is cut into 32 stretches of `groups` groups of 32 elements; a block has 32 / BLOCKS of them.
     const int groups = ((V + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) >> 5;   // at most SAMPLE_GROUPS
     const int b0 = min(rank * STRETCHES * groups * 32, V), b1 = min((rank + 1) * STRETCHES * groups * 32, V);
 
@@ -173,6 +174,7 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
     const float* slice = KEPT ? slice_s : x + b0;   // the block's part of the row
     block_argmax(best, best_i, sv, si);
     if (BLOCKS > 1) {
+        cluster.barrier_wait();   // every block of the cluster has started: another's shared memory may be written
         if (tid < BLOCKS) {   // every block gets every block's
             sample_at<BLOCKS>(cluster, best_of, tid)[rank] = best;
             sample_at<BLOCKS>(cluster, best_i_of, tid)[rank] = best_i;
