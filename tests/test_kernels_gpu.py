@@ -285,6 +285,28 @@ def test_gemm_float32_tiles_and_parts(N, K, pad):
         assert torch.equal(ops().gemm_nt_simt(a[130 - M:], w, bias), whole[130 - M:]), M
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (12, 1000, 777), (99, 4096, 1024), (3, 40000, 300)])
+def test_gemm_float32_waits_for_a_w_that_was_just_written(M, N, K):
+    """W written by the kernel launched just before, in memory that holds NaN until then: the products (plain, per head, of a batch)
+    see it whole, as they do when the GPU was waited for in between; with `w_ready` and a W that is, the same bits."""
+    a = rnd((M, K), torch.float32, 1)
+    for seed in range(4):
+        x = rnd((N, 2 * K), torch.float32, 10 + seed)
+        w = ops().gated_act(x, "silu")
+        torch.cuda.synchronize()
+        want = ops().gemm_nt_simt(a, w, w_ready=True)
+
+        def just_written():
+            torch.full((N, K), float("nan"), device=DEV)   # (given back at once: the block that the next result of this size takes)
+            return ops().gated_act(x, "silu")
+
+        assert torch.equal(ops().gemm_nt_simt(a, just_written()), want)
+        out = torch.empty((M, 1, N), device=DEV)
+        ops().gemm_heads(a.view(M, 1, K), just_written().view(1, N, K), out)
+        assert torch.equal(out[:, 0], want)
+        assert torch.equal(ops().gemm_members(a.view(1, M, K), just_written().view(1, N, K))[0], want)
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,K", [(1, 53, 72), (37, 64, 16), (130, 136, 104), (64, 384, 96), (8, 4096, 4096)])
 def test_gemm_bf16(M, N, K, out_dtype):

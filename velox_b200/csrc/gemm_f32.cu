@@ -59,7 +59,7 @@ __device__ __forceinline__ void gf_load(float* dst, const float* __restrict__ X,
 template <int TM, int TN, int TY, int TX, bool VEC, bool SPLIT>
 __global__ void __launch_bounds__(TX* TY)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C, int M,
-                int N, int K, int lda, int ldw, int ldc, long long sa, long long sw, long long sc, int parts, int part_len) {
+                int N, int K, int lda, int ldw, int ldc, long long sa, long long sw, long long sc, int parts, int part_len, int w_ready) {
     constexpr int BM = TM * TY, BN = TN * TX, NT = TX * TY, STAGE = (BM + BN) * GF32_LD;
     extern __shared__ __align__(16) float gf_smem[];
     A += (size_t)blockIdx.z * sa;
@@ -75,12 +75,16 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     constexpr int WX = TX / LX;   // warps side by side
     const int tx = (warp % WX) * LX + lane % LX, ty = (warp / WX) * (32 / LX) + lane / LX;
 
-    // W depends on no earlier kernel: its first tiles are asked for before the wait
+    auto ask_w = [&]() {
 #pragma unroll
-    for (int s = 0; s < GF32_STAGES - 1; ++s)
-        if (s < chunks) gf_load<BN, NT, VEC>(gf_smem + s * STAGE + BM * GF32_LD, W, n0, N, ldw, kbeg + s * GF32_BK, kend);
+        for (int s = 0; s < GF32_STAGES - 1; ++s)
+            if (s < chunks) gf_load<BN, NT, VEC>(gf_smem + s * STAGE + BM * GF32_LD, W, n0, N, ldw, kbeg + s * GF32_BK, kend);
+    };
+    // a W that the caller calls ready depends on no earlier kernel: its first tiles are asked for before the wait
+    if (w_ready) ask_w();
     pdl_wait();
     pdl_trigger();
+    if (!w_ready) ask_w();
 #pragma unroll
     for (int s = 0; s < GF32_STAGES - 1; ++s) {
         if (s < chunks) gf_load<BM, NT, VEC>(gf_smem + s * STAGE, A, m0, M, lda, kbeg + s * GF32_BK, kend);
@@ -180,6 +184,7 @@ struct GfCall {
     float* C;
     int M, N, K, lda, ldw, ldc, batch;
     long long sa, sw, sc;
+    int w_ready;
 };
 
 template <int TM, int TN, int TY, int TX, bool VEC, bool SPLIT>
@@ -209,7 +214,8 @@ static int gf_launch(const GfCall& g, int parts, int len, cudaStream_t stream) {
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, g.A, g.W, g.bias, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc, g.sa, g.sw, g.sc, parts, len);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, g.A, g.W, g.bias, g.C, g.M, g.N, g.K, g.lda, g.ldw, g.ldc, g.sa, g.sw, g.sc, parts, len,
+                                       g.w_ready);
     if (e != cudaSuccess) return (int)e;
     VX_LAUNCH_CHECK();
     return VX_OK;
@@ -244,8 +250,8 @@ static int gf_choose(const GfCall& g, bool vec, long long sms, cudaStream_t stre
 // A product of at least 8 tiles an SM keeps k whole (151,936 columns: 162 against 181 microseconds at one row); with fewer, the
 // parts of k go to the blocks of a cluster (4096 x 1024: 38 whole, 11 cut).
 int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc, int batch,
-                long long sa, long long sw, long long sc, cudaStream_t stream) {
-    const GfCall g = {A, W, bias, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc};
+                long long sa, long long sw, long long sc, int w_ready, cudaStream_t stream) {
+    const GfCall g = {A, W, bias, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready};
     // rows that begin on 16-byte addresses are fetched 16 bytes at a time, others four
     const bool vec = !((lda | ldw) & 3) && !((sa | sw) & 3) && !((((uintptr_t)A) | ((uintptr_t)W)) & 15);
     static int sms_cache[VX_MAX_DEVICES];

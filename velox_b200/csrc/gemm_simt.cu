@@ -76,15 +76,18 @@ gemm_nt_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const fl
 
 // in_dtype: element type of A and W; out_dtype: element type of C.
 // A batch of `batch` products: member z reads A + z sa, W + z sw and writes C + z sc (strides in elements).
-extern "C" int vx_gemm_nt_simt_batched(const void* A, const void* W, const float* bias, void* C, int M, int N,
-                                       int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
-                                       long long sc, int in_dtype, int out_dtype, cudaStream_t stream) {
+// `w_ready`: W (a model's weights, say) is not something the kernel launched just before this one writes; the float32 product
+// then asks for its first tiles before it waits for that kernel.
+extern "C" int vx_gemm_nt_simt_ready(const void* A, const void* W, const float* bias, void* C, int M, int N,
+                                     int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
+                                     long long sc, int in_dtype, int out_dtype, int w_ready, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return VX_OK;
     if (K <= 0 || lda < K || ldw < K || ldc < N) return VX_ERR_SHAPE;
     dim3 grid((N + GS_BN - 1) / GS_BN, (M + GS_BM - 1) / GS_BM, batch);
     if (grid.y > 65535 || batch > 65535) return VX_ERR_LIMIT;
     if (in_dtype == VX_F32 && out_dtype == VX_F32)
-        return vx_gemm_f32((const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
+        return vx_gemm_f32((const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready,
+                           stream);
     if (in_dtype == VX_BF16 && out_dtype == VX_BF16)
         VX_LAUNCH_K(VX_K_GEMM, (gemm_nt_simt_kernel<bf16, bf16>), grid, 256, 0, stream, (const bf16*)A, (const bf16*)W, bias, (bf16*)C, M, N, K, lda, ldw, ldc, sa, sw, sc);
     else if (in_dtype == VX_BF16 && out_dtype == VX_F32)
@@ -93,6 +96,12 @@ extern "C" int vx_gemm_nt_simt_batched(const void* A, const void* W, const float
         return VX_ERR_DTYPE;
     VX_LAUNCH_CHECK();
     return VX_OK;
+}
+
+extern "C" int vx_gemm_nt_simt_batched(const void* A, const void* W, const float* bias, void* C, int M, int N,
+                                       int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
+                                       long long sc, int in_dtype, int out_dtype, cudaStream_t stream) {
+    return vx_gemm_nt_simt_ready(A, W, bias, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, in_dtype, out_dtype, 0, stream);
 }
 
 extern "C" int vx_gemm_nt_simt(const void* A, const void* W, const float* bias, void* C, int M, int N,

@@ -120,6 +120,7 @@ def _declare(lib) -> None:
         "vx_moe_gather_rows": [P, I, P, I, P, I, I, P],
         "vx_moe_gemm_tcgen05": [P, P, P, I, I, I, I, I, I, I, I, P, P, I, P, P],
         "vx_gemm_nt_simt": [P, P, P, P, I, I, I, I, I, I, I, I, P],
+        "vx_gemm_nt_simt_ready": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, I, P],
         "vx_gemm_tcgen05": [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_tcgen05_pair": [P, P, P, P, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_skinny": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P],
@@ -1009,9 +1010,11 @@ def paged_prefill_attention_tc(q: torch.Tensor, q_row_stride: int, k_pool, v_poo
     return out
 
 
-def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """a [M,K] times w [N,K] transposed, float32 multiply-adds on the CUDA cores.  `w` is a weight: not
-    something the kernel launched just before this one writes (its first tiles are fetched before the wait for that kernel)."""
+def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None,
+                 w_ready: bool = False) -> torch.Tensor:
+    """a [M,K] times w [N,K] transposed, float32 multiply-adds on the CUDA cores.  `w_ready` says that `w` is not something the
+    kernel launched just before this one writes (a model's weights never are): its first tiles may then be fetched before the wait for
+    that kernel."""
     _dev(a, w, bias)
     _need(a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1], "gemm: a [M,K], w [N,K]")
     _need(a.stride(1) == 1 and w.stride(1) == 1 and a.dtype == w.dtype, "gemm: rows contiguous, one element type")
@@ -1021,18 +1024,19 @@ def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optiona
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm: float32 bias of N elements")
     out = torch.empty((m, n), dtype=out_dtype, device=a.device)
-    _check(library().vx_gemm_nt_simt(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0), w.stride(0), n,
-                                     dtype_code(a.dtype), dtype_code(out_dtype), _stream()), "gemm_nt_simt")
+    _check(library().vx_gemm_nt_simt_ready(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0), w.stride(0), n, 1, 0, 0, 0,
+                                           dtype_code(a.dtype), dtype_code(out_dtype), 1 if w_ready else 0, _stream()), "gemm_nt_simt")
     return out
 
 
 GEMM_HEADS_FEW_ROWS = 8   # rows up to which the products per head take the kernel that gives every output column a warp
 
 
-def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_ready: bool = False) -> torch.Tensor:
     """One product per head: out[:, h, :] = a[:, h, :] w[h]^T with a [M, H, K], w [H, N, K] (contiguous), out [M, H, N];
     `a` and `out` may be views into wider rows (their last dimension contiguous).  float32 multiply-adds (in float32, the
-    order of a sum is fixed by K alone, whatever the number of rows; bfloat16 steps of up to 8 rows take a kernel of their own)."""
+    order of a sum is fixed by K alone, whatever the number of rows; bfloat16 steps of up to 8 rows take a kernel of their own, which
+    always reads `w` as one that is ready).  `w_ready`: see `gemm_nt_simt`."""
     _dev(a, w, out)
     _need(a.dim() == 3 and w.dim() == 3 and out.dim() == 3 and w.is_contiguous() and a.shape[1] == w.shape[0]
           and a.shape[2] == w.shape[2] and out.shape == (a.shape[0], w.shape[0], w.shape[1]), "gemm_heads: a [M,H,K], w [H,N,K], out [M,H,N]")
@@ -1044,9 +1048,9 @@ def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Ten
         _check(library().vx_gemm_few_rows_batched(_ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), k, out.stride(0), h, a.stride(1),
                                                   n * k, out.stride(1), dtype_code(out.dtype), _stream()), "gemm_few_rows_heads")
         return out
-    _check(library().vx_gemm_nt_simt_batched(_ptr(a), _ptr(w), None, _ptr(out), m, n, k, a.stride(0), k, out.stride(0), h,
-                                             a.stride(1), n * k, out.stride(1), dtype_code(a.dtype), dtype_code(out.dtype),
-                                             _stream()), "gemm_nt_simt_heads")
+    _check(library().vx_gemm_nt_simt_ready(_ptr(a), _ptr(w), None, _ptr(out), m, n, k, a.stride(0), k, out.stride(0), h,
+                                           a.stride(1), n * k, out.stride(1), dtype_code(a.dtype), dtype_code(out.dtype),
+                                           1 if w_ready else 0, _stream()), "gemm_nt_simt_heads")
     return out
 
 
@@ -1785,9 +1789,10 @@ def gemm_inputs(xs: torch.Tensor, w: torch.Tensor, seg_rows: int, out_dtype: tor
     return out
 
 
-def gemm_members(xs: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
+def gemm_members(xs: torch.Tensor, ws: torch.Tensor, w_ready: bool = False) -> torch.Tensor:
     """A batch of products of one shape: out[i] = xs[i] ws[i]^T with xs [n, M, K], ws [n, N, K] (contiguous).  float32:
-    multiply-adds on the CUDA cores, every sum over k in ascending order; bfloat16: the library product."""
+    multiply-adds on the CUDA cores, the order of a sum fixed by K alone; bfloat16: the library product.  `w_ready`: see
+    `gemm_nt_simt`."""
     _dev(xs, ws)
     _need(xs.dim() == 3 and ws.dim() == 3 and xs.is_contiguous() and ws.is_contiguous() and xs.dtype == ws.dtype
           and xs.shape[0] == ws.shape[0] and xs.shape[2] == ws.shape[2], "gemm_members: xs [n, M, K], ws [n, N, K] of one element type")
@@ -1796,9 +1801,9 @@ def gemm_members(xs: torch.Tensor, ws: torch.Tensor) -> torch.Tensor:
         _full_precision_sums()
         return torch.bmm(xs, ws.transpose(1, 2))
     out = torch.empty((n, m, ws.shape[1]), dtype=xs.dtype, device=xs.device)
-    _check(library().vx_gemm_nt_simt_batched(_ptr(xs), _ptr(ws), None, _ptr(out), m, ws.shape[1], k, k, k, ws.shape[1], n, m * k,
-                                             ws.shape[1] * k, m * ws.shape[1], dtype_code(xs.dtype), dtype_code(out.dtype), _stream()),
-           "gemm_members")
+    _check(library().vx_gemm_nt_simt_ready(_ptr(xs), _ptr(ws), None, _ptr(out), m, ws.shape[1], k, k, k, ws.shape[1], n, m * k,
+                                           ws.shape[1] * k, m * ws.shape[1], dtype_code(xs.dtype), dtype_code(out.dtype),
+                                           1 if w_ready else 0, _stream()), "gemm_members")
     return out
 
 

@@ -192,9 +192,9 @@ class LatentAttention(Mixer):
         qa = torch.empty((t, H, C + R), dtype=x.dtype, device=x.device)   # folded queries: [W_uk^T q | rotated part]
         ops.latent_prep(down, q, qa, self.norm_weight, self.eps, self.rotary[0], interleaved,
                         ctx.positions, slots, cache.pages, H, D, R, C)
-        ops.gemm_heads(q.view(t, H, D + R)[:, :, :D], self.uk_t, qa[:, :, :C])
+        ops.gemm_heads(q.view(t, H, D + R)[:, :, :D], self.uk_t, qa[:, :, :C], w_ready=True)
         latent = ops.latent_attention(qa, cache.pages, group.block_table, ctx.seq_of_token, ctx.positions, self.scale, H, C, R,
                                       max_kv=ctx.max_kv, window=self.window)
         o = torch.empty((t, H, Dv), dtype=x.dtype, device=x.device)
-        ops.gemm_heads(latent, self.uv, o)
+        ops.gemm_heads(latent, self.uv, o, w_ready=True)
         return self.out(self._gated(o.view(t, H * Dv), x))

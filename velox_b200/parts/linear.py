@@ -18,9 +18,10 @@ from ..csrc import ops
 
 def matmul(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+    """`weight` belongs to a model: nothing that a kernel of the step writes (the products may fetch it ahead of earlier kernels)."""
     out_dtype = out_dtype or x.dtype
     if x.dtype == torch.float32:
-        return ops.gemm_nt_simt(x, weight, bias, out_dtype)
+        return ops.gemm_nt_simt(x, weight, bias, out_dtype, w_ready=True)
     return ops.gemm_bf16(x, weight, bias, out_dtype)
 
 

@@ -91,7 +91,7 @@ class WkvMixer(Mixer):
             x = ops.gemm_inputs(mixed, self.proj, HD, torch.float32)   # [tokens, r | k | v | g | w1]
             low, gate, cols = x[:, 4 * HD:], x[:, 3 * HD:4 * HD], (0, HD, 2 * HD)
         else:
-            x = ops.gemm_members(mixed[:4], self.proj[:4 * HD].view(4, HD, self.hidden_size))   # [r, k, v, g][tokens, H D]
+            x = ops.gemm_members(mixed[:4], self.proj[:4 * HD].view(4, HD, self.hidden_size), w_ready=True)   # [r, k, v, g][tokens, H D]
             low, gate, cols = matmul(mixed[4], self.proj[4 * HD:], None, torch.float32), x[3], (0, tokens * HD, 2 * tokens * HD)
         log_decay = ops.low_rank_decay(low, self.decay_up, self.decay_bias)
         o = ops.linear_attention_walk(x, *cols, cache.parts[1].state, ctx.cu_seqlens, ctx.state_slots, ctx.n_seqs, H, D, D,
