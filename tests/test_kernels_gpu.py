@@ -1,4 +1,5 @@
 """Each kernel alone against its plain reference, at sizes other than the models'."""
+import ctypes
 import math
 
 import numpy as np
@@ -488,6 +489,27 @@ def test_decode_attention_forms_agree(D, H, Hk, window, S):
     close(first, want, torch.bfloat16)
     for shape in (1, 8):
         assert torch.equal(run(shape), first), shape
+
+
+@pytest.mark.parametrize("D,H,Hk,window", [(128, 8, 2, 0), (64, 16, 1, 0), (128, 6, 6, 333)])
+def test_decode_attention_in_pieces_of_any_number_of_tiles(D, H, Hk, window):
+    """The C entry points take 1 to 32 tiles of 16 keys a piece: even numbers, odd ones (whose last sub-piece is half of one, with
+    another piece's keys behind it) and more tiles than a request has."""
+    S, lens = 16, [600, 16, 33, 257, 40, 5]
+    q, kp, vp, bt, sot, pos, want = paged_case(torch.bfloat16, [(n - 1, 1) for n in lens], H, Hk, D, S, window, seed=19)
+    stream, no_alloc = torch.cuda.current_stream().cuda_stream, ops().library().vx_paged_decode_attention_static
+    ptr, num, real = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    no_alloc.argtypes = [ptr, num, ptr, ptr, ptr, num, ptr, ptr, ptr, num, ptr, num, real] + [num] * 7 + [ptr]
+    for tiles in (1, 2, 3, 5, 15, 16, 31, 32):
+        pieces = -(-(-(-max(lens) // 16)) // tiles) + (1 if window else 0)
+        scratch = torch.full((len(lens) * H * pieces * (D + 2),), float("nan"), device=DEV)
+        args = (q.data_ptr(), H * D, kp.data_ptr(), vp.data_ptr(), bt.data_ptr(), bt.shape[1], None, sot.data_ptr(), pos.data_ptr())
+        rest = (H * D, 1 / math.sqrt(D), window, len(lens), H, Hk, D, S, tiles)
+        out, static = torch.zeros((len(lens), H * D), dtype=torch.bfloat16, device=DEV), torch.zeros((len(lens), H * D), dtype=torch.bfloat16, device=DEV)
+        assert ops().library().vx_paged_decode_attention(*args, scratch.data_ptr(), pieces, out.data_ptr(), *rest, 1, stream) == 0
+        close(out, want, torch.bfloat16, what="%d tiles a piece" % tiles)
+        assert no_alloc(*args, pieces, static.data_ptr(), *rest, stream) == 0
+        assert torch.equal(static, out), tiles
 
 
 def test_decode_attention_shows_a_score_that_is_no_number():

@@ -192,8 +192,10 @@ __device__ __forceinline__ void dec_sub_piece(DecPart<D, NG>& part, const unsign
 #pragma unroll
             for (int n = 0; n < NG; ++n) mma_bf16(s[t][n], a, qf[kk][n][0], qf[kk][n][1]);
         }
-    // scale, mask, softmax over the sub-piece's keys (base 2)
-    const bool inside = key0 >= start && key0 + 16 * DEC_SUB <= kv_len;
+    // scale, mask, softmax over the sub-piece's keys (base 2); keys from key_end on are past the last, or another piece's (a piece
+    // of an odd number of tiles ends with a sub-piece of one)
+    const int key_end = min(kv_len, key0 + (tiles << 4));
+    const bool inside = key0 >= start && key0 + 16 * DEC_SUB <= key_end;
     unsigned p[DEC_SUB][NG][2];   // [keys lane/4 .. | + 8], two heads each, then transposed: two keys of one head
 #pragma unroll
     for (int n = 0; n < NG; ++n) {
@@ -208,7 +210,7 @@ __device__ __forceinline__ void dec_sub_piece(DecPart<D, NG>& part, const unsign
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const int key = kc + 16 * t + ((c >> 1) << 3);
-                    if (key < start || key >= kv_len) s[t][n][c] = -INFINITY;
+                    if (key < start || key >= key_end) s[t][n][c] = -INFINITY;
                 }
         }
         float mx[2], less[2];
