@@ -418,7 +418,7 @@ def test_bounded_logits_and_products_per_head():
 def test_latent_attention_on_the_tensor_cores(C, R, H, window, max_kv):
     """bfloat16 rows of the sizes that go to the tensor-core kernel, with and without runs: lengths around a tile's edges
     (32 rows), widths of an odd number of 16 elements, heads that do not fill a block, a window.  The result is rounded
-    to bfloat16 (2^-9); weights in two bfloat16 halves (2^-17), float32 sums and the scores' rounding
+    to bfloat16 (2^-9); float32 sums and the scores' rounding
     (2^-24 of sums up to 40 times the score) are well below: 2^-8 of a row's largest value."""
     from velox_b200.csrc import ops
     lens, S = [1, 31, 32, 33, 64, 65, 270, 600], 16
@@ -442,3 +442,26 @@ def test_latent_attention_on_the_tensor_cores(C, R, H, window, max_kv):
                                max_kv=max_kv, window=window).cpu().double()
     err = (got - want).abs().amax(-1) / want.abs().amax(-1)
     assert torch.isfinite(got).all() and err.max() <= 2.0 ** -8, err.max()
+
+
+@pytest.mark.parametrize("C", [64, 128, 256, 512])
+def test_latent_attention_keeps_float32_weights(C):
+    """Values that cancel but for a difference of 2^-12 between two softmax weights of 0.2 to 0.7, beside a key of weight 1 and value 0:
+    the result is that difference.  Weights and sums rounded to 24 bits leave it within some 2^-10 of itself, its own rounding 2^-9: 2^-7.
+    (Weights of 16 bits: off by up to 2^-18 of 2^-12.5, 2^-5.5.)"""
+    from velox_b200.csrc import ops
+    H, R, S = 16, 16, 16
+    rows = torch.zeros(1, 1, S, C + R)
+    rows[..., 0, 1:3, C] = -1.0      # the two keys score -x of a head's query ...
+    rows[..., 0, 2, C + 1] = -1.0    # ... and the second 2^-12 less
+    rows[..., 0, 1, :C], rows[..., 0, 2, :C] = 1.0, -1.0
+    qa = torch.zeros(1, H, C + R)
+    qa[0, :, C] = torch.linspace(0.4, 1.6, H).bfloat16().float()
+    qa[0, :, C + 1] = 2.0 ** -12
+    x = qa[0, :, C].double()
+    w1, w2 = torch.exp(-x), torch.exp(-x - 2.0 ** -12)
+    want = ((w1 - w2) / (1 + w1 + w2))[:, None]
+    t = lambda v, dtype=torch.bfloat16: v.to(dtype).to(DEV)
+    got = ops.latent_attention(t(qa), t(rows), torch.zeros(1, 1, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV),
+                               torch.full((1,), 2, dtype=torch.int32, device=DEV), 1.0, H, C, R).cpu().double()[0]
+    assert ((got - want).abs() <= 2.0 ** -7 * want).all(), ((got - want).abs() / want).max()

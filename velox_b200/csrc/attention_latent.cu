@@ -245,11 +245,14 @@ latent_attention_kernel(const T* __restrict__ qa, const T* __restrict__ pool, co
 // block's sixteen heads are the 16 rows, keys (for the scores) or channels (for the sums) the columns.  Rows stay bfloat16 in
 // shared memory (cp.async, two tiles in flight); a warp forms the scores of 8 of a tile's 32 keys for all heads, every warp takes
 // the softmax of all of them (the same operations in the same order), and adds up a quarter of the channels.  The weights go to
-// the tensor cores in two bfloat16 parts, w = hi + lo up to 2^-17 of w, far below the result's own rounding; sums are float32.
+// the tensor cores whole, each as the sum of three bfloat16 parts of 8 bits of its 24 (a part may be zero, so a value that is infinite
+// gives NaN); sums are float32, a tile's on the tensor cores, the tiles' on the CUDA cores.
 // A decode step's blocks have a tile or two each, and what bounds them is the length of the chain from one to the next: the
 // kernel above takes 17 us a tile (144 steps of five shared-memory reads a score, then 32 rows one after another).
-// With their joins, us: 8 requests of 270 keys, 16 heads, C 512, R 64 34.5 -> 13.9; one of 4,000 63 -> 22; 4 of 2,000, 40 heads 70 -> 27; 64 of
-// 1,000 158 -> 41; error against 64 bits the same to four digits (0.00165 of the result, its rounding).
+// With their joins, us, that kernel and this: 8 requests of 270 keys, 16 heads, C 512, R 64 33.4 -> 13.2; one of 4,000 63 -> 22; 4 of 2,000,
+// 40 heads 70 -> 28; 64 of 1,000 162 -> 45.  Error of the sums against 64 bits, before they are rounded to bfloat16, same order: 3.0e-7 -> 3.3e-7,
+// 6.1e-7 -> 3.8e-7, 4.9e-7 -> 3.5e-7, 4.0e-7 -> 3.5e-7; with values that cancel 1e-5 to 2e-5 -> 4e-6 to 5e-6.  (Weights in two parts,
+// one accumulator over all tiles: 3 % faster, but 2e-6 to 4e-6 and 4e-5 to 8e-5.)
 template <int NT>   // n-tiles of 8 channels a warp: C / 32
 __global__ void __launch_bounds__(AL_WARPS * 32)
 latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict__ pool, const int* __restrict__ block_table,
@@ -343,8 +346,9 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
             }
         }
         __syncthreads();
-        // weights of all 32 keys, as A operands of two steps of 16 keys: [step][A register] two keys each
-        unsigned hi[2][4], lo[2][4];
+        // weights of all 32 keys, as A operands of two steps of 16 keys: [part][step][A register] two keys each
+        unsigned wa[3][2][4];
+        float alpha[2];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const float* row = s_s + (g + 8 * half) * SLD + c2;
@@ -361,7 +365,7 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
             const float m_new = fmaxf(m[half], mx), less = m_new == -INFINITY ? 0.f : m_new;
-            const float alpha = expf(m[half] - less);   // m = -inf before the first tile: 0
+            alpha[half] = expf(m[half] - less);   // m = -inf before the first tile: 0
             m[half] = m_new;
             float sum = 0.f;
 #pragma unroll
@@ -369,33 +373,42 @@ latent_attention_mma_kernel(const bf16* __restrict__ qa, const bf16* __restrict_
                 p[i] = expf(p[i] - less);
                 sum += p[i];
             }
-            l[half] = l[half] * alpha + sum;
-#pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                acc[i][2 * half] *= alpha;
-                acc[i][2 * half + 1] *= alpha;
-            }
+            l[half] = l[half] * alpha[half] + sum;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
-                const float2 back = __bfloat1622float2(h);
-                hi[i >> 1][(i & 1) * 2 + half] = *reinterpret_cast<const unsigned*>(&h);
-                lo[i >> 1][(i & 1) * 2 + half] = pack_bf16(p[2 * i] - back.x, p[2 * i + 1] - back.y);
+#pragma unroll
+                for (int part = 0; part < 3; ++part) {   // (what a part leaves is exact in float32)
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(p[2 * i], p[2 * i + 1]);
+                    const float2 back = __bfloat1622float2(h);
+                    wa[part][i >> 1][(i & 1) * 2 + half] = *reinterpret_cast<const unsigned*>(&h);
+                    p[2 * i] -= back.x;
+                    p[2 * i + 1] -= back.y;
+                }
             }
         }
         // sums over the keys for channels 8 NT warp ..
         const bf16* v_at = kt + (((mi & 1) << 3) + (lane & 7)) * ld + warp * 8 * NT + ((mi >> 1) << 3);
 #pragma unroll
-        for (int step = 0; step < 2; ++step)
+        for (int i = 0; i < NT; i += 2) {
+            // (a tile's sums start from zero and are added by the CUDA cores: the tensor cores cut off what an addition does not hold,
+            // which over a long row of tiles came to 1e-5 of the sum)
+            float t0[4] = {0.f, 0.f, 0.f, 0.f}, t1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int i = 0; i < NT; i += 2) {
+            for (int step = 0; step < 2; ++step) {
                 unsigned b[4];
                 ldmatrix_x4_trans(b[0], b[1], b[2], b[3], v_at + step * 16 * ld + i * 8);
-                mma_bf16(acc[i], hi[step], b[0], b[1]);
-                mma_bf16(acc[i + 1], hi[step], b[2], b[3]);
-                mma_bf16(acc[i], lo[step], b[0], b[1]);
-                mma_bf16(acc[i + 1], lo[step], b[2], b[3]);
+#pragma unroll
+                for (int part = 0; part < 3; ++part) {
+                    mma_bf16(t0, wa[part][step], b[0], b[1]);
+                    mma_bf16(t1, wa[part][step], b[2], b[3]);
+                }
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[i][j] = fmaf(acc[i][j], alpha[j >> 1], t0[j]);
+                acc[i + 1][j] = fmaf(acc[i + 1][j], alpha[j >> 1], t1[j]);
+            }
+        }
         __syncthreads();   // (the tile's place and the scores may be overwritten)
         ask(tile + 2);
     }
