@@ -55,21 +55,36 @@ def library():
 _CALLS = None
 
 
+class _NoCalls:
+    """Stands for the call module where it cannot be had: every operation is left to its wrapper."""
+
+    def __getattr__(self, name):
+        return _left_to_the_wrapper
+
+
+def _left_to_the_wrapper(*args):
+    return None
+
+
 def _calls():
-    """The module of the operations that are called most (`calls/calls.cpp`); built first if needed."""
+    """The module of the operations that are called most (`calls/calls.cpp`); built first if needed.  Where it cannot be built or
+    loaded (it needs Python's headers and torch's, which the kernel library does not) the wrappers below call the same kernels by
+    themselves, some 10 us later a call; a warning says so."""
     global _CALLS
     if _CALLS is None:
         library()
         import importlib.machinery
         import importlib.util
-        path = _build.build_calls()
-        loader = importlib.machinery.ExtensionFileLoader("velox_b200_calls", path)
         try:
+            path = _build.build_calls()
+            loader = importlib.machinery.ExtensionFileLoader("velox_b200_calls", path)
             module = importlib.util.module_from_spec(importlib.util.spec_from_loader("velox_b200_calls", loader))
             loader.exec_module(module)
             module.bind(_LIB._name)
-        except (ImportError, OSError) as e:
-            raise KernelError("the call module %s could not be loaded: %s" % (path, e))
+        except (_build.BuildError, ImportError, OSError) as e:
+            import warnings
+            warnings.warn("the call module cannot be had, kernels are called through ctypes: %s" % e, RuntimeWarning, stacklevel=3)
+            module = _NoCalls()
         _CALLS = module
     return _CALLS
 
@@ -280,9 +295,10 @@ def add_rmsnorm(residual: torch.Tensor, delta: Optional[torch.Tensor], weight: t
     Without `rows` the sum is written back into `residual` (if there is a delta
     and `update_residual`).  With `rows` (int32 indices) only those rows are
     read, and the sums go to `residual_out` if given."""
-    out = (_CALLS or _calls()).add_rmsnorm(residual, delta, weight, eps, out_dtype, rows, residual_out, update_residual)
-    if out is not None:
-        return _called(out, "add_rmsnorm")
+    if residual.is_cuda:
+        out = (_CALLS or _calls()).add_rmsnorm(residual, delta, weight, eps, out_dtype, rows, residual_out, update_residual)
+        if out is not None:
+            return _called(out, "add_rmsnorm")
     _dev(residual, delta, weight, rows)
     _need(residual.dtype == torch.float32 and residual.is_contiguous(), "add_rmsnorm: float32 contiguous residual")
     _need(weight.dtype == torch.float32, "add_rmsnorm: float32 weight")
@@ -322,7 +338,7 @@ def gated_act(gate_up: torch.Tensor, activation: str, block: int = 0,
     """act(gate) * up.  block == 0: rows are [all gates | all ups]; block > 0: rows
     are tiles of `block` gates followed by their `block` ups.  float32 input may give a
     bfloat16 result (`out_dtype`)."""
-    if activation in ACTIVATIONS:
+    if gate_up.is_cuda and activation in ACTIVATIONS:
         out = (_CALLS or _calls()).gated_act(gate_up, ACTIVATIONS[activation], int(block), out_dtype or gate_up.dtype)
         if out is not None:
             return _called(out, "gated_act")
@@ -347,11 +363,12 @@ def qk_norm_rope_kv(qkv: torch.Tensor, q_weight, k_weight, eps: float, inv_freq,
     `magnitude`.  Without a slot mapping a row may hold queries only (`num_kv_heads` 0)."""
     v_head_dim = int(v_head_dim) or head_dim
     num_v_heads = int(num_v_heads) or num_kv_heads
-    done = (_CALLS or _calls()).qk_norm_rope_kv(qkv, q_weight, k_weight, eps, inv_freq, rot_dim, positions, slot_mapping, k_pool, v_pool,
-                                                num_heads, num_kv_heads, head_dim, v_head_dim, 1 if interleaved else 0, num_v_heads,
-                                                magnitude)
-    if done is not None:
-        return _called(done, "qk_norm_rope_kv")
+    if qkv.is_cuda:
+        done = (_CALLS or _calls()).qk_norm_rope_kv(qkv, q_weight, k_weight, eps, inv_freq, rot_dim, positions, slot_mapping, k_pool, v_pool,
+                                                    num_heads, num_kv_heads, head_dim, v_head_dim, 1 if interleaved else 0, num_v_heads,
+                                                    magnitude)
+        if done is not None:
+            return _called(done, "qk_norm_rope_kv")
     _dev(qkv, q_weight, k_weight, inv_freq, positions, slot_mapping, k_pool, v_pool)
     _need(qkv.is_contiguous() and positions.dtype == torch.int32, "qk_norm_rope_kv: contiguous qkv, int32 positions")
     page_size = 1
@@ -1817,7 +1834,7 @@ def _full_precision_sums() -> None:
 
 def gemm_bf16(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """a [M,K] times w [N,K] transposed on the tensor cores, float32 accumulation."""
-    if bias is None and _MATMUL_SET:
+    if bias is None and _MATMUL_SET and a.is_cuda:
         few = a.shape[0] <= SKINNY_MAX_ROWS
         out = (_CALLS or _calls()).gemm_bf16(a, w, out_dtype or torch.bfloat16)
         if out is not None:
