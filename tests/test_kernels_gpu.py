@@ -890,6 +890,12 @@ def test_call_module_leaves_refusals_to_the_wrappers():
         o.gated_act(x[:, :63].contiguous(), "silu")
 
 
+def test_call_module_passes_on_what_a_truth_value_raises():
+    with pytest.raises(RuntimeError, match="ambiguous"):
+        ops().add_rmsnorm(torch.zeros(4, 64, device=DEV), torch.zeros(4, 64, device=DEV), torch.ones(64, device=DEV), 1e-6, torch.float32,
+                          update_residual=torch.ones(2))
+
+
 @pytest.mark.parametrize("K", [32, 96, 288, 1024, 1280, 2080, 2560])
 @pytest.mark.parametrize("variant", [0, 3, 7, 8])
 def test_skinny_product_with_batches_that_are_not_whole(K, variant):

@@ -120,7 +120,9 @@ PyObject* add_rmsnorm(PyObject*, PyObject* const* o, Py_ssize_t n) {
     if (delta && (delta.a->scalar_type() != kind || !delta.a->is_contiguous() || delta.a->sizes() != residual->sizes())) NOT_HERE;
     const int64_t width = residual->size(1), count = rows ? rows.a->numel() : residual->size(0);
     if (!small(width) || !small(count)) NOT_HERE;
-    void* sums = rows ? residual_out.ptr() : (delta && PyObject_IsTrue(o[7]) == 1 ? residual->data_ptr() : nullptr);
+    const int update = !rows && delta ? PyObject_IsTrue(o[7]) : 0;
+    if (update < 0) return nullptr;   // (its truth value raised)
+    void* sums = rows ? residual_out.ptr() : (update ? residual->data_ptr() : nullptr);
     at::Tensor out = fresh(count, width, kind, *residual);
     LAUNCH(rc, entry.add_rmsnorm(residual->data_ptr(), delta.ptr(), rows.ptr(), sums, weight->data_ptr(), out.data_ptr(), (int)count,
                                  (int)width, eps, code, s));
