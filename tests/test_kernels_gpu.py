@@ -929,6 +929,21 @@ def test_gemm_tcgen05_tiles_of_any_width(M, N, K, columns):
     ops().check_device_errors()
 
 
+@pytest.mark.parametrize("wide", [0, 1, 2, 15, 48, 255, 300, -1])
+def test_gemm_tcgen05_takes_any_wide_as_a_truth_value(wide):
+    """The C entry point: 0 for tiles of 128 columns, anything else for tiles of 256, the same sums either way."""
+    M, N, K = 130, 464, 200
+    g = torch.Generator().manual_seed(3)
+    a, w = torch.randn(M, K, generator=g).bfloat16().to(DEV), torch.randn(N, K, generator=g).bfloat16().to(DEV)
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device=DEV)
+    word = ops()._error_word(a.device)
+    assert ops().library().vx_gemm_tcgen05(a.data_ptr(), w.data_ptr(), None, out.data_ptr(), M, N, K, K, K, N, 0, 0, wide, word.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream) == 0
+    ops().note_bounded_wait()
+    ops().check_device_errors()
+    assert torch.equal(out, ops().gemm_tcgen05(a, w))
+
+
 def test_tcgen05_tile_fills_rounds():
     """The choice of tiles stays within what the kernels take."""
     for m in (1, 128, 129, 312, 777, 2048, 40000):

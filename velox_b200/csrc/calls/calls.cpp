@@ -25,7 +25,7 @@ struct Entries {
     int (*qk_norm_rope_kv)(void*, int, P, P, float, P, int, P, P, void*, void*, int, int, int, int, int, int, int, int, int, float, void*);
     int (*gated_act)(P, void*, int, int, int, int, int, int, void*);
     int (*gemm_skinny)(P, P, P, void*, int, int, int, int, int, int, int, int, int, int, void*);
-    int (*gemm_tcgen05)(P, P, P, void*, int, int, int, int, int, int, int, int, int, void*, void*);
+    int (*gemm_tcgen05_columns)(P, P, P, void*, int, int, int, int, int, int, int, int, int, void*, void*);
     int (*gemm_tcgen05_pair)(P, P, P, void*, int, int, int, int, int, int, int, int, void*, void*);
     int (*prefill)(P, int, int, P, P, int, P, int, P, P, P, void*, int, float, int, int, int, int, int, int, int, void*, int, void*, void*);
     int (*decode)(P, int, P, P, P, int, P, P, P, void*, int, void*, int, float, int, int, int, int, int, int, int, int, int, void*);
@@ -203,22 +203,22 @@ PyObject* gemm_bf16(PyObject*, PyObject* const* o, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// (a, w, bias, epilogue code, activation, wide, pair, error word)
+// (a, w, bias, epilogue code, activation, columns of a tile or 0, pair, error word)
 PyObject* gemm_tcgen05(PyObject*, PyObject* const* o, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 8) NOT_HERE;
     Arg a(o[0]), w(o[1]), error(o[7]);
     Optional bias(o[2]);
     Scalars sc;
-    const int code = sc.i(o[3]), act = sc.i(o[4]), wide = sc.i(o[5]), pair = sc.i(o[6]);
+    const int code = sc.i(o[3]), act = sc.i(o[4]), columns = sc.i(o[5]), pair = sc.i(o[6]);
     if (sc.bad || !a || !w || !is(error, at::kInt) || !bias.is(at::kFloat) || !tcgen05_takes(*a, *w)) NOT_HERE;
     const int64_t M = a->size(0), N = w->size(0), cols = code == 1 ? N / 2 : N;
     if ((bias && bias.a->numel() != N) || cols % 8) NOT_HERE;
     at::Tensor out = fresh(M, cols, at::kBFloat16, *a);
     LAUNCH(rc, pair ? entry.gemm_tcgen05_pair(a->data_ptr(), w->data_ptr(), bias.ptr(), out.data_ptr(), (int)M, (int)N, (int)a->size(1),
                                               (int)a->stride(0), (int)w->stride(0), (int)cols, code, act, error->data_ptr(), s)
-                    : entry.gemm_tcgen05(a->data_ptr(), w->data_ptr(), bias.ptr(), out.data_ptr(), (int)M, (int)N, (int)a->size(1),
-                                         (int)a->stride(0), (int)w->stride(0), (int)cols, code, act, wide, error->data_ptr(), s));
+                    : entry.gemm_tcgen05_columns(a->data_ptr(), w->data_ptr(), bias.ptr(), out.data_ptr(), (int)M, (int)N, (int)a->size(1),
+                                                 (int)a->stride(0), (int)w->stride(0), (int)cols, code, act, columns, error->data_ptr(), s));
     return result(rc, std::move(out));
     END_HANDLE_TH_ERRORS
 }
@@ -297,7 +297,7 @@ PyObject* bind(PyObject*, PyObject* arg) {
         {"vx_qk_norm_rope_kv_shared", (void**)&entry.qk_norm_rope_kv},
         {"vx_gated_act", (void**)&entry.gated_act},
         {"vx_gemm_skinny_act", (void**)&entry.gemm_skinny},
-        {"vx_gemm_tcgen05", (void**)&entry.gemm_tcgen05},
+        {"vx_gemm_tcgen05_columns", (void**)&entry.gemm_tcgen05_columns},
         {"vx_gemm_tcgen05_pair", (void**)&entry.gemm_tcgen05_pair},
         {"vx_paged_prefill_attention_tc", (void**)&entry.prefill},
         {"vx_paged_decode_attention_shape", (void**)&entry.decode},

@@ -261,10 +261,10 @@ static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mw, const float* 
 // gated: 0 plain, C is [M, N]; 1: W's rows come in tiles of 8 gate rows followed by
 // their 8 up rows and C is [M, N/2] = act(gate) * up; 2: C is [M, N] = act(.), relu or its square.  `error` is a device int that
 // a block sets (TC_ERR_*) if one of its bounded waits runs out; the caller zeroes it
-// and reads it when it wants to know.  `wide` picks 128 x 256 tiles (0: 128 x 128; 16 to 256, a multiple of 16: tiles of as many
-// columns).
-extern "C" int vx_gemm_tcgen05(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int lda,
-                               int ldw, int ldc, int gated, int act, int wide, int* error, cudaStream_t stream) {
+// and reads it when it wants to know.  `columns`: tiles of 128 rows and so many columns (16 to 256, a multiple of 16; 0: 128, by the kernel
+// with the deeper ring).
+extern "C" int vx_gemm_tcgen05_columns(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int lda,
+                                       int ldw, int ldc, int gated, int act, int columns, int* error, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return VX_OK;
     if (K <= 0 || (K & 7) || (N & 15) || !error) return VX_ERR_SHAPE;
     if ((lda & 7) || (ldw & 7) || (ldc & 7) || lda < K || ldw < K) return VX_ERR_ALIGN;
@@ -272,15 +272,21 @@ extern "C" int vx_gemm_tcgen05(const void* A, const void* W, const float* bias, 
     if (gated < 0 || gated > TC_ACT || (gated && (act < 0 || act > VX_ACT_LAST)) || (gated == TC_GATED && bias)) return VX_ERR_SHAPE;
     if (gated == TC_ACT && !tc_cheap_act(act)) return VX_ERR_SHAPE;
     if (ldc < (gated == TC_GATED ? N / 2 : N)) return VX_ERR_SHAPE;
-    if (wide < 0 || wide > 256 || (wide > 1 && (wide & 15))) return VX_ERR_SHAPE;
+    if (columns < 0 || columns > 256 || (columns & 15)) return VX_ERR_SHAPE;
     CUtensorMap ma, mw;
-    const int bn = wide > 1 ? wide : (wide ? 256 : 128);
+    const int bn = columns ? columns : 128;
     if (!tc_make_map(&ma, A, M, K, lda, TC_BM) || !tc_make_map(&mw, W, N, K, ldw, bn)) return VX_ERR_DRIVER;
     bf16* c = (bf16*)C;
 #define TC_GO(BN_, ST_, E_) tc_launch<BN_, ST_, E_>(ma, mw, bias, c, M, N, K, ldc, act, error, stream, nullptr, nullptr, 0, nullptr, nullptr, 0.f, 0.f, bn)
-    if (wide) return gated == TC_GATED ? TC_GO(256, 4, TC_GATED) : (gated == TC_ACT ? TC_GO(256, 4, TC_ACT) : TC_GO(256, 4, TC_PLAIN));
+    if (columns) return gated == TC_GATED ? TC_GO(256, 4, TC_GATED) : (gated == TC_ACT ? TC_GO(256, 4, TC_ACT) : TC_GO(256, 4, TC_PLAIN));
     return gated == TC_GATED ? TC_GO(128, 6, TC_GATED) : (gated == TC_ACT ? TC_GO(128, 6, TC_ACT) : TC_GO(128, 6, TC_PLAIN));
 #undef TC_GO
+}
+
+// The same with tiles of 256 columns if `wide` is not 0, else of 128.
+extern "C" int vx_gemm_tcgen05(const void* A, const void* W, const float* bias, void* C, int M, int N, int K, int lda,
+                               int ldw, int ldc, int gated, int act, int wide, int* error, cudaStream_t stream) {
+    return vx_gemm_tcgen05_columns(A, W, bias, C, M, N, K, lda, ldw, ldc, gated, act, wide ? 256 : 0, error, stream);
 }
 
 // The grouped product of a routed feed-forward: A [rows, K] in group order, W [groups, N, K], row tiles of up to

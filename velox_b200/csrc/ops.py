@@ -137,6 +137,7 @@ def _declare(lib) -> None:
         "vx_gemm_nt_simt": [P, P, P, P, I, I, I, I, I, I, I, I, P],
         "vx_gemm_nt_simt_ready": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, I, P],
         "vx_gemm_tcgen05": [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P],
+        "vx_gemm_tcgen05_columns": [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_tcgen05_pair": [P, P, P, P, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_skinny": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P],
         "vx_paged_prefill_attention_tc": [P, I, I, P, P, I, P, I, P, P, P, P, I, F, I, I, I, I, I, I, I, P, I, P, P],
@@ -1734,7 +1735,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
     _need(not columns or (16 <= columns <= 256 and columns % 16 == 0 and not pair), "gemm_tcgen05: tiles of 16 to 256 columns by single blocks")
     _need(not (pair and activation), "gemm_tcgen05: a plain activation on tiles of single blocks")
     if gated_activation is None or gated_activation in ACTIVATIONS:
-        out = (_CALLS or _calls()).gemm_tcgen05(a, w, bias, code, ACTIVATIONS.get(gated_activation, 0) if pair else act, columns or (1 if wide else 0),
+        out = (_CALLS or _calls()).gemm_tcgen05(a, w, bias, code, ACTIVATIONS.get(gated_activation, 0) if pair else act, columns or (256 if wide else 0),
                                                 1 if pair else 0, _error_word(a.device))
         if out is not None:
             out = _called(out, "gemm_tcgen05_pair" if pair else "gemm_tcgen05")
@@ -1756,8 +1757,9 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
                                               cols, 1 if gated_activation else 0, ACTIVATIONS.get(gated_activation, 0),
                                               _ptr(_error_word(a.device)), _stream()), "gemm_tcgen05_pair")
     else:
-        _check(library().vx_gemm_tcgen05(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0), w.stride(0), cols,
-                                         code, act, columns or (1 if wide else 0), _ptr(_error_word(a.device)), _stream()), "gemm_tcgen05")
+        _check(library().vx_gemm_tcgen05_columns(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0), w.stride(0), cols,
+                                                 code, act, columns or (256 if wide else 0), _ptr(_error_word(a.device)), _stream()),
+               "gemm_tcgen05")
     note_bounded_wait()
     return out
 
