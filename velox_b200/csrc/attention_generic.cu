@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) paged_attention_generic_kernel
     int chunk) {
     pdl_wait();
     pdl_trigger();
-    __shared__ __align__(16) float q_s[ATT_MAX_D];
+    __shared__ __align__(FOUR ? 16 : 4) float q_s[ATT_MAX_D];   // (aligned for the other form, its loop over d is half as fast)
     __shared__ float acc_s[ATT_WARPS][ATT_MAX_D];
     __shared__ float m_s[ATT_WARPS], l_s[ATT_WARPS];
 
