@@ -358,8 +358,8 @@ def test_sample_temperature_and_top_p(vocab):
 
 @pytest.mark.parametrize("vocab", [25000, 60001, 151936, 262144])
 def test_sample_gives_the_same_token_in_every_form(vocab):
-    """On 148 SMs 1 and 12 rows are drawn by eight blocks a row, 20 by four, 40 by two and 80 by one (fewer where the vocabulary is
-    small), with the row's parts kept in shared memory or, where they don't fit, read again.  Every form adds in the same order, so a
+    """On a B200 1 and 12 rows are drawn by eight blocks a row, 20 by four, 40 by two and 80 by one (fewer where the vocabulary is
+    small), with the row's parts kept in shared memory or, where they don't fit or nothing is drawn, read again.  Every form adds in the same order, so a
     row's token is the same in all of them, bit for bit, and each form is held against float64.  60,001: rows that begin on no 16-byte
     address.  Ties of the maximum lie in different blocks' parts."""
     from velox_b200.sampling.rng import uniform

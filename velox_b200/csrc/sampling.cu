@@ -1,6 +1,6 @@
 // Token sampling from float32 logits: greedy, temperature, temperature + top-p.
 //
-// A cluster of one to eight blocks per row, as many as the rows leave SMs for.  For row r with temperature T, nucleus mass P and a
+// A cluster of one to eight blocks per row, as many as let all rows' clusters run at once.  For row r with temperature T, nucleus mass P and a
 // uniform number u in [0,1) that the host drew for this (request, step):
 //   T <= 1e-7:  the argmax, the lowest index winning ties.
 //   otherwise:  e_i = 2^((x_i - max) log2(e) / T);  with 0 < P < 1 only the most
@@ -12,8 +12,8 @@
 // Each block reads its part of the row once, all loads in flight together, and keeps it in shared memory (where it fits)
 // when it is needed again; maxima, histograms and masses are put together through the cluster's shared memory, where
 // every block reads all of them and comes to the same conclusion by itself.  With one block per row one SM pulled the
-// row from L2 five times: at 151,936 elements 86 us by nucleus, 38 with a temperature alone, 6.5 greedy; now 28.6 / 12.9 / 3.5
-// for one row, 37 / 19 / 4.5 for 20, 55 / 28 / 5.8 for 64 (from 75 rows on there is one block per row as before).
+// row from L2 five times: at 151,936 elements 86 us by nucleus, 38 with a temperature alone, 6.5 greedy; now 28.5 / 13.0 / 3.4
+// for one row, 37 / 19.5 / 4.3 for 19, 54 / 28 / 5.7 for 64 (from 75 rows on there is one block per row as before: 84 / 39 / 6.7).
 // The threshold t is found ten bits a pass: a histogram, over the next ten bits of
 // the patterns of e (positive floats order like their patterns), of the mass in each
 // bin, as exact integers so that the order of the additions does not matter, then a
@@ -135,9 +135,8 @@ __device__ __forceinline__ T* sample_at(cg::cluster_group& cluster, T* p, int bl
 }
 
 template <int BLOCKS, bool KEPT>
-__global__ void __cluster_dims__(BLOCKS, 1, 1) __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
-              const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+__device__ __forceinline__ void sample_row(const float* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
+                                           const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
     cg::cluster_group cluster = cg::this_cluster();
     if (BLOCKS > 1) cluster.barrier_arrive();   // (here this block's shared memory exists: waited for before the first store into another's)
     pdl_wait();
@@ -292,7 +291,10 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
             if (lane == 31) gm[g] = incl;
         }
     }
-    const int last_neg = block_min_int(last_kept >= 0 ? -last_kept : INT_MAX, si);   // (its barriers make the masses visible)
+    // (with several blocks the last kept element goes to the first with the rest, below; the barriers make the masses visible)
+    const int my_last = last_kept >= 0 ? -last_kept : INT_MAX;
+    const int last_neg = BLOCKS > 1 ? block_min_int(my_last, si) : 0;
+    if (BLOCKS == 1) __syncwarp();   // (a stretch is its warp's)
     const bool leads = warp % BLOCKS == 0;   // one warp of every stretch goes on
     float mine = 0.f;   // the groups' masses added up in group order
     if (leads) {
@@ -339,6 +341,14 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
         }
     }
     cand = block_min_int(cand, si);
+    if (BLOCKS == 1) {
+        if (cand == INT_MAX) {   // (uniform) rounding left nobody above the target: the last kept token
+            const int neg = block_min_int(my_last, si);
+            cand = neg == INT_MAX ? best_i : -neg;
+        }
+        if (tid == 0) out[r] = cand;
+        return;
+    }
     if (tid == 0) {
         sample_at<BLOCKS>(cluster, cand_of, 0)[rank] = cand;
         sample_at<BLOCKS>(cluster, last_of, 0)[rank] = last_neg;
@@ -351,28 +361,65 @@ sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __re
         cand = min(cand, cand_of[b]);
         neg = min(neg, last_of[b]);
     }
-    // rounding left nobody above the target: the last kept token
     out[r] = cand != INT_MAX ? cand : (neg == INT_MAX ? best_i : -neg);
+}
+
+template <int BLOCKS, bool KEPT>
+__global__ void __cluster_dims__(BLOCKS, 1, 1) __launch_bounds__(SAMPLE_THREADS)
+sample_cluster_kernel(const float* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
+                      const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+    sample_row<BLOCKS, KEPT>(logits, ld, V, temperature, top_p, uniform, out);
+}
+template <bool KEPT>
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+sample_kernel(const float* __restrict__ logits, int ld, int V, const float* __restrict__ temperature,
+              const float* __restrict__ top_p, const float* __restrict__ uniform, int* __restrict__ out) {
+    sample_row<1, KEPT>(logits, ld, V, temperature, top_p, uniform, out);
 }
 
 #define SAMPLE_PART_MAX (160 * 1024)   // most bytes of a row that a block keeps
 #define SAMPLE_PART_MIN 12288          // fewest elements worth a block: below, the cluster's barriers cost more than the pass (301 elements: 9.8 us in one block, 18 in eight)
-static int sample_sm_count() {
-    static int sms[VX_MAX_DEVICES];
-    return vx_sm_count(sms);
+// All forms at the first call on a device: a later call may come from inside a stream capture.  `at_once`: how many clusters of
+// 2, 4 and 8 blocks (a block fills an SM) find room together, which is less than the SMs divided by their blocks, as a cluster lies within one
+// of the GPU's groups of SMs: 74, 33 and 15 on a B200.  (Chosen by the number of SMs, 37 rows of 151,936 by clusters of four, greedy, took 8.4 us;
+// one block a row 6.5, clusters of two 5.2.)
+struct SampleSetup {
+    bool done;
+    int at_once[3];
+};
+template <int BLOCKS>
+static cudaError_t configure_sample_clusters(int* at_once) {
+    cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel<BLOCKS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(BLOCKS);
+    cfg.blockDim = dim3(SAMPLE_THREADS);
+    cfg.dynamicSmemBytes = SAMPLE_PART_MAX;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = BLOCKS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(at_once, sample_cluster_kernel<BLOCKS, true>, &cfg) != cudaSuccess) {
+        *at_once = 0;   // (not to be had: no clusters of this size)
+        cudaGetLastError();
+    }
+    return cudaSuccess;
 }
-// All forms at the first call on a device: a later call may come from inside a stream capture.
-static int configure_sample() {
-    static bool configured[VX_MAX_DEVICES];
+static int configure_sample(const int** at_once) {
+    static SampleSetup setups[VX_MAX_DEVICES];
     const int dev = vx_current_device();
     if (dev < 0) return VX_ERR_LIMIT;
-    if (configured[dev]) return VX_OK;
-    cudaError_t e = cudaFuncSetAttribute(sample_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(sample_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
+    SampleSetup& setup = setups[dev];
+    *at_once = setup.at_once;
+    if (setup.done) return VX_OK;
+    cudaError_t e = cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_PART_MAX);
+    if (e == cudaSuccess) e = configure_sample_clusters<2>(&setup.at_once[0]);
+    if (e == cudaSuccess) e = configure_sample_clusters<4>(&setup.at_once[1]);
+    if (e == cudaSuccess) e = configure_sample_clusters<8>(&setup.at_once[2]);
     if (e != cudaSuccess) return (int)e;
-    configured[dev] = true;
+    setup.done = true;
     return VX_OK;
 }
 
@@ -382,28 +429,33 @@ extern "C" int vx_sample(const float* logits, int ld, int rows, int vocab, const
     if (vocab <= 0 || ld < vocab) return VX_ERR_SHAPE;
     if (vocab > (1 << 18)) return VX_ERR_LIMIT;  // the fixed-point mass of a row has to fit 64 bits
     if (temperature && !uniform) return VX_ERR_SHAPE;
-    // As many blocks a row as the rows leave SMs for (a block fills an SM's registers; clusters beyond one round cost more
-    // than their blocks save: 64 rows greedy 6.7 us with one block each, 16 with eight), and the row's parts in shared memory where they fit.
-    const int sms = sample_sm_count();
-    int blocks = 8ll * rows <= sms ? 8 : 4ll * rows <= sms ? 4 : 2ll * rows <= sms ? 2 : 1;
+    const int* at_once;
+    if (const int rc = configure_sample(&at_once)) return rc;
+    // As many blocks a row as let all clusters run at once (a second round of clusters costs more than their blocks save),
+    // and the row's parts in shared memory where they fit.
+    int blocks = rows <= at_once[2] ? 8 : rows <= at_once[1] ? 4 : rows <= at_once[0] ? 2 : 1;
     while (blocks > 1 && vocab / blocks < SAMPLE_PART_MIN) blocks /= 2;
     const size_t groups = ((vocab + SAMPLE_WARPS - 1) / SAMPLE_WARPS + 31) >> 5;   // (as in the kernel)
-    const size_t part = temperature ? SAMPLE_WARPS / blocks * groups * 32 * sizeof(float) : 0;
-#define SAMPLE_GO(BLOCKS, KEPT)                                                                                       \
-    VX_LAUNCH_K(VX_K_SAMPLE, (sample_kernel<BLOCKS, KEPT>), rows * BLOCKS, SAMPLE_THREADS, KEPT ? part : 0, stream, logits, ld, vocab, \
+    const size_t part = SAMPLE_WARPS / blocks * groups * 32 * sizeof(float);
+    // A block keeps its part of the row where that fits and the row is read again; a row of one block only if it is short
+    // (25,000 elements, 75 rows, us, kept and not: temperature 11.2 and 10.6, nucleus 22.0 and 21.5; 5,000: 5.8 and 5.9, 11.6 and 12.1).
+    const bool kept = temperature && part <= SAMPLE_PART_MAX && (blocks > 1 || vocab <= SAMPLE_PART_MIN);
+#define SAMPLE_GO(KERNEL, KEPT)                                                                                       \
+    VX_LAUNCH_K(VX_K_SAMPLE, (KERNEL), rows * blocks, SAMPLE_THREADS, KEPT ? part : 0, stream, logits, ld, vocab, \
                 temperature, top_p, uniform, out)
-    const int rc = configure_sample();
-    if (rc != VX_OK) return rc;
-    if (part <= SAMPLE_PART_MAX) {
-        if (blocks == 8) SAMPLE_GO(8, true);
-        else if (blocks == 4) SAMPLE_GO(4, true);
-        else if (blocks == 2) SAMPLE_GO(2, true);
-        else SAMPLE_GO(1, true);
-    } else {   // (never with eight blocks: 2^18 / 8 elements fit)
-        if (blocks == 4) SAMPLE_GO(4, false);
-        else if (blocks == 2) SAMPLE_GO(2, false);
-        else SAMPLE_GO(1, false);
+#define SAMPLE_CLUSTER(BLOCKS, KEPT) SAMPLE_GO((sample_cluster_kernel<BLOCKS, KEPT>), KEPT)
+    if (kept) {
+        if (blocks == 8) SAMPLE_CLUSTER(8, true);
+        else if (blocks == 4) SAMPLE_CLUSTER(4, true);
+        else if (blocks == 2) SAMPLE_CLUSTER(2, true);
+        else SAMPLE_GO(sample_kernel<true>, true);
+    } else {
+        if (blocks == 8) SAMPLE_CLUSTER(8, false);
+        else if (blocks == 4) SAMPLE_CLUSTER(4, false);
+        else if (blocks == 2) SAMPLE_CLUSTER(2, false);
+        else SAMPLE_GO(sample_kernel<false>, false);
     }
+#undef SAMPLE_CLUSTER
 #undef SAMPLE_GO
     VX_LAUNCH_CHECK();
     return VX_OK;
