@@ -269,13 +269,22 @@ def test_gemm_simt_fp32(M, N, K):
     assert torch.equal(alone[0], ops().gemm_nt_simt(a, w)[M - 1])
 
 
-@pytest.mark.parametrize("N,K,pad", [(64, 256, 0), (65, 512, 0), (130, 777, 0), (63, 1000, 3), (100, 2051, 1), (1024, 2048, 4), (40000, 300, 0)])
+def float32_parts(K):
+    """How the 32-bit product cuts k: (parts, their length)."""
+    parts = min(8, max(1, K // (256 if K >= 1024 else 64)))
+    length = -(-(-(-K // parts)) // 32) * 32
+    return -(-K // length), length
+
+
+@pytest.mark.parametrize("N,K,pad", [(64, 256, 0), (65, 512, 0), (130, 777, 0), (63, 1000, 3), (100, 2051, 1), (1024, 2048, 4), (40000, 300, 0),
+                                     (8192, 128, 0), (8192, 256, 0), (8190, 512, 4), (8192, 1001, 0), (8192, 1024, 0)])
 def test_gemm_float32_tiles_and_parts(N, K, pad):
     """The 32-bit product at the edges of its row tiles (4, 8, 16, 32, 64) and of the parts of k, rows that begin on 16-byte
-    addresses and rows that do not; every row the same bits however many rows the call has.  A sum's error is at most
-    (the additions that a term passes through) units of 2^-24 of the sum of the terms' sizes: half a part, the parts, two."""
-    parts = min(8, max(1, K // 256))
-    steps = -(-K // parts) // 2 + 32 + parts + 2
+    addresses and rows that do not, tiles enough to keep k whole and too few; every row the same bits however many rows the call has.
+    A sum's error is at most (the additions that a term passes through) units of 2^-24 of the sum of the terms' sizes: half a
+    part, the parts, two."""
+    parts, length = float32_parts(K)
+    steps = length // 2 + parts + 2
     w = rnd((N, K + pad), torch.float32, 7)[:, :K]
     a = rnd((130, K + pad), torch.float32, 6)[:, :K]
     bias = rnd((N,), torch.float32, 8)
@@ -284,6 +293,18 @@ def test_gemm_float32_tiles_and_parts(N, K, pad):
     assert (abs(f64(whole) - (f64(a) @ f64(w).T + f64(bias))) <= limit).all()
     for M in (1, 3, 4, 5, 8, 9, 16, 17, 32, 33, 63, 64, 65, 129):
         assert torch.equal(ops().gemm_nt_simt(a[130 - M:], w, bias), whole[130 - M:]), M
+
+
+@pytest.mark.parametrize("K", [256, 512, 1000, 1024])
+def test_gemm_float32_error_follows_the_parts(K):
+    """Normal terms: a chain's j-th addition is rounded at the size of j^1/2 terms, so P parts of length L, two chains of L/2 each, come to an error
+    of c 2^-24 (L/4 + 1 + (P + 1)/2)^1/2 of the result, c about 0.43 for roundings spread evenly: 0.6 allows for the draw.  (Two parts
+    at k = 512 would come to 0.43 x 8.2 = 3.5 units, eight may have 0.6 x 4.6 = 2.8.)"""
+    parts, length = float32_parts(K)
+    a, w = rnd((64, K), torch.float32, 21), rnd((512, K), torch.float32, 22)
+    want = f64(a) @ f64(w).T
+    err = np.linalg.norm(f64(ops().gemm_nt_simt(a, w)) - want) / np.linalg.norm(want)
+    assert err <= 0.6 * 2.0 ** -24 * math.sqrt(length / 4 + 1 + (parts + 1) / 2), err
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (12, 1000, 777), (99, 4096, 1024), (3, 40000, 300)])

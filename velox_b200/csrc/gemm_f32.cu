@@ -75,16 +75,13 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
     constexpr int WX = TX / LX;   // warps side by side
     const int tx = (warp % WX) * LX + lane % LX, ty = (warp / WX) * (32 / LX) + lane / LX;
 
-    auto ask_w = [&]() {
-#pragma unroll
-        for (int s = 0; s < GF32_STAGES - 1; ++s)
-            if (s < chunks) gf_load<BN, NT, VEC>(gf_smem + s * STAGE + BM * GF32_LD, W, n0, N, ldw, kbeg + s * GF32_BK, kend);
-    };
     // a W that the caller calls ready depends on no earlier kernel: its first tiles are asked for before the wait
-    if (w_ready) ask_w();
-    pdl_wait();
+    if (!w_ready) pdl_wait();
+#pragma unroll
+    for (int s = 0; s < GF32_STAGES - 1; ++s)
+        if (s < chunks) gf_load<BN, NT, VEC>(gf_smem + s * STAGE + BM * GF32_LD, W, n0, N, ldw, kbeg + s * GF32_BK, kend);
+    pdl_wait();   // (a second time it returns at once)
     pdl_trigger();
-    if (!w_ready) ask_w();
 #pragma unroll
     for (int s = 0; s < GF32_STAGES - 1; ++s) {
         if (s < chunks) gf_load<BM, NT, VEC>(gf_smem + s * STAGE, A, m0, M, lda, kbeg + s * GF32_BK, kend);
@@ -221,17 +218,15 @@ static int gf_launch(const GfCall& g, int parts, int len, cudaStream_t stream) {
     return VX_OK;
 }
 
-template <int TM, int TN, int TY, int TX>
-static bool gf_whole(const GfCall& g, long long sms) {
-    constexpr int BM = TM * TY, BN = TN * TX;
-    return (long long)((g.N + BN - 1) / BN) * ((g.M + BM - 1) / BM) * g.batch >= 8 * sms;
+static long long gf_tiles(const GfCall& g, int bm, int bn) {
+    return (long long)((g.N + bn - 1) / bn) * ((g.M + bm - 1) / bm) * g.batch;
 }
 
 template <int TM, int TN, int TY, int TX>
-static int gf_choose(const GfCall& g, bool vec, long long sms, cudaStream_t stream) {
+static int gf_choose(const GfCall& g, bool vec, bool whole, cudaStream_t stream) {
     int parts, len;
     gf_parts(g.K, &parts, &len);
-    if (parts > 1 && !gf_whole<TM, TN, TY, TX>(g, sms))
+    if (parts > 1 && !whole)
         return vec ? gf_launch<TM, TN, TY, TX, true, true>(g, parts, len, stream) : gf_launch<TM, TN, TY, TX, false, true>(g, parts, len, stream);
     return vec ? gf_launch<TM, TN, TY, TX, true, false>(g, parts, len, stream) : gf_launch<TM, TN, TY, TX, false, false>(g, parts, len, stream);
 }
@@ -247,8 +242,14 @@ static int gf_choose(const GfCall& g, bool vec, long long sms, cudaStream_t stre
 // Tiles of 64 rows x 128 columns and of 128 x 128 (8 x 8 outputs a thread) were tried: 36 to 47 microseconds where these
 // take 21 to 38, and no faster at 2,000 rows.  Error against 64 bits at K = 1024 / 3072 / 9728: 2.1e-7 / 2.6e-7 / 4.5e-7 (before, one
 // ascending sum: 5.7e-7 / 9.9e-7 / 1.8e-6).
-// A product of at least 8 tiles an SM keeps k whole (151,936 columns: 162 against 181 microseconds at one row); with fewer, the
-// parts of k go to the blocks of a cluster (4096 x 1024: 38 whole, 11 cut).
+// Whether the parts of k go to the blocks of a cluster: not where there are tiles enough without.  Up to 32 rows that takes 8 tiles an SM
+// (151,936 columns, one row: 162 whole, 181 cut; 4096 x 1024: 38 and 11), above, with tiles of 64 rows, 2.5 (rows x N x K,
+// whole and cut: 150 x 8192 x 2048 197 and 201; 1000 x 4096 x 512 114 and 183; at 2.2 tiles an SM 300 x 4096 x 2048 197 and 170).
+// Below k = 1,024, where a part is short against the cluster's barriers, less: whole from K / 170 tiles of 32 rows an SM on, as these as long as
+// four an SM hold them all, else as tiles of 64 rows (whole, and cut in the better of the two tiles): 128 x 4096 x 128 7.7 and 9.3 to 11.8;
+// 128 x 8192 x 256 19.3 and 28.7 (the kernel before these: 25.2); 300 x 4096 x 256 26.6 and 33; 150 x 2048 x 256 12.7 and 11.7, cut; 128 x 8192 x 512
+// 37 and 50; 300 x 2048 x 512 37 and 32, cut.  Rows that begin on no 16-byte address wait for their loads and are cut longer: 128 x 8192 x
+// 1001 129 and 102 (the kernel before these: 94, the one size at which it is ahead).
 int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc, int batch,
                 long long sa, long long sw, long long sc, int w_ready, cudaStream_t stream) {
     const GfCall g = {A, W, bias, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready};
@@ -256,13 +257,17 @@ int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int
     const bool vec = !((lda | ldw) & 3) && !((sa | sw) & 3) && !((((uintptr_t)A) | ((uintptr_t)W)) & 15);
     static int sms_cache[VX_MAX_DEVICES];
     const long long sms = vx_sm_count(sms_cache);
-    if (M <= 4 && gf_whole<4, 4, 1, 32>(g, sms)) return gf_choose<4, 4, 1, 32>(g, vec, sms, stream);   // (143 against 162 microseconds there)
+    if (M <= 4 && gf_tiles(g, 4, 128) >= 8 * sms) return gf_choose<4, 4, 1, 32>(g, vec, true, stream);   // (143 against 162 microseconds there)
     // up to 8 rows: the wide rows pay where W is large
-    if (M <= 8 && (long long)N * K >= (6 << 20)) return gf_choose<8, 2, 1, 32>(g, vec, sms, stream);
-    if (M <= 16) return gf_choose<4, 4, 4, 16>(g, vec, sms, stream);
+    if (M <= 8 && (long long)N * K >= (6 << 20)) return gf_choose<8, 2, 1, 32>(g, vec, gf_tiles(g, 8, 64) >= 8 * sms, stream);
+    if (M <= 16) return gf_choose<4, 4, 4, 16>(g, vec, gf_tiles(g, 16, 64) >= 8 * sms, stream);
     int parts, len;
     gf_parts(K, &parts, &len);
-    const long long blocks32 = (long long)((N + 63) / 64) * ((M + 31) / 32) * batch * parts;
-    if (M <= 32 || blocks32 <= 4 * sms) return gf_choose<8, 4, 4, 16>(g, vec, sms, stream);
-    return gf_choose<8, 4, 8, 16>(g, vec, sms, stream);
+    const long long t32 = gf_tiles(g, 32, 64), t64 = gf_tiles(g, 64, 64);
+    if (M <= 32) return gf_choose<8, 4, 4, 16>(g, vec, t32 >= 8 * sms, stream);
+    // a narrow k: the parts are short against the cluster's barriers, the shorter the fewer tiles it takes to do without
+    if (K <= 128 || (vec && K < 1024 && t32 * 170 >= K * sms))
+        return t32 <= 4 * sms ? gf_choose<8, 4, 4, 16>(g, vec, true, stream) : gf_choose<8, 4, 8, 16>(g, vec, true, stream);
+    if (t32 * parts <= 4 * sms) return gf_choose<8, 4, 4, 16>(g, vec, false, stream);
+    return gf_choose<8, 4, 8, 16>(g, vec, 2 * t64 >= 5 * sms, stream);
 }
