@@ -246,7 +246,14 @@ static int pick_variant(int N, int K) {
     const int tiles = (N + 15) / 16, chunks = K / 32;
     if (tiles <= 2 * sms) return 3;
     if (tiles >= 8 * sms && chunks % 64 == 0) return 3;
-    if (chunks % 40 == 0) return 8;
+    if (chunks % 40 == 0) {
+        // Five warps by three blocks an SM, or four warps by four: the rounds of the SMs times the trips of a block (its
+        // batches, and a half for its end).  Microseconds, 4 rows, (7) and (8): 7168 x 5120 12.0, 14.8; 8192 x 5120 13.4, 15.6; 24576 x
+        // 5120 37.5, 38.5; 7168 x 2560 7.3, 8.6; 8192 x 1280 4.9, 5.4; 6144 x 5120 10.1, 10.0; 10240 x 5120 18.2, 17.6; 15360 x
+        // 1280 8.9, 8.0; 14208 x 5120 22.7, 23.4, the rule's worst (it takes (8)).
+        const int rounds8 = (tiles + 3 * sms - 1) / (3 * sms), rounds7 = (tiles + 4 * sms - 1) / (4 * sms);
+        return rounds7 * (2 * ((chunks + 31) / 32) + 1) < rounds8 * (2 * (chunks / 40) + 1) ? 7 : 8;
+    }
     if (tiles < 8 * sms || chunks % 32 == 0) return 7;
     return 3;
 }
