@@ -25,6 +25,9 @@
 // follow each other without a gap, and the products after this one then read their rows through the 28 KB that is left:
 // steps of 1 request of 16,000 keys and of 8 of 4,096 took 1,058 and 1,687 us instead of 983 and 1,447 (12 layers of the 4B, 8B
 // shape), and 1,033 and 1,488 with three blocks an SM.
+// Groups above eight heads of 128 take twice the instructions a key, and where the pieces are many a lone warp of a scheduler is the bound: 64
+// requests of 1,000 keys, 64 heads on 4, 36 us, 64 of 4,096 105 (heads in the 16 rows, eight warps an SM: 32 and 100; but 16
+// requests of 4,096 30.3 against 29.7 now, 64 of 300 20.1 against 18.0, one of 16,000 with 32 heads on 2 18.6 against 8.8).
 // Before, blocks of 4 to 6 warps walked pieces tile by tile, each tile with a softmax of its own and the queries in
 // the 16 rows of mma.sync: 15.2 us for one request of 500 keys (now 5.6), 20.5 for one of 16,000 (14.0), 41.5 for 20 of
 // 2,000 (33), 173 for 64 of 4,096 (165).
@@ -309,6 +312,24 @@ __device__ __forceinline__ void dec_write_piece(const float (&o)[NI][NG][4], con
         }
 }
 
+// Which piece of which request and kv head block `number` takes: a head's pieces one after another, but where no request has more
+// than two, the first ones, which are whole, before the second ones, which are not: the longest come first, and the last round of the
+// SMs is short (64 requests of 300 keys, 16 and 32 query heads on 8: 20.2 and 22.2 -> 18.4 and 20.2 us).
+__device__ __forceinline__ void dec_locate(int number, int Hk, int max_pieces, int& b, int& hk, int& piece) {
+    if (max_pieces == 2) {
+        const int half = (int)gridDim.x >> 1;
+        piece = number >= half;
+        number -= piece * half;
+        b = number / Hk;
+        hk = number % Hk;
+    } else {
+        const int per_request = Hk * max_pieces;
+        b = number / per_request;
+        hk = (number % per_request) / max_pieces;
+        piece = number % max_pieces;
+    }
+}
+
 // A warp (a block of its own) per piece, RING tiles of K and V in shared memory.
 template <int D, int NG, int RING>
 __global__ void __launch_bounds__(32)
@@ -322,8 +343,8 @@ paged_decode_attention_kernel(const bf16* __restrict__ q, int q_row_stride, cons
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int TILE_BYTES = 16 * D * 2;
     const int lane = threadIdx.x;
-    const int number = (int)blockIdx.x, per_request = Hk * max_pieces;
-    const int b = number / per_request, hk = (number % per_request) / max_pieces, piece = number % max_pieces;
+    int b, hk, piece;
+    dec_locate((int)blockIdx.x, Hk, max_pieces, b, hk, piece);
     const int G = H / Hk;
     // The step's description was copied to the device before any kernel of the
     // step ran, so it may be read before the wait on earlier kernels.
