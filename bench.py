@@ -397,8 +397,9 @@ def dobepel_kernels(pk, sz):
         2.0 * T * top * F * E)
     I = top * F + sz["shared_ff"]
     wq = (torch.randn((2 * I, E), device=dev) * 0.02).to(bf)
+    pair, columns = ops.tcgen05_tile(T, 2 * I, E, h.device)
     row("Qwen3 gate_up, %d rows (tcgen05, fused activation)" % T, us(lambda: ops.gemm_tcgen05(
-        h, wq, None, gated_activation="silu", pair=ops.tcgen05_pair_better(T, 2 * I, h.device))), 2.0 * T * 2 * I * E)
+        h, wq, None, gated_activation="silu", pair=pair, columns=columns)), 2.0 * T * 2 * I * E)
     hd = torch.randn((B, E), device=dev).to(bf)
     pland = ops.moe_route(hd, wr, None, NE, top, ops.moe_tile_rows(hd, B * top))
     many = [(torch.randn((NE, 2 * F, E), device=dev) * 0.02).to(bf) for _ in range(max(2, int(3e8 // (NE * 2 * F * E * 2))))]

@@ -1691,18 +1691,6 @@ def tcgen05_tile(m: int, n: int, k: int, device) -> Tuple[bool, int]:
     return columns == 0, columns
 
 
-def tcgen05_pair_better(m: int, n: int, device) -> bool:
-    """Whether 256 x 256 tiles by pairs of blocks beat 128 x 256 tiles by single blocks for
-    an [m, n] result: both kinds of block spend the same time on a tile (a pair a little
-    less: each SM reads half of W's tile from its shared memory), so the kind that needs
-    fewer rounds of the GPU's SMs wins; padding rows count as work."""
-    sms = _sm_count(device)
-    cols = -(-n // 256)
-    single = -(-(-(-m // 128) * cols) // sms)
-    paired = -(-(-(-m // 256) * cols) // max(1, sms // 2))
-    return paired * 0.97 < single
-
-
 TCGEN05_ACTIVATIONS = ("relu", "relu2")   # what the tcgen05 products apply to every sum (gates: any activation)
 
 
