@@ -437,10 +437,13 @@ DECODE_CASES = [
     ([900, 64, 257], 16, 1, 64, 16, 0),              # 16 query heads share one kv head
     ([1300, 40, 590, 5], 4, 2, 128, 16, 540),        # a window that crosses split boundaries
     ([3000], 32, 8, 128, 16, 0),                     # the flagship's head layout, 12 pieces
-    # the kernel's other block shapes, chosen from requests x kv heads x pieces against 148 SMs:
-    ([1000] + [(i * 97) % 1000 + 1 for i in range(19)], 16, 8, 128, 16, 0),   # 640 pieces: blocks of 5 warps
-    ([1000] + [(i * 61) % 1000 + 1 for i in range(25)], 16, 8, 128, 16, 0),   # 832 pieces: blocks of 6 warps
-    ([1000] + [(i * 43) % 1000 + 1 for i in range(29)], 16, 8, 64, 16, 0),    # 960 pieces: blocks of 4 warps, two an SM
+    # more pieces than SMs: a warp per piece (above, a block of eight warps per piece)
+    ([1000] + [(i * 97) % 1000 + 1 for i in range(19)], 16, 8, 128, 16, 0),   # 640 pieces
+    ([1000] + [(i * 61) % 1000 + 1 for i in range(25)], 16, 8, 128, 16, 0),   # 832 pieces
+    ([1000] + [(i * 43) % 1000 + 1 for i in range(29)], 16, 8, 64, 16, 0),    # 960 pieces, heads of 64
+    # two pieces at most: the first ones before the second ones
+    ([512, 257, 256, 1] + [(i * 37) % 512 + 1 for i in range(20)], 16, 8, 128, 16, 0),
+    ([900, 300, 256, 7] + [(i * 91) % 900 + 1 for i in range(30)], 16, 4, 64, 32, 300),   # (a window of 300 keys)
 ]
 
 
@@ -486,8 +489,8 @@ def test_decode_attention_token_rows_and_batch_independence():
 
 
 def test_decode_attention_gives_the_same_bits_in_every_block_shape():
-    """The kernel picks warps per block and stages from the step's size; a request's
-    output must not notice (1, 20, 26 and 30 requests reach its four shapes on 148 SMs)."""
+    """The kernel gives a piece a block of eight warps or one warp, by the step's size; a request's
+    output must not notice (1 request has fewer pieces than a GPU has SMs, 20, 26 and 30 have more)."""
     H, Hk, D, S = 16, 8, 128, 16
     lens = [1000] + [(i * 43) % 1000 + 1 for i in range(29)]
     q, kp, vp, bt, sot, pos, want = paged_case(torch.bfloat16, [(n - 1, 1) for n in lens], H, Hk, D, S, 0, seed=15)
@@ -934,6 +937,17 @@ def test_skinny_product_with_batches_that_are_not_whole(K, variant):
     s = size.view(M, N // 16, 2, 8)
     bound = (K + 2) * 2.0 ** -24 * 2 * (s[:, :, 0] * s[:, :, 1]).reshape(M, -1)
     assert ((gated - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("N", [4736, 4752, 7104, 7120, 9472, 9488, 13312])
+@pytest.mark.parametrize("K", [1280, 5120])
+def test_skinny_product_where_the_choice_of_warps_turns(N, K):
+    """Numbers of tiles around whole rounds of a B200's SMs (two, three and four blocks each), where the choice between four, five and
+    eight warps turns.  The bound is the one above."""
+    g = torch.Generator().manual_seed(N)
+    a, w = torch.randn(3, K, generator=g).bfloat16().to(DEV), torch.randn(N, K, generator=g).bfloat16().to(DEV)
+    out = ops().gemm_skinny(a, w, None, torch.float32).double()
+    assert ((out - a.double() @ w.double().T).abs() <= K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)).all()
 
 
 @pytest.mark.parametrize("columns", [16, 48, 128, 144, 176, 208, 240, 256])
