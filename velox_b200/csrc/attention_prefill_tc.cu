@@ -30,9 +30,9 @@
 //               tiled TMA loads (128-byte swizzle), one 16-key x 64-column box per
 //               lane, into two shared-memory buffers each; the two query tiles once
 //               (warp 11).
-// Registers move from warps 8-11 to the softmax warps (setmaxnreg).  In the steady
-// state the tensor core sets the pace: 32 products of 128 x 128 x 16 per key tile
-// take about 3,450 cycles, of which a softmax thread is busy for 1,830.
+// Registers move from warps 8-11 to the softmax warps (setmaxnreg).  The two query tiles' softmaxes (a thread is busy for
+// 1,830 cycles a key tile) and the 32 products of 128 x 128 x 16 per key tile take turns; with the products issued by an elected
+// lane (tc_elect) 1,000 tokens on 15,000 keys take 261 us (274 under `lane == 0`), 8,192 tokens 666 (689).
 //
 // Keys past the request's last key and below its window are masked; the values of a
 // tile that reaches past the last key are cleared in shared memory first, because a
@@ -41,9 +41,7 @@
 // Every wait on an mbarrier is bounded.  If one runs out the block records a code
 // in the caller's error word, the other roles run out of their own bounded waits,
 // and the block frees its tensor memory and returns.
-#include <cuda.h>
-
-#include "common.cuh"
+#include "tcgen05_gemm.cuh"
 
 #define PT_ROWS 128
 #define PT_KEYS 128
@@ -86,27 +84,20 @@ __device__ __forceinline__ void pt_tma_load_2d(unsigned dst, const CUtensorMap* 
 // Shared-memory descriptors, 128-byte swizzle, version 1.  K-major (Q and K: rows
 // 128 bytes apart, groups of 8 rows 1024 bytes apart); MN-major (V: the 64-column
 // halves 16 KB apart = leading offset, groups of 8 keys 1024 bytes apart).
-__device__ __forceinline__ unsigned long long pt_desc_kmajor(unsigned addr) {
-    return (unsigned long long)((addr >> 4) & 0x3FFF) | (1ull << 16) | ((unsigned long long)(1024 >> 4) << 32) |
-           (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ unsigned long long pt_desc_mnmajor(unsigned addr) {
-    return (unsigned long long)((addr >> 4) & 0x3FFF) | ((unsigned long long)(PT_HALF_BYTES >> 4) << 16) |
-           ((unsigned long long)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ void pt_mma_ss(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
-                                          unsigned idesc, unsigned accumulate) {
+// Their lower words; the upper one is TC_DESC_HI for both.
+__device__ __forceinline__ unsigned pt_kmajor(unsigned addr) { return tc_desc_lo(addr); }
+__device__ __forceinline__ unsigned pt_mnmajor(unsigned addr) { return ((addr >> 4) & 0x3FFF) | ((unsigned)(PT_HALF_BYTES >> 4) << 16); }
+__device__ __forceinline__ void pt_mma_ss(unsigned tmem_d, unsigned a_lo, unsigned b_lo, unsigned idesc, unsigned accumulate) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(TC_DESC_HI) : "memory");
 }
-__device__ __forceinline__ void pt_mma_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc, unsigned idesc,
-                                          unsigned accumulate) {
+__device__ __forceinline__ void pt_mma_ts(unsigned tmem_d, unsigned tmem_a, unsigned b_lo, unsigned idesc, unsigned accumulate) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}\n"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+        "{\n .reg .pred p;\n .reg .b64 b;\n setp.ne.b32 p, %4, 0;\n mov.b64 b, {%2, %5};\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(TC_DESC_HI) : "memory");
 }
 __device__ __forceinline__ float pt_ex2(float x) {
     float y;
@@ -230,7 +221,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
     }
     pdl_wait();
     pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // Blocks are handed out in the order of blockIdx.x: the longest first (the last tokens of a prompt), over
     // all kv heads, so that the short ones fill the gaps at the end (with the kv head in blockIdx.y a head's
     // short blocks would come before the next head's long ones: 2,048 tokens took 50 instead of 34 us by the
@@ -402,7 +393,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
         }
     } else {
         // ---------------- tensor core ----------------
-        if (lane == 0) {
+        {   // (the whole warp, one elected lane issues: see tc_elect)
             // S = Q K^T: float32 out, bf16 A and B, both K-major, N = 128 keys, M = 128 rows
             const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(PT_KEYS >> 3) << 17) |
                                      ((unsigned)(PT_ROWS >> 4) << 24);
@@ -411,13 +402,15 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                                      ((unsigned)(PT_ROWS >> 4) << 24);
             auto issue_s = [&](int q, int t) {   // scores of query tile q on key tile t, over the tile's scores/probabilities
                 const unsigned qa = pt_smem_u32(q_s + q * PT_TILE_BYTES), ka = pt_smem_u32(k_s + ((t - lo) & 1) * PT_TILE_BYTES);
+                const unsigned qd = pt_kmajor(qa), kd = pt_kmajor(ka);
+                if (tc_elect()) {
 #pragma unroll
-                for (int k = 0; k < PT_D / 16; ++k) {
-                    const unsigned o = (unsigned)((k >> 2) * PT_HALF_BYTES + (k & 3) * 32);
-                    pt_mma_ss(tmem_base + (unsigned)(q * 128), pt_desc_kmajor(qa + o), pt_desc_kmajor(ka + o), idesc_s,
-                              k > 0 ? 1u : 0u);
+                    for (int k = 0; k < PT_D / 16; ++k) {
+                        const unsigned o = (unsigned)((k >> 2) * PT_HALF_BYTES + (k & 3) * 32) >> 4;
+                        pt_mma_ss(tmem_base + (unsigned)(q * 128), qd + o, kd + o, idesc_s, k > 0 ? 1u : 0u);
+                    }
+                    pt_commit(pt_smem_u32(&bars.s_full[q]));
                 }
-                pt_commit(pt_smem_u32(&bars.s_full[q]));
             };
             bool ok = true;
             // the first key tile's scores
@@ -432,7 +425,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                     }
                 }
             }
-            if (ok) pt_commit(pt_smem_u32(&bars.k_empty[0]));
+            if (ok && tc_elect()) pt_commit(pt_smem_u32(&bars.k_empty[0]));
             for (int t = lo; t < hi && ok; ++t) {
                 const int u = t - lo, b = u & 1;
                 bool have_v = false, have_k = false;
@@ -445,18 +438,20 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                         ok = ok && pt_mbar_wait(pt_smem_u32(&bars.p_ready[q]), (unsigned)(n & 1));
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                        const unsigned va = pt_smem_u32(v_s + b * PT_TILE_BYTES);
+                        const unsigned vd = pt_mnmajor(pt_smem_u32(v_s + b * PT_TILE_BYTES));
+                        if (tc_elect()) {
 #pragma unroll
-                        for (int k = 0; k < PT_KEYS / 16; ++k)   // 16 keys a step: 8 columns of packed P, 2 KB of V
-                            pt_mma_ts(tmem_base + (unsigned)(256 + q * 128), tmem_base + (unsigned)(q * 128 + k * 8),
-                                      pt_desc_mnmajor(va + (unsigned)(k * 2048)), idesc_o, (n > 0 || k > 0) ? 1u : 0u);
-                        if (EXT) {
+                            for (int k = 0; k < PT_KEYS / 16; ++k)   // 16 keys a step: 8 columns of packed P, 2 KB of V
+                                pt_mma_ts(tmem_base + (unsigned)(256 + q * 128), tmem_base + (unsigned)(q * 128 + k * 8), vd + (unsigned)(k * 2048 >> 4),
+                                          idesc_o, (n > 0 || k > 0) ? 1u : 0u);
+                            if (EXT) {
 #pragma unroll
-                            for (int k = 0; k < PT_KEYS / 16; ++k)   // the probabilities' low halves, 64 columns on
-                                pt_mma_ts(tmem_base + (unsigned)(256 + q * 128), tmem_base + (unsigned)(q * 128 + 64 + k * 8),
-                                          pt_desc_mnmajor(va + (unsigned)(k * 2048)), idesc_o, 1u);
+                                for (int k = 0; k < PT_KEYS / 16; ++k)   // the probabilities' low halves, 64 columns on
+                                    pt_mma_ts(tmem_base + (unsigned)(256 + q * 128), tmem_base + (unsigned)(q * 128 + 64 + k * 8),
+                                              vd + (unsigned)(k * 2048 >> 4), idesc_o, 1u);
+                            }
+                            pt_commit(pt_smem_u32(&bars.pv_done[q]));
                         }
-                        pt_commit(pt_smem_u32(&bars.pv_done[q]));
                     }
                     if (t + 1 >= tile_a[q] && t + 1 < tile_b[q]) {
                         // the next scores of this query tile go where its probabilities were: the tensor core
@@ -468,10 +463,12 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                     }
                 }
                 if (!ok) break;
-                pt_commit(pt_smem_u32(&bars.v_empty[b]));
-                if (t + 1 < hi) pt_commit(pt_smem_u32(&bars.k_empty[b ^ 1]));
+                if (tc_elect()) {
+                    pt_commit(pt_smem_u32(&bars.v_empty[b]));
+                    if (t + 1 < hi) pt_commit(pt_smem_u32(&bars.k_empty[b ^ 1]));
+                }
             }
-            if (!ok) { failed = 1; atomicExch(error, 12); }
+            if (!ok && lane == 0) { failed = 1; atomicExch(error, 12); }
         }
     }
     } else {

@@ -60,7 +60,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     unsigned char* tiles = (unsigned char*)(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
     pdl_wait();
     pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int nkb = (K + TC_BK - 1) / TC_BK;
     // Tiles are numbered with the row tile running fastest, so that blocks working
     // at the same time share a tile of W and walk over the rows of A (which stays
@@ -93,68 +93,55 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (warp == 0) {
         // ---- producer: one continuous stream of stages over all of this block's tiles ----
-        if (lane == 0) {
-            int it = 0;
-            for (int ti = 0; ti < my_tiles && !failed; ++ti) {
-                const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
-                const int rt = tile % mtiles;
-                const int m0 = row_tiles ? row_tiles[3 * rt + 1] : rt * TC_BM;
-                const int n0 = (tile / mtiles) * bn + (row_tiles ? row_tiles[3 * rt] * N : 0);   // (row of W)
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (it >= STAGES &&
-                        !tc_mbar_wait(tc_smem_u32(&empty_bar[s]), (unsigned)(((it / STAGES) - 1) & 1))) {
-                        failed = 1;
-                        atomicExch(error, TC_ERR_PRODUCER);
-                        break;
-                    }
-                    const unsigned bar = tc_smem_u32(&full_bar[s]);
-                    tc_mbar_expect_tx(bar, A_BYTES + (unsigned)bn * (TC_BK * 2));
-                    unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
-                    tc_tma_load_2d(tc_smem_u32(st), &map_a, kb * TC_BK, m0, bar);
-                    tc_tma_load_2d(tc_smem_u32(st + A_BYTES), &map_w, kb * TC_BK, n0, bar);
+        int s = 0;
+        unsigned phase = 1;   // (the first time round a stage is free: the phase before the first has ended)
+        for (int ti = 0; ti < my_tiles; ++ti) {
+            const int tile = (int)blockIdx.x + ti * (int)gridDim.x;
+            const int rt = tile % mtiles;
+            const int m0 = row_tiles ? row_tiles[3 * rt + 1] : rt * TC_BM;
+            const int n0 = (tile / mtiles) * bn + (row_tiles ? row_tiles[3 * rt] * N : 0);   // (row of W)
+            for (int kb = 0; kb < nkb; ++kb) {
+                if (!tc_mbar_wait(tc_smem_u32(&empty_bar[s]), phase)) {
+                    if (lane == 0) { failed = 1; atomicExch(error, TC_ERR_PRODUCER); }
+                    ti = my_tiles;
+                    break;
                 }
+                if (tc_elect()) {
+                    const unsigned bar = tc_smem_u32(&full_bar[s]), st = tc_smem_u32(tiles) + s * STAGE_BYTES;
+                    tc_mbar_expect_tx(bar, A_BYTES + (unsigned)bn * (TC_BK * 2));
+                    tc_tma_load_2d(st, &map_a, kb * TC_BK, m0, bar);
+                    tc_tma_load_2d(st + A_BYTES, &map_w, kb * TC_BK, n0, bar);
+                }
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
         }
     } else if (warp == 1) {
         // ---- tensor core: tile ti accumulates into buffer ti & 1 ----
-        if (lane == 0) {
-            // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = bn, M = 128
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) |
-                                   ((unsigned)(TC_BM >> 4) << 24);
-            int it = 0;
-            for (int ti = 0; ti < my_tiles && !failed; ++ti) {
-                const int buf = ti & 1;
-                // the epilogue must have emptied this buffer (it last held tile ti - 2)
-                if (ti >= 2 && !tc_mbar_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1))) {
-                    failed = 1;
-                    atomicExch(error, TC_ERR_MMA);
-                    break;
-                }
+        // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = bn, M = 128
+        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(TC_BM >> 4) << 24);
+        int s = 0;
+        unsigned phase = 0;
+        bool ok = true;
+        for (int ti = 0; ok && ti < my_tiles; ++ti) {
+            const int buf = ti & 1;
+            // the epilogue must have emptied this buffer (it last held tile ti - 2)
+            ok = ti < 2 || tc_mbar_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1));
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const unsigned tmem_d = tmem_base + (unsigned)(buf * BN);
+            for (int kb = 0; ok && kb < nkb; ++kb) {
+                ok = tc_mbar_wait(tc_smem_u32(&full_bar[s]), phase);
+                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const unsigned tmem_d = tmem_base + (unsigned)(buf * BN);
-                bool ok = true;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!tc_mbar_wait(tc_smem_u32(&full_bar[s]), (unsigned)((it / STAGES) & 1))) {
-                        failed = 1;
-                        atomicExch(error, TC_ERR_MMA);
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const unsigned a_addr = tc_smem_u32(tiles + (size_t)s * STAGE_BYTES);
-                    const unsigned long long adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + A_BYTES);
-#pragma unroll
-                    for (int k4 = 0; k4 < TC_BK / 16; ++k4)   // 32 bytes further along K inside the swizzle atom
-                        tc_mma(tmem_d, adesc + (unsigned long long)(k4 * 2), bdesc + (unsigned long long)(k4 * 2),
-                               idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
+                const unsigned a_lo = tc_desc_lo(tc_smem_u32(tiles) + s * STAGE_BYTES);
+                if (tc_elect()) {
+                    tc_mma_run<1, TC_BK / 16>(tmem_d, a_lo, a_lo + (A_BYTES >> 4), idesc, kb > 0);
                     tc_commit(tc_smem_u32(&empty_bar[s]));   // the stage is free once these have read it
                 }
-                if (!ok) break;
-                tc_commit(tc_smem_u32(&acc_full[buf]));      // the accumulator is complete once all have finished
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
+            if (ok && tc_elect()) tc_commit(tc_smem_u32(&acc_full[buf]));   // the accumulator is complete once all have finished
         }
+        if (!ok && lane == 0) { failed = 1; atomicExch(error, TC_ERR_MMA); }
     } else {
         // ---- epilogue: warp w reads lanes 32 * (w % 4) .. + 31 of tensor memory ----
         const int quarter = warp & 3;

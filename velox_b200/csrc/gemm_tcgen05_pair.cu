@@ -30,52 +30,13 @@
 // memory and return.
 //
 // Sizes: K a multiple of 8, rows of A, W and C 16-byte aligned, N a multiple of 16.
-#include "tcgen05_gemm.cuh"
+#include "tcgen05_pair.cuh"
 
 #define TP_BN 256
 #define TP_HALF 128   // rows of W a block loads
 #define TP_ERR_PRODUCER 4
 #define TP_ERR_MMA 5
 #define TP_ERR_EPILOGUE 6
-
-__device__ __forceinline__ unsigned tp_cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-// The address, in the cluster's shared window, of `addr` in the block of rank `rank`.
-__device__ __forceinline__ unsigned tp_map_to_rank(unsigned addr, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void tp_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-// A tiled load into this block's shared memory whose bytes are counted on an mbarrier
-// that may live in the other block of the pair (`bar`: an address in the cluster's window).
-__device__ __forceinline__ void tp_tma_load_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void tp_mma(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
-                                       unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}\n"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-// One arrival, when the products issued so far have completed, on the mbarrier at this
-// offset in both blocks of the pair.
-__device__ __forceinline__ void tp_commit_both(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-                 ::"r"(bar), "h"((unsigned short)3) : "memory");
-}
-__device__ __forceinline__ void tp_arrive_remote(unsigned bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
 
 template <int STAGES, bool GATED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS)
@@ -90,7 +51,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     unsigned char* tiles = (unsigned char*)(((uintptr_t)tp_smem_raw + 1023) & ~(uintptr_t)1023);
     pdl_wait();
     pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const unsigned rank = tp_cluster_rank();
     const int nkb = (K + TC_BK - 1) / TC_BK;
     const int mtiles = (M + 2 * TC_BM - 1) / (2 * TC_BM), ntiles = (N + TP_BN - 1) / TP_BN;
@@ -122,65 +83,55 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
     if (warp == 0) {
         // ---- producer (both blocks): this block's halves of every stage ----
-        if (lane == 0) {
-            int it = 0;
-            for (int ti = 0; ti < my_tiles && !failed; ++ti) {
-                const int tile = pair + ti * pairs;
-                const int m0 = (tile % mtiles) * (2 * TC_BM) + (int)rank * TC_BM;
-                const int n0 = (tile / mtiles) * TP_BN + (int)rank * TP_HALF;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (it >= STAGES &&
-                        !tc_mbar_wait(tc_smem_u32(&empty_bar[s]), (unsigned)(((it / STAGES) - 1) & 1))) {
-                        failed = 1;
-                        atomicExch(error, TP_ERR_PRODUCER);
-                        break;
-                    }
-                    if (rank == 0) tc_mbar_expect_tx(tc_smem_u32(&full_bar[s]), 2 * STAGE_BYTES);
-                    const unsigned bar = tp_map_to_rank(tc_smem_u32(&full_bar[s]), 0);
-                    unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
-                    tp_tma_load_2d(tc_smem_u32(st), &map_a, kb * TC_BK, m0, bar);
-                    tp_tma_load_2d(tc_smem_u32(st + A_BYTES), &map_w, kb * TC_BK, n0, bar);
+        int s = 0;
+        unsigned phase = 1;   // (the first time round a stage is free: the phase before the first has ended)
+        for (int ti = 0; ti < my_tiles; ++ti) {
+            const int tile = pair + ti * pairs;
+            const int m0 = (tile % mtiles) * (2 * TC_BM) + (int)rank * TC_BM;
+            const int n0 = (tile / mtiles) * TP_BN + (int)rank * TP_HALF;
+            for (int kb = 0; kb < nkb; ++kb) {
+                if (!tc_mbar_wait(tc_smem_u32(&empty_bar[s]), phase)) {
+                    if (lane == 0) { failed = 1; atomicExch(error, TP_ERR_PRODUCER); }
+                    ti = my_tiles;
+                    break;
                 }
+                if (tc_elect()) {
+                    if (rank == 0) tc_mbar_expect_tx(tc_smem_u32(&full_bar[s]), 2 * STAGE_BYTES);
+                    const unsigned bar = tp_map_to_rank(tc_smem_u32(&full_bar[s]), 0), st = tc_smem_u32(tiles) + s * STAGE_BYTES;
+                    tp_tma_load_2d(st, &map_a, kb * TC_BK, m0, bar);
+                    tp_tma_load_2d(st + A_BYTES, &map_w, kb * TC_BK, n0, bar);
+                }
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
         }
     } else if (warp == 1) {
         // ---- tensor cores of the pair, driven by the leading block ----
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             // instruction descriptor: float32 accumulator, bfloat16 A and B, both K-major, N = 256, M = 256
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TP_BN >> 3) << 17) |
                                    ((unsigned)((2 * TC_BM) >> 4) << 24);
-            int it = 0;
-            for (int ti = 0; ti < my_tiles && !failed; ++ti) {
+            int s = 0;
+            unsigned phase = 0;
+            bool ok = true;
+            for (int ti = 0; ok && ti < my_tiles; ++ti) {
                 const int buf = ti & 1;
-                if (ti >= 2 && !tc_mbar_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1))) {
-                    failed = 1;
-                    atomicExch(error, TP_ERR_MMA);
-                    break;
-                }
+                ok = ti < 2 || tc_mbar_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1));
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const unsigned tmem_d = tmem_base + (unsigned)(buf * TP_BN);
-                bool ok = true;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!tc_mbar_wait(tc_smem_u32(&full_bar[s]), (unsigned)((it / STAGES) & 1))) {
-                        failed = 1;
-                        atomicExch(error, TP_ERR_MMA);
-                        ok = false;
-                        break;
-                    }
+                for (int kb = 0; ok && kb < nkb; ++kb) {
+                    ok = tc_mbar_wait(tc_smem_u32(&full_bar[s]), phase);
+                    if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                    const unsigned a_addr = tc_smem_u32(tiles + (size_t)s * STAGE_BYTES);
-                    const unsigned long long adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + A_BYTES);
-#pragma unroll
-                    for (int k4 = 0; k4 < TC_BK / 16; ++k4)
-                        tp_mma(tmem_d, adesc + (unsigned long long)(k4 * 2), bdesc + (unsigned long long)(k4 * 2),
-                               idesc, (kb > 0 || k4 > 0) ? 1u : 0u);
-                    tp_commit_both(tc_smem_u32(&empty_bar[s]));
+                    const unsigned a_lo = tc_desc_lo(tc_smem_u32(tiles) + s * STAGE_BYTES);
+                    if (tc_elect()) {
+                        tc_mma_run<2, TC_BK / 16>(tmem_d, a_lo, a_lo + (A_BYTES >> 4), idesc, kb > 0);
+                        tp_commit_mask(tc_smem_u32(&empty_bar[s]), 3);
+                    }
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
                 }
-                if (!ok) break;
-                tp_commit_both(tc_smem_u32(&acc_full[buf]));
+                if (ok && tc_elect()) tp_commit_mask(tc_smem_u32(&acc_full[buf]), 3);
             }
+            if (!ok && lane == 0) { failed = 1; atomicExch(error, TP_ERR_MMA); }
         }
     } else {
         // ---- epilogue (both blocks): warp w reads lanes 32 * (w % 4) .. + 31 of its block's tensor memory ----

@@ -39,16 +39,33 @@ __device__ __forceinline__ void tc_tma_load_2d(unsigned dst, const CUtensorMap* 
 // Shared-memory descriptor of a K-major tile with 128-byte swizzle: rows 128 bytes
 // apart, groups of 8 rows 1024 bytes apart (the tile is exactly one swizzle atom
 // wide), version 1, layout type 2 (128-byte swizzle).
-__device__ __forceinline__ unsigned long long tc_smem_desc(unsigned addr) {
-    return (unsigned long long)((addr >> 4) & 0x3FFF) | (1ull << 16) | ((unsigned long long)(1024 >> 4) << 32) |
-           (1ull << 46) | (2ull << 61);
+// In two words: the upper one is the same for every tile.
+#define TC_DESC_HI 0x40004040u
+__device__ __forceinline__ unsigned tc_desc_lo(unsigned addr) { return ((addr >> 4) & 0x3FFF) | (1u << 16); }
+// One lane of the warp, the same every time.  A role that one thread has (loads, products) is run by its whole warp, and the
+// elected lane issues: its operands then stay in the warp's uniform registers.  Under `if (lane == 0)` every operand of every
+// instruction is moved there first: gated products with short tiles took up to 1.3 times as long (777 x 6144 x 1024 on tiles of 160
+// columns 21.2 us, 18.9 so; 2048 x 19456 x 2560 by pairs 154, 141; 2048 x 24576 x 4096 by pairs 288, 273).
+__device__ __forceinline__ bool tc_elect() {
+    unsigned p;
+    asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+    return p != 0;
 }
-__device__ __forceinline__ void tc_mma(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
-                                       unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+// STEPS products of 16 k each (32 bytes further along K inside the swizzle atom) from descriptors given by their lower words;
+// the first adds to the accumulator if `add` is not 0, the others always.
+template <int CG, int STEPS>
+__device__ __forceinline__ void tc_mma_run(unsigned tmem_d, unsigned a_lo, unsigned b_lo, unsigned idesc, unsigned add) {
+#pragma unroll
+    for (int k = 0; k < STEPS; ++k) {
+        if (CG == 2)
+            asm volatile("{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+                         " tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %3, p;\n}\n"
+                         ::"r"(tmem_d), "r"(a_lo + 2 * k), "r"(b_lo + 2 * k), "r"(idesc), "r"(k ? 1u : add), "r"(TC_DESC_HI) : "memory");
+        else
+            asm volatile("{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+                         " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
+                         ::"r"(tmem_d), "r"(a_lo + 2 * k), "r"(b_lo + 2 * k), "r"(idesc), "r"(k ? 1u : add), "r"(TC_DESC_HI) : "memory");
+    }
 }
 __device__ __forceinline__ void tc_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
