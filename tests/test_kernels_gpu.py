@@ -307,6 +307,41 @@ def test_gemm_float32_error_follows_the_parts(K):
     assert err <= 0.6 * 2.0 ** -24 * math.sqrt(length / 4 + 1 + (parts + 1) / 2), err
 
 
+@pytest.mark.parametrize("N,K,pad", [(1, 257, 0), (127, 320, 4), (129, 1025, 3), (1024, 2049, 3), (32768, 264, 0), (256, 4096, 0)])
+def test_gemm_float32_by_three_parts(N, K, pad):
+    """The 32-bit product on the tensor cores (k above 256) at the edges of its tiles (16, 32, 64, 128 rows, 128 columns), runs (32 k),
+    chunks (64) and parts.  A term passes at most ten additions in its accumulator, each cut off below 2^-23 of the sum of the terms' sizes, the
+    run's among those of its part and the part's, rounded to 2^-24; the products left out are below 3 x 2^-24."""
+    parts = min(8, max(1, K // 256))
+    steps = 2 * 10 + -(-K // (32 * parts)) + 2 + parts + 3
+    w = rnd((N, K + pad), torch.float32, 7)[:, :K]
+    a = rnd((257, K + pad), torch.float32, 6)[:, :K]
+    whole = ops().gemm_nt_simt(a, w)
+    assert (abs(f64(whole) - f64(a) @ f64(w).T) <= steps * 2.0 ** -24 * (abs(f64(a)) @ abs(f64(w)).T)).all()
+    for M in (1, 15, 16, 17, 31, 33, 64, 65, 127, 128, 129):
+        assert torch.equal(ops().gemm_nt_simt(a[257 - M:], w), whole[257 - M:]), M
+
+
+def test_gemm_float32_infinities_nan_and_tiny_sums():
+    """Infinities, NaN, sums that overflow and operands so small that their parts vanish in bfloat16: what multiply-adds give."""
+    K = 512
+    a, w = rnd((5, K), torch.float32, 1), rnd((70, K), torch.float32, 2)
+    a[1, 7], w[3, 9], w[4, 10], w[6], w[8] = math.inf, -math.inf, math.nan, 0.0, 1.0
+    a[2] = 3e38
+    a[3] *= 1e-20
+    w[5] = w[5].abs() * 1e-16
+    got = f64(ops().gemm_nt_simt(a, w))
+    assert got[2, 8] == math.inf
+    rows = [0, 1, 3, 4]
+    got, A, W = got[rows], f64(a)[rows], f64(w)
+    with np.errstate(invalid="ignore"):
+        want, size = A @ W.T, abs(A) @ abs(W).T
+    assert np.array_equal(np.isnan(got), np.isnan(want))     # (infinity times 0 in row 1, column 6; the NaN's column)
+    infinite, finite = np.isinf(want), np.isfinite(want)
+    assert infinite.any() and np.array_equal(got[infinite], want[infinite])
+    assert (abs(got[finite] - want[finite]) <= (K * 2.0 ** -24 * size + K * 2.0 ** -149)[finite]).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (12, 1000, 777), (99, 4096, 1024), (3, 40000, 300)])
 def test_gemm_float32_waits_for_a_w_that_was_just_written(M, N, K):
     """W written by the kernel launched just before, in memory that holds NaN until then: the products (plain, per head, of a batch)

@@ -1,8 +1,8 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]): the plain matrix product.
 //
-// Multiply-adds on the CUDA cores in float32, no tensor cores, no reduced
-// precision mode.  float32 operands, the 32-bit path's, go to the kernel in
-// gemm_f32.cu; the kernel here takes bfloat16 ones and is the reference against
+// float32 operands, the 32-bit path's, go to the kernels in gemm_f32_tc.cu and gemm_f32.cu.
+// The kernel here takes bfloat16 ones (multiply-adds on the CUDA cores in float32, no tensor
+// cores, no reduced precision mode) and is the reference against
 // which the tensor-core products are checked.  The order of a sum is fixed by K alone
 // (here: ascending k), so a row's result does not depend on how many rows the call has.  Any M, N, K.
 #include "common.cuh"
@@ -77,17 +77,25 @@ gemm_nt_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const fl
 // in_dtype: element type of A and W; out_dtype: element type of C.
 // A batch of `batch` products: member z reads A + z sa, W + z sw and writes C + z sc (strides in elements).
 // `w_ready`: W (a model's weights, say) is not something the kernel launched just before this one writes; the float32 product
-// then asks for its first tiles before it waits for that kernel.
-extern "C" int vx_gemm_nt_simt_ready(const void* A, const void* W, const float* bias, void* C, int M, int N,
-                                     int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
-                                     long long sc, int in_dtype, int out_dtype, int w_ready, cudaStream_t stream) {
+// then asks for its first chunks before it waits for that kernel.  `error` (may be null): a device int that the float32 product sets if it
+// gives up its wait for the tensor core; its results are NaN then.
+//
+// Which float32 product: N and K alone say (a row's result must not depend on how many rows the call has).  The tensor cores, except
+// for k up to 256, where they have no time to get going (1 x 1024 x 256: multiply-adds 3.5 us, tensor cores 6.6; 37 x 64 x 64 3.8, 3.5), and
+// for more than 32,768 columns, a vocabulary's head, of which a step wants a few rows (4 x 151936 x 1024: 144, 193).
+extern "C" int vx_gemm_nt_simt_checked(const void* A, const void* W, const float* bias, void* C, int M, int N,
+                                       int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
+                                       long long sc, int in_dtype, int out_dtype, int w_ready, int* error, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || batch <= 0) return VX_OK;
     if (K <= 0 || lda < K || ldw < K || ldc < N) return VX_ERR_SHAPE;
     dim3 grid((N + GS_BN - 1) / GS_BN, (M + GS_BM - 1) / GS_BM, batch);
     if (grid.y > 65535 || batch > 65535) return VX_ERR_LIMIT;
-    if (in_dtype == VX_F32 && out_dtype == VX_F32)
-        return vx_gemm_f32((const float*)A, (const float*)W, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready,
-                           stream);
+    if (in_dtype == VX_F32 && out_dtype == VX_F32) {
+        const float *a = (const float*)A, *w = (const float*)W;
+        if (K > 256 && N <= 32768)
+            return vx_gemm_f32_tc(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready, error, stream);
+        return vx_gemm_f32(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready, stream);
+    }
     if (in_dtype == VX_BF16 && out_dtype == VX_BF16)
         VX_LAUNCH_K(VX_K_GEMM, (gemm_nt_simt_kernel<bf16, bf16>), grid, 256, 0, stream, (const bf16*)A, (const bf16*)W, bias, (bf16*)C, M, N, K, lda, ldw, ldc, sa, sw, sc);
     else if (in_dtype == VX_BF16 && out_dtype == VX_F32)
@@ -96,6 +104,12 @@ extern "C" int vx_gemm_nt_simt_ready(const void* A, const void* W, const float* 
         return VX_ERR_DTYPE;
     VX_LAUNCH_CHECK();
     return VX_OK;
+}
+
+extern "C" int vx_gemm_nt_simt_ready(const void* A, const void* W, const float* bias, void* C, int M, int N,
+                                     int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
+                                     long long sc, int in_dtype, int out_dtype, int w_ready, cudaStream_t stream) {
+    return vx_gemm_nt_simt_checked(A, W, bias, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, in_dtype, out_dtype, w_ready, nullptr, stream);
 }
 
 extern "C" int vx_gemm_nt_simt_batched(const void* A, const void* W, const float* bias, void* C, int M, int N,

@@ -148,6 +148,7 @@ def _declare(lib) -> None:
         "vx_sample": [P, I, I, I, P, P, P, P, P],
         "vx_qk_norm_rope_kv_pairs": [P, I, P, P, F, P, I, P, P, P, P, I, I, I, I, I, I, I, I, P],
         "vx_paged_attention_generic_cap": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, P],
+        "vx_gemm_nt_simt_checked": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, I, P, P],
         "vx_gemm_nt_simt_batched": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, P],
         "vx_linear_attention_walk": [P, I, I, I, I, P, P, I, F, P, I, I, P, F, F, P, P, P, P, I, I, I, I, I, P],
         "vx_linear_attention_walk_parts": [P, I, I, I, I, P, P, I, F, P, I, I, P, F, F, P, P, P, P, I, I, I, I, I, I, P],
@@ -1028,9 +1029,20 @@ def paged_prefill_attention_tc(q: torch.Tensor, q_row_stride: int, k_pool, v_poo
     return out
 
 
+def _simt(a, w, bias, out, m, n, k, lda, ldw, ldc, batch, sa, sw, sc, w_ready, what) -> None:
+    """(The float32 product's waits for the tensor core are bounded: it reports into the error word.)"""
+    exact = a.dtype == torch.float32
+    _check(library().vx_gemm_nt_simt_checked(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, lda, ldw, ldc, batch, sa, sw, sc,
+                                             dtype_code(a.dtype), dtype_code(out.dtype), 1 if w_ready else 0,
+                                             _ptr(_error_word(a.device)) if exact else None, _stream()), what)
+    if exact:
+        note_bounded_wait()
+
+
 def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None,
                  w_ready: bool = False) -> torch.Tensor:
-    """a [M,K] times w [N,K] transposed, float32 multiply-adds on the CUDA cores.  `w_ready` says that `w` is not something the
+    """a [M,K] times w [N,K] transposed: float32 multiply-adds on the CUDA cores, or (float32 operands, k above 256) the tensor cores
+    with every operand in three bfloat16 parts, which is no less exact.  `w_ready` says that `w` is not something the
     kernel launched just before this one writes (a model's weights never are): its first tiles may then be fetched before the wait for
     that kernel."""
     _dev(a, w, bias)
@@ -1042,8 +1054,7 @@ def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optiona
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm: float32 bias of N elements")
     out = torch.empty((m, n), dtype=out_dtype, device=a.device)
-    _check(library().vx_gemm_nt_simt_ready(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, a.stride(0), w.stride(0), n, 1, 0, 0, 0,
-                                           dtype_code(a.dtype), dtype_code(out_dtype), 1 if w_ready else 0, _stream()), "gemm_nt_simt")
+    _simt(a, w, bias, out, m, n, k, a.stride(0), w.stride(0), n, 1, 0, 0, 0, w_ready, "gemm_nt_simt")
     return out
 
 
@@ -1052,7 +1063,7 @@ GEMM_HEADS_FEW_ROWS = 8   # rows up to which the products per head take the kern
 
 def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_ready: bool = False) -> torch.Tensor:
     """One product per head: out[:, h, :] = a[:, h, :] w[h]^T with a [M, H, K], w [H, N, K] (contiguous), out [M, H, N];
-    `a` and `out` may be views into wider rows (their last dimension contiguous).  float32 multiply-adds (in float32, the
+    `a` and `out` may be views into wider rows (their last dimension contiguous).  Sums in float32, as in `gemm_nt_simt` (of float32 operands, the
     order of a sum is fixed by K alone, whatever the number of rows; bfloat16 steps of up to 8 rows take a kernel of their own, which
     always reads `w` as one that is ready).  `w_ready`: see `gemm_nt_simt`."""
     _dev(a, w, out)
@@ -1066,9 +1077,7 @@ def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, w_ready: boo
         _check(library().vx_gemm_few_rows_batched(_ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), k, out.stride(0), h, a.stride(1),
                                                   n * k, out.stride(1), dtype_code(out.dtype), _stream()), "gemm_few_rows_heads")
         return out
-    _check(library().vx_gemm_nt_simt_ready(_ptr(a), _ptr(w), None, _ptr(out), m, n, k, a.stride(0), k, out.stride(0), h,
-                                           a.stride(1), n * k, out.stride(1), dtype_code(a.dtype), dtype_code(out.dtype),
-                                           1 if w_ready else 0, _stream()), "gemm_nt_simt_heads")
+    _simt(a, w, None, out, m, n, k, a.stride(0), k, out.stride(0), h, a.stride(1), n * k, out.stride(1), w_ready, "gemm_nt_simt_heads")
     return out
 
 
@@ -1798,7 +1807,7 @@ def gemm_inputs(xs: torch.Tensor, w: torch.Tensor, seg_rows: int, out_dtype: tor
 
 def gemm_members(xs: torch.Tensor, ws: torch.Tensor, w_ready: bool = False) -> torch.Tensor:
     """A batch of products of one shape: out[i] = xs[i] ws[i]^T with xs [n, M, K], ws [n, N, K] (contiguous).  float32:
-    multiply-adds on the CUDA cores, the order of a sum fixed by K alone; bfloat16: the library product.  `w_ready`: see
+    the products of `gemm_nt_simt`, the order of a sum fixed by K alone; bfloat16: the library product.  `w_ready`: see
     `gemm_nt_simt`."""
     _dev(xs, ws)
     _need(xs.dim() == 3 and ws.dim() == 3 and xs.is_contiguous() and ws.is_contiguous() and xs.dtype == ws.dtype
@@ -1808,9 +1817,7 @@ def gemm_members(xs: torch.Tensor, ws: torch.Tensor, w_ready: bool = False) -> t
         _full_precision_sums()
         return torch.bmm(xs, ws.transpose(1, 2))
     out = torch.empty((n, m, ws.shape[1]), dtype=xs.dtype, device=xs.device)
-    _check(library().vx_gemm_nt_simt_ready(_ptr(xs), _ptr(ws), None, _ptr(out), m, ws.shape[1], k, k, k, ws.shape[1], n, m * k,
-                                           ws.shape[1] * k, m * ws.shape[1], dtype_code(xs.dtype), dtype_code(out.dtype),
-                                           1 if w_ready else 0, _stream()), "gemm_members")
+    _simt(xs, ws, None, out, m, ws.shape[1], k, k, k, ws.shape[1], n, m * k, ws.shape[1] * k, m * ws.shape[1], w_ready, "gemm_members")
     return out
 
 

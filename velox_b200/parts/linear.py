@@ -2,9 +2,10 @@
 (src/paged/qwen3.rs:120-132, 226-239).
 
 The one place where a matrix product is chosen:
-  float32   the engine's own multiply-add kernel on the CUDA cores: true 32-bit,
-            every output element summed over k in an order that K alone fixes, so a
-            row's result does not depend on the rows beside it.
+  float32   the engine's own kernels, true 32-bit: multiply-adds on the CUDA cores, or the
+            tensor cores with every operand in three bfloat16 parts (24 bits, no less exact);
+            N and K say which, and every output element is summed over k in an order that K alone
+            fixes, so a row's result does not depend on the rows beside it.
   bfloat16  the tensor-core product (see `matmul`).
 """
 from __future__ import annotations
