@@ -257,6 +257,40 @@ def test_attention_finds_one_far_key_among_hundreds(dtype, far):
     assert torch.allclose(out[0, :D].float(), vp[page, 0, off].float(), atol=5e-2)
 
 
+@pytest.mark.parametrize("H,Hk,D,Dv", [(4, 2, 128, 128), (3, 3, 64, 128), (10, 2, 36, 20), (8, 1, 128, 64)])
+def test_float32_attention_whatever_tokens_a_block_has(H, Hk, D, Dv):
+    """The 32-bit path of layers without a window: blocks of up to eight neighbouring tokens, whole rounds of 128 keys and remainders; with a
+    soft cap, a bias by distance, sinks and a gate.  Against the kernel that a window beyond all keys selects, whose sums have another
+    order (the tolerance of `close`), and every token alone bit for bit; what no token sees may be anything."""
+    S, lens = 16, [(1, 0), (1, 127), (1, 400), (13, 250), (40, 3), (9, 1000)]     # (new tokens, cached)
+    need = [-(-(n + c) // S) for n, c in lens]
+    bt = torch.zeros((len(lens), max(need)), dtype=torch.int32)
+    order, at = torch.randperm(sum(need), generator=torch.Generator().manual_seed(0)).to(torch.int32), 0
+    for i, n in enumerate(need):
+        bt[i, :n], at = order[at:at + n], at + n
+    k, v = rnd((sum(need), Hk, S, D), torch.float32, 1), rnd((sum(need), Hk, S, Dv), torch.float32, 2)
+    for i, (n, c) in enumerate(lens):     # what lies behind a request's last key
+        if (n + c) % S:
+            page = int(bt[i, need[i] - 1])
+            v[page, :, (n + c) % S:] = float("nan")
+            k[page, :, (n + c) % S:] = float("inf")
+    bt = bt.to(DEV)
+    seq = torch.tensor([i for i, (n, c) in enumerate(lens) for _ in range(n)], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([c + j for n, c in lens for j in range(n)], dtype=torch.int32, device=DEV)
+    T = len(pos)
+    q = rnd((T, H * D + H), torch.float32, 3)
+    more = dict(v_head_dim=Dv, softcap=20.0, bias_exponent=8.0, sinks=rnd((H,), torch.float32, 4), gate_col=H * D)
+
+    def run(q, seq, pos, window, **kw):
+        return ops().paged_attention_generic(q, q.shape[1], k, v, bt, seq, pos, D ** -0.5, window, H, Hk, D, len(pos), **kw)
+
+    for kw in (dict(v_head_dim=Dv), more):
+        whole = run(q, seq, pos, 0, **kw)
+        close(whole, f64(run(q, seq, pos, 4096, **kw)), torch.float32)
+        for t in range(T):
+            assert torch.equal(run(q[t:t + 1], seq[t:t + 1], pos[t:t + 1], 0, **kw)[0], whole[t]), t
+
+
 # ----------------------------------------------------------------------------
 @pytest.mark.parametrize("M,N,K", [(1, 53, 71), (37, 64, 16), (130, 129, 100), (5, 384, 96)])
 def test_gemm_simt_fp32(M, N, K):

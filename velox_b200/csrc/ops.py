@@ -181,6 +181,7 @@ def _declare(lib) -> None:
         "vx_stretch_log_decay_form": [P, I, F, P, P, I, I, I, P],
         "vx_head_norm_gate_heads": [P, P, I, P, I, P, I, I, I, F, I, I, I, P],
         "vx_paged_attention_generic_chunk": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, I, I, I, P],
+        "vx_paged_attention_generic_requests": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, I, I, I, I, P],
         "vx_biased_attention_chunk": [P, I, P, P, P, I, P, P, P, P, P, I, F, F, I, I, I, I, I, I, I, I, I, P, I, P, I, F, I, I, I, P],
         "vx_gemm_skinny_act": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P],
         "vx_gemm_skinny_inputs": [P, P, P, I, I, I, I, I, I, I, c_longlong, I, I, P],
@@ -428,12 +429,12 @@ def paged_attention_generic(q: torch.Tensor, q_row_stride: int, k_pool, v_pool, 
           "paged_attention: head sizes %d / %d (the general kernel takes sizes up to %d)"
           % (head_dim, v_head_dim, ATTENTION_MAX_HEAD_DIM))
     out = torch.empty((tokens, num_heads * v_head_dim), dtype=torch.float32 if out_float32 else q.dtype, device=q.device)
-    _check(library().vx_paged_attention_generic_chunk(
+    _check(library().vx_paged_attention_generic_requests(
         _ptr(q), q_row_stride, _ptr(k_pool), _ptr(v_pool), _ptr(block_table), block_table.shape[1],
         _ptr(seq_of_token), _ptr(positions), _ptr(out), num_heads * v_head_dim, float(scale), int(window), tokens,
         num_heads, num_kv_heads, head_dim, page_size, dtype_code(q.dtype), v_head_dim, int(keep_first),
         float(bias_exponent), _ptr(sinks), int(gate_col), float(softcap), int(v_stride), int(v_share),
-        1 if out_float32 else 0, int(chunk), _stream()), "paged_attention_generic")
+        1 if out_float32 else 0, int(chunk), int(block_table.shape[0]), _stream()), "paged_attention_generic")
     return out
 
 
