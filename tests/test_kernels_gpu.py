@@ -398,6 +398,37 @@ def test_gemm_float32_waits_for_a_w_that_was_just_written(M, N, K):
         assert torch.equal(ops().gemm_members(a.view(1, M, K), just_written().view(1, N, K))[0], want)
 
 
+TURNED_SHAPES = [(1, 16, 1, 0, 1), (2, 32, 1, 0, 2), (1, 48, 5, 0, 2), (2, 64, 4, 0, 1), (1, 112, 8, 0, 1), (1, 128, 1, 0, 2), (2, 160, 1, 32, 1),
+                 (2, 256, 3, 0, 1), (1, 240, 1, 16, 1), (2, 208, 1, 64, 1)]     # blocks of a tile, rows of A, runs of k, rows of the last W tiles, blocks an SM
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 256, 64), (16, 2064, 1032), (33, 400, 520), (64, 1040, 1000), (65, 16, 8), (312, 2576, 1088), (777, 528, 256), (800, 19456, 72)])
+def test_gemm_turned(M, N, K):
+    """The turned product with every kind of tile, and with the one that is chosen: rows and columns that no tile divides, k that no block of 64
+    divides, fewer W tiles than the rest with narrow ones; plain and gated, both results.  Rows of NaN behind a and w are not read."""
+    a = torch.full((M + 8, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    w = torch.full((N + 16, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    a[:M], w[:N] = rnd((M, K), torch.bfloat16, 6), rnd((N, K), torch.bfloat16, 7, 0.05)
+    a, w = a[:M], w[:N]
+    want = f64(a) @ f64(w).T
+    g = want.reshape(M, N // 16, 2, 8)
+    gated = (P.silu(g[:, :, 0]) * g[:, :, 1]).reshape(M, N // 2)
+    error, lib, stream = torch.zeros(1, dtype=torch.int32, device=DEV), ops().library(), ops()._stream()
+    for cg, n, runs, narrow, per_sm in TURNED_SHAPES:
+        runs = min(runs, -(-K // 64))
+        full = max(0, -(-N // (128 * cg)) - 2)
+        for is_gated, dtype in ((0, torch.bfloat16), (1, torch.bfloat16), (0, torch.float32), (1, torch.float32)):
+            out = torch.full((M, N // 2 if is_gated else N), float("nan"), dtype=dtype, device=DEV)
+            assert lib.vx_gemm_turned_shape(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, out.shape[1], is_gated, 0, ops().dtype_code(dtype), 1,
+                                            cg, n, runs, full, narrow, per_sm, error.data_ptr(), stream) == 0
+            close(out, gated if is_gated else want, torch.bfloat16, what=str((cg, n, runs, narrow, per_sm)))
+    for dtype in (torch.bfloat16, torch.float32):
+        close(ops().gemm_turned(a, w, dtype), want, torch.bfloat16)
+        close(ops().gemm_turned(a, w, dtype, gated_activation="silu", w_ready=True), gated, torch.bfloat16)
+    assert int(error.item()) == 0
+    ops().check_device_errors()
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,K", [(1, 53, 72), (37, 64, 16), (130, 136, 104), (64, 384, 96), (8, 4096, 4096)])
 def test_gemm_bf16(M, N, K, out_dtype):

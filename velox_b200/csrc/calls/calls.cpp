@@ -27,6 +27,7 @@ struct Entries {
     int (*gemm_skinny)(P, P, P, void*, int, int, int, int, int, int, int, int, int, int, void*);
     int (*gemm_tcgen05_columns)(P, P, P, void*, int, int, int, int, int, int, int, int, int, void*, void*);
     int (*gemm_tcgen05_pair)(P, P, P, void*, int, int, int, int, int, int, int, int, void*, void*);
+    int (*gemm_turned)(P, P, void*, int, int, int, int, int, int, int, int, int, int, void*, void*);
     int (*prefill)(P, int, int, P, P, int, P, int, P, P, P, void*, int, float, int, int, int, int, int, int, int, void*, int, void*, void*);
     int (*decode)(P, int, P, P, P, int, P, P, P, void*, int, void*, int, float, int, int, int, int, int, int, int, int, int, void*);
 } entry;
@@ -223,6 +224,24 @@ PyObject* gemm_tcgen05(PyObject*, PyObject* const* o, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// (a, w, gated, activation, out dtype, w is ready, error word)
+PyObject* gemm_turned(PyObject*, PyObject* const* o, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 7) NOT_HERE;
+    Arg a(o[0]), w(o[1]), error(o[6]);
+    Scalars sc;
+    const int gated = sc.i(o[2]), act = sc.i(o[3]), ready = sc.i(o[5]);
+    if (sc.bad || !a || !w || !THPDtype_Check(o[4]) || !is(error, at::kInt) || !tcgen05_takes(*a, *w)) NOT_HERE;
+    const at::ScalarType kind = ((THPDtype*)o[4])->scalar_type;
+    const int64_t M = a->size(0), N = w->size(0), cols = gated ? N / 2 : N;
+    if (code_of(kind) < 0 || cols % 8) NOT_HERE;
+    at::Tensor out = fresh(M, cols, kind, *a);
+    LAUNCH(rc, entry.gemm_turned(a->data_ptr(), w->data_ptr(), out.data_ptr(), (int)M, (int)N, (int)a->size(1), (int)a->stride(0),
+                                 (int)w->stride(0), (int)cols, gated, act, code_of(kind), ready, error->data_ptr(), s));
+    return result(rc, std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
 PyObject* tcgen05_supported(PyObject*, PyObject* const* o, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 2) NOT_HERE;
@@ -299,6 +318,7 @@ PyObject* bind(PyObject*, PyObject* arg) {
         {"vx_gemm_skinny_act", (void**)&entry.gemm_skinny},
         {"vx_gemm_tcgen05_columns", (void**)&entry.gemm_tcgen05_columns},
         {"vx_gemm_tcgen05_pair", (void**)&entry.gemm_tcgen05_pair},
+        {"vx_gemm_turned", (void**)&entry.gemm_turned},
         {"vx_paged_prefill_attention_tc", (void**)&entry.prefill},
         {"vx_paged_decode_attention_shape", (void**)&entry.decode},
     };
@@ -311,7 +331,7 @@ PyObject* bind(PyObject*, PyObject* arg) {
 
 #define FAST(f) {#f, (PyCFunction)(void (*)(void))f, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"bind", bind, METH_O, nullptr}, FAST(add_rmsnorm), FAST(qk_norm_rope_kv), FAST(gated_act), FAST(gemm_bf16),
-                         FAST(gemm_tcgen05), FAST(tcgen05_supported), FAST(prefill_attention), FAST(decode_attention),
+                         FAST(gemm_tcgen05), FAST(gemm_turned), FAST(tcgen05_supported), FAST(prefill_attention), FAST(decode_attention),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "velox_b200_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -333,7 +333,7 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     float* sums = reinterpret_cast<float*>(tiles);   // [bm][128]: this part's sums, in place of the stages
 #pragma unroll
     for (int j = 0; j < COLS; ++j)
-        if (col0 + j < bm) sums[(col0 + j) * GT_BN + row] = acc[j];
+        if (col0 + j < bm) sums[(col0 + j) * GT_BN + row] = bad ? __int_as_float(0x7fc00000) : acc[j];
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     const int used = min(bm, g.M - m0) * GT_BN;

@@ -138,6 +138,9 @@ def _declare(lib) -> None:
         "vx_gemm_nt_simt_ready": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, I, P],
         "vx_gemm_tcgen05": [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_tcgen05_columns": [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P],
+        "vx_gemm_turned": [P, P, P, I, I, I, I, I, I, I, I, I, I, P, P],
+        "vx_gemm_turned_shape": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, I, I, I, I, I, P, P],
+        "vx_gemm_turned_wins": [I, I, I, I],
         "vx_gemm_tcgen05_pair": [P, P, P, P, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_skinny": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P],
         "vx_paged_prefill_attention_tc": [P, I, I, P, P, I, P, I, P, P, P, P, I, F, I, I, I, I, I, I, I, P, I, P, P],
@@ -1037,7 +1040,7 @@ def _simt(a, w, bias, out, m, n, k, lda, ldw, ldc, batch, sa, sw, sc, w_ready, w
                                              dtype_code(a.dtype), dtype_code(out.dtype), 1 if w_ready else 0,
                                              _ptr(_error_word(a.device)) if exact else None, _stream()), what)
     if exact:
-        note_bounded_wait()
+        note_marked_wait()
 
 
 def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None,
@@ -1635,6 +1638,41 @@ _BOUNDED_WAIT_LAUNCHES = 0   # launches of kernels with bounded waits, ever
 _BOUNDED_WAIT_CHECKED = 0    # ... at the last check of the error word
 
 
+_MARKED_WAIT_LAUNCHES = 0    # launches of kernels that write NaN where a wait runs out, ever
+_MARKED_WAIT_CHECKED = 0     # ... at the last look at the error word
+_LOOKS = {}                  # device: (host copy of its error word, the copy's event)
+
+
+def marked_wait_launches() -> int:
+    return _MARKED_WAIT_LAUNCHES
+
+
+def note_marked_wait(n: int = 1) -> None:
+    """A kernel was launched whose waits are bounded and whose results are NaN if one runs out: they cannot pass for results, so
+    the error word is looked at without waiting for the kernel (see `check_pending_device_errors`)."""
+    global _MARKED_WAIT_LAUNCHES
+    _MARKED_WAIT_LAUNCHES += n
+
+
+def _look_at_error_words() -> None:
+    """What the error words held when they were last copied to the host, if that copy has arrived; and the next copy.  A decode step that waited
+    for its own word instead would keep the next one from being launched behind it (130 us of an idle GPU a step)."""
+    global _MARKED_WAIT_CHECKED
+    _MARKED_WAIT_CHECKED = _MARKED_WAIT_LAUNCHES
+    for key, word in _ERROR_WORDS.items():
+        with torch.cuda.device(word.device):
+            if key in _LOOKS:
+                copy, event = _LOOKS[key]
+                if not event.query():
+                    continue
+                if int(copy[0]):
+                    check_device_errors()
+            else:
+                copy, event = _LOOKS[key] = (torch.zeros(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event())
+            copy.copy_(word, non_blocking=True)
+            event.record()
+
+
 def bounded_wait_launches() -> int:
     return _BOUNDED_WAIT_LAUNCHES
 
@@ -1653,18 +1691,21 @@ def bounded_wait_pending() -> bool:
 
 
 def check_pending_device_errors() -> None:
-    """`check_device_errors()` if a kernel with bounded waits ran since the last check,
-    else nothing (and no synchronisation).  What steps a model calls this before it
+    """`check_device_errors()` if a kernel with bounded waits ran since the last check;
+    without a synchronisation, a look at the word as it was a step or so ago, if only
+    kernels ran that write NaN where a wait runs out; else nothing.  What steps a model calls this before it
     hands out a step's results; it does not have to know which kernels a part chose."""
     if bounded_wait_pending():
         check_device_errors()
+    elif _MARKED_WAIT_LAUNCHES != _MARKED_WAIT_CHECKED:
+        _look_at_error_words()
 
 
 def check_device_errors() -> None:
     """Raises if a kernel has reported that one of its bounded waits ran out since
     the last check (its results are then missing).  Synchronises the device."""
-    global _BOUNDED_WAIT_CHECKED
-    _BOUNDED_WAIT_CHECKED = _BOUNDED_WAIT_LAUNCHES
+    global _BOUNDED_WAIT_CHECKED, _MARKED_WAIT_CHECKED
+    _BOUNDED_WAIT_CHECKED, _MARKED_WAIT_CHECKED = _BOUNDED_WAIT_LAUNCHES, _MARKED_WAIT_LAUNCHES
     for key, word in _ERROR_WORDS.items():
         code = int(word.item())
         if code:
@@ -1762,6 +1803,45 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
     return out
 
 
+_TURNED = {}
+
+
+def turned_wins(m: int, n: int, k: int, gated: bool) -> bool:
+    """Whether the turned product (rows of W on the tensor core's M side) is the fastest for m rows of a model's weights
+    [n, k]; the rule and what was measured: `vx_gemm_turned_wins`."""
+    key = (m, n, k, gated)
+    wins = _TURNED.get(key)
+    if wins is None:
+        if len(_TURNED) >= 4096:
+            _TURNED.clear()
+        wins = _TURNED[key] = library().vx_gemm_turned_wins(m, n, k, 1 if gated else 0) == 1
+    return wins
+
+
+def gemm_turned(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, gated_activation: Optional[str] = None,
+                w_ready: bool = False) -> torch.Tensor:
+    """a [M,K] times w [N,K] transposed on the tcgen05 tensor cores with w's rows on their M side (bfloat16 in, float32 accumulation).  With
+    `gated_activation`, w's rows come in tiles of 8 gate rows followed by their 8 up rows and the result is act(gate) * up, [M, N/2].
+    `w_ready`: see `gemm_nt_simt`."""
+    _dev(a, w)
+    out_dtype = out_dtype or torch.bfloat16
+    _need(gated_activation is None or gated_activation in ACTIVATIONS, "gemm_turned: unknown activation %r" % gated_activation)
+    gated, act = (0, 0) if gated_activation is None else (1, ACTIVATIONS[gated_activation])
+    out = (_CALLS or _calls()).gemm_turned(a, w, gated, act, out_dtype, 1 if w_ready else 0, _error_word(a.device))
+    if out is not None:
+        out = _called(out, "gemm_turned")
+    else:
+        _need(a.dim() == 2 and w.dim() == 2 and a.shape[1] == w.shape[1], "gemm_turned: a [M,K], w [N,K]")
+        _need(tcgen05_supported(a, w), "gemm_turned: bfloat16, K a multiple of 8, N a multiple of 16, 16-byte aligned rows")
+        m, k = a.shape
+        n = w.shape[0]
+        out = torch.empty((m, n // 2 if gated else n), dtype=out_dtype, device=a.device)
+        _check(library().vx_gemm_turned(_ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), w.stride(0), out.shape[1], gated, act,
+                                        dtype_code(out_dtype), 1 if w_ready else 0, _ptr(_error_word(a.device)), _stream()), "gemm_turned")
+    note_marked_wait()
+    return out
+
+
 SKINNY_MAX_ROWS = 8
 _MATMUL_SET = False
 
@@ -1830,8 +1910,12 @@ def _full_precision_sums() -> None:
         _MATMUL_SET = True
 
 
-def gemm_bf16(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """a [M,K] times w [N,K] transposed on the tensor cores, float32 accumulation."""
+def gemm_bf16(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None,
+              w_ready: bool = False) -> torch.Tensor:
+    """a [M,K] times w [N,K] transposed on the tensor cores, float32 accumulation.  `w_ready`: see `gemm_nt_simt`; only then is
+    the turned product taken where it is the fastest (part of what it gains are weights on their way before the wait)."""
+    if w_ready and bias is None and a.is_cuda and turned_wins(a.shape[0], w.shape[0], a.shape[1], False) and tcgen05_supported(a, w):
+        return gemm_turned(a, w, out_dtype, w_ready=True)
     if bias is None and _MATMUL_SET and a.is_cuda:
         few = a.shape[0] <= SKINNY_MAX_ROWS
         out = (_CALLS or _calls()).gemm_bf16(a, w, out_dtype or torch.bfloat16)

@@ -23,7 +23,7 @@ def matmul(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     out_dtype = out_dtype or x.dtype
     if x.dtype == torch.float32:
         return ops.gemm_nt_simt(x, weight, bias, out_dtype, w_ready=True)
-    return ops.gemm_bf16(x, weight, bias, out_dtype)
+    return ops.gemm_bf16(x, weight, bias, out_dtype, w_ready=True)
 
 
 class Linear:
