@@ -1803,6 +1803,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
     return out
 
 
+TURNED_MAX_ROWS = 800   # from which on `turned_wins` never holds
 _TURNED = {}
 
 
@@ -1914,7 +1915,7 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[t
               w_ready: bool = False) -> torch.Tensor:
     """a [M,K] times w [N,K] transposed on the tensor cores, float32 accumulation.  `w_ready`: see `gemm_nt_simt`; only then is
     the turned product taken where it is the fastest (part of what it gains are weights on their way before the wait)."""
-    if w_ready and bias is None and a.is_cuda and turned_wins(a.shape[0], w.shape[0], a.shape[1], False) and tcgen05_supported(a, w):
+    if w_ready and bias is None and SKINNY_MAX_ROWS < a.shape[0] <= TURNED_MAX_ROWS and a.is_cuda and turned_wins(a.shape[0], w.shape[0], a.shape[1], False) and tcgen05_supported(a, w):
         return gemm_turned(a, w, out_dtype, w_ready=True)
     if bias is None and _MATMUL_SET and a.is_cuda:
         few = a.shape[0] <= SKINNY_MAX_ROWS
