@@ -424,7 +424,9 @@ __global__ void __launch_bounds__(ATS_THREADS, 1) paged_attention_shared_kernel(
     __shared__ int count_s[ATS_WARPS], start_s;
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int *seq_of_token = g.seq_of_token, *positions = g.positions;
-    // the block's tokens begin with the blockIdx.x-th that begins a run: at a multiple of eight, or after another request's
+    // (tokens at positions that do not follow each other make more runs than the grid has blocks: then a block takes several)
+    for (int wanted = blockIdx.x;; wanted += gridDim.x) {
+    // the block's tokens begin with the wanted-th that begins a run: at a multiple of eight, or after another request's
     if (threadIdx.x == 0) start_s = -1;
     for (int base = 0, seen = 0; base < g.tokens; base += ATS_THREADS) {
         const int t = base + threadIdx.x;
@@ -440,12 +442,12 @@ __global__ void __launch_bounds__(ATS_THREADS, 1) paged_attention_shared_kernel(
             before += w < warp ? count_s[w] : 0;
             seen += count_s[w];
         }
-        if (begins && before + __popc(votes & ((1u << lane) - 1)) == (int)blockIdx.x) start_s = t;
-        if (seen > (int)blockIdx.x) break;   // (uniform)
+        if (begins && before + __popc(votes & ((1u << lane) - 1)) == wanted) start_s = t;
+        if (seen > wanted) break;   // (uniform)
     }
     __syncthreads();
     const int t0 = start_s;
-    if (t0 < 0) return;
+    if (t0 < 0) return;   // (uniform)
     const int seq = seq_of_token[t0], pos0 = positions[t0], H = g.H, Hk = g.Hk;
     int nt = 1;
     while (nt < ATS_TOKENS && t0 + nt < g.tokens && ((pos0 + nt) & (ATS_TOKENS - 1)) && seq_of_token[t0 + nt] == seq && positions[t0 + nt] == pos0 + nt) ++nt;
@@ -491,6 +493,8 @@ __global__ void __launch_bounds__(ATS_THREADS, 1) paged_attention_shared_kernel(
             g.out[(size_t)t * g.out_row_stride + (size_t)h * g.Dv + d] = o / L * gate;
         }
     }
+    __syncthreads();
+    }
 }
 
 // `v_share` > 1: that many consecutive key heads read one value head (the value pool has Hk / v_share heads);
@@ -520,7 +524,7 @@ extern "C" int vx_paged_attention_generic_requests(const void* q, int q_row_stri
     if (dtype == VX_F32 && four && small && window == 0 && chunk == 0) {
         static bool configured[VX_MAX_DEVICES];
         if (int rc = vx_configure_smem(paged_attention_shared_kernel, ATS_SMEM, configured)) return rc;
-        // (runs of tokens: a request has one for every eight positions, and two that are not whole)
+        // (runs of tokens: a request's neighbouring ones have one for every eight positions, and two that are not whole)
         const int group = H / Hk, runs = requests > 0 && requests < tokens ? (int)min((long long)tokens, tokens / ATS_TOKENS + 2ll * requests) : tokens;
         const AtsCall g = {(const float*)q, (const float*)k_pool, (const float*)v_pool, block_table, seq_of_token, positions, (float*)out, sinks, scale,
                            bias_exp, softcap, q_row_stride, max_blocks, out_row_stride, tokens, H, Hk, D, S, Dv, gate_col, v_stride, v_share};
