@@ -398,6 +398,24 @@ def test_gemm_float32_waits_for_a_w_that_was_just_written(M, N, K):
         assert torch.equal(ops().gemm_members(a.view(1, M, K), just_written().view(1, N, K))[0], want)
 
 
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K,wide", [(1, 512, 128, 192), (8, 130, 512, 512), (5, 7, 32, 40), (3, 16, 96, 96), (8, 512, 192, 200), (2, 64, 256, 257), (7, 24, 384, 384),
+                                        (8, 40, 160, 160), (4, 48, 520, 520)])
+def test_gemm_heads_of_few_rows(M, N, K, wide, out_dtype):
+    """Products per head of up to eight rows: every cut of k that the tensor cores take (whole, two and four parts), sizes and strides that they
+    do not; heads inside wider rows of A and of the result.  float32 results: the error of float32 sums of k terms."""
+    H = 3
+    a, w = rnd((M, H, wide), torch.bfloat16, 1), rnd((H, N, K), torch.bfloat16, 2, 0.05)
+    out = torch.full((M, H, N + 3), 7.0, dtype=out_dtype, device=DEV)
+    ops().gemm_heads(a[:, :, :K], w, out[:, :, :N])
+    want = np.einsum("mhk,hnk->mhn", f64(a[:, :, :K]), f64(w))
+    if out_dtype == torch.float32:
+        assert (abs(f64(out[:, :, :N]) - want) <= 2 * K * 2.0 ** -24 * np.einsum("mhk,hnk->mhn", abs(f64(a[:, :, :K])), abs(f64(w)))).all()
+    else:
+        close(out[:, :, :N], want, torch.bfloat16)
+    assert (out[:, :, N:] == 7.0).all()
+
+
 TURNED_SHAPES = [(1, 16, 1, 0, 1), (2, 32, 1, 0, 2), (1, 48, 5, 0, 2), (2, 64, 4, 0, 1), (1, 112, 8, 0, 1), (1, 128, 1, 0, 2), (2, 160, 1, 32, 1),
                  (2, 256, 3, 0, 1), (1, 240, 1, 16, 1), (2, 208, 1, 64, 1)]     # blocks of a tile, rows of A, runs of k, rows of the last W tiles, blocks an SM
 

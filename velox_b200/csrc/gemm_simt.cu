@@ -7,6 +7,7 @@
 // (here: ascending k), so a row's result does not depend on how many rows the call has.  Any M, N, K.
 #include "common.cuh"
 #include "gemm_f32.cuh"
+#include "mma_helpers.cuh"
 
 #define GS_BM 64
 #define GS_BN 64
@@ -183,6 +184,77 @@ gemm_few_rows_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, TC*
     }
 }
 
+// The same on mma.sync for the sizes of a latent attention's products per head (K up to 512 in pieces of 128, rows of A and W on 16-byte
+// addresses): a warp forms 16 columns of the result (rows of W) from up to 128 k, and everything it reads is on its way
+// before anything is used, W before the wait.  What bounds it is that one trip to memory; the kernel above takes three or four, one after another
+// (16 heads, 8 rows, N 512, K 128: 8.2 us, so 2.1; N 128, K 512: 8.3, 2.3).  Both operands hold k in the order
+// in which a lane's 16 bytes lie (8 of its 32 k after each other), so no rearrangement is needed; the parts of k are added in ascending order.
+#define GH_WARPS 4
+#define GH_CHUNKS 4    // pieces of 32 k of a warp
+template <int KS>
+__global__ void __launch_bounds__(GH_WARPS * 32)
+gemm_few_rows_mma_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, bf16* __restrict__ C, int M, int N, int K, int lda,
+                         int ldw, int ldc, long long sa, long long sw, long long sc) {
+    __shared__ float sums[KS > 1 ? GH_WARPS : 1][KS > 1 ? 16 * 8 : 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int part = warp % KS, n0 = (blockIdx.x * (GH_WARPS / KS) + warp / KS) * 16, k0 = part * (K / KS) + t * 8, chunks = K / KS / 32;
+    W += (size_t)blockIdx.y * sw;
+    uint4 w[GH_CHUNKS][2], x[GH_CHUNKS];
+#pragma unroll
+    for (int j = 0; j < GH_CHUNKS; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int n = n0 + g + 8 * h;
+            w[j][h] = j < chunks && n < N ? *reinterpret_cast<const uint4*>(W + (size_t)n * ldw + k0 + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    pdl_wait();
+    pdl_trigger();
+    A += (size_t)blockIdx.y * sa;
+    C += (size_t)blockIdx.y * sc;
+#pragma unroll
+    for (int j = 0; j < GH_CHUNKS; ++j)
+        x[j] = j < chunks && g < M ? *reinterpret_cast<const uint4*>(A + (size_t)g * lda + k0 + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < GH_CHUNKS; ++j) {
+        const unsigned first[4] = {w[j][0].x, w[j][1].x, w[j][0].y, w[j][1].y}, second[4] = {w[j][0].z, w[j][1].z, w[j][0].w, w[j][1].w};
+        // (each product of 16 k from zero, then added: a chain in the tensor core's accumulator cuts off where an addition rounds)
+        float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16(lo, first, x[j].x, x[j].y);
+        mma_bf16(hi, second, x[j].z, x[j].w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) c[i] = (c[i] + lo[i]) + hi[i];
+    }
+    if (KS > 1) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sums[warp][(g + 8 * (i >> 1)) * 8 + 2 * t + (i & 1)] = c[i];
+        __syncthreads();
+        if (part) return;
+#pragma unroll
+        for (int p = 1; p < KS; ++p)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c[i] += sums[warp + p][(g + 8 * (i >> 1)) * 8 + 2 * t + (i & 1)];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int n = n0 + g + 8 * (i >> 1), m = 2 * t + (i & 1);
+        if (n < N && m < M) C[(size_t)m * ldc + n] = from_f32<bf16>(c[i]);
+    }
+}
+
+static int gh_launch(const bf16* A, const bf16* W, bf16* C, int M, int N, int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
+                     long long sc, cudaStream_t stream) {
+    const int ks = K > 256 ? 4 : (K > 128 ? 2 : 1), rows = GH_WARPS / ks * 16;
+    dim3 grid((N + rows - 1) / rows, batch);
+#define GH_GO(KS_) VX_LAUNCH_K(VX_K_GEMM, (gemm_few_rows_mma_kernel<KS_>), grid, GH_WARPS * 32, 0, stream, A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc)
+    if (ks == 4) GH_GO(4);
+    else if (ks == 2) GH_GO(2);
+    else GH_GO(1);
+#undef GH_GO
+    VX_LAUNCH_CHECK();
+    return VX_OK;
+}
+
 // A, W bfloat16; C bfloat16 or float32 (`out_dtype`).  M <= 8, K a multiple of 8 up to 4,096, W's rows on 16-byte
 // addresses (ldw and sw multiples of 8, the pointer aligned).
 extern "C" int vx_gemm_few_rows_batched(const void* A, const void* W, void* C, int M, int N, int K, int lda, int ldw, int ldc,
@@ -192,6 +264,11 @@ extern "C" int vx_gemm_few_rows_batched(const void* A, const void* W, void* C, i
     if ((ldw & 7) || (sw & 7) || (((uintptr_t)W) & 15)) return VX_ERR_ALIGN;
     dim3 grid((N + GF_WARPS - 1) / GF_WARPS, batch);
     if (batch > 65535) return VX_ERR_LIMIT;
+    // on the tensor cores where K goes into whole pieces (32, 64, 96 or 128 k; twice or four times as many), A can be read 16 bytes at a time
+    // and the result is rounded to bfloat16
+    const int pieces = K > 256 ? 128 : (K > 128 ? 64 : 32);
+    if (out_dtype == VX_BF16 && K <= 512 && K % pieces == 0 && !((lda | sa) & 7) && !(((uintptr_t)A) & 15))
+        return gh_launch((const bf16*)A, (const bf16*)W, (bf16*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
     const size_t smem = (size_t)M * K * sizeof(float);
     static bool configured[2][VX_MAX_DEVICES];
     if (out_dtype == VX_BF16) {
