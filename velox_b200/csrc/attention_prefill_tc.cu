@@ -49,7 +49,6 @@
 #define PT_QTILES 2                  // query tiles a block works on
 #define PT_THREADS 384
 #define PT_MMA_WARP 8                // warps 0-3: softmax of query tile 0, 4-7: of tile 1, 8: tensor core, 9-11: producers
-#define PT_SPIN_LIMIT (1 << 24)
 #define PT_LOG2E 1.4426950408889634f
 #define PT_HALF_BYTES (128 * 128)   // 128 rows x 64 columns of bf16: one swizzled half of a tile
 #define PT_TILE_BYTES (2 * PT_HALF_BYTES)
@@ -65,16 +64,6 @@ __device__ __forceinline__ void pt_mbar_expect_tx(unsigned bar, unsigned bytes) 
 }
 __device__ __forceinline__ void pt_mbar_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool pt_mbar_wait(unsigned bar, unsigned parity) {
-    for (int i = 0; i < PT_SPIN_LIMIT; ++i) {
-        unsigned ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
-    return false;
 }
 __device__ __forceinline__ void pt_tma_load_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
     asm volatile(
@@ -349,7 +338,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
         const int which = warp - (PT_MMA_WARP + 1);           // keys / values
         const int g = (lane & 15) >> 1, half = lane & 1;
         const CUtensorMap* map = which ? &map_v : &map_k;
-        for (int i = 0; i < ntiles && !failed; ++i) {
+        for (int i = 0; i < ntiles; ++i) {
             const int b = i & 1;
             const int key_base = (lo + i) * PT_KEYS;
             // Groups of 16 keys outside [kv_lo, kv_hi) repeat the nearest group inside: they
@@ -359,16 +348,14 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
             const int page = bt[key / S];   // (asked for before the wait below)
             const unsigned full = pt_smem_u32(which ? &bars.v_full[b] : &bars.k_full[b]);
             bool ok = true;
-            if (lane == 0) {
-                if (i >= 2)
-                    ok = pt_mbar_wait(pt_smem_u32(which ? &bars.v_empty[b] : &bars.k_empty[b]),
-                                      (unsigned)(((i >> 1) - 1) & 1));
-                if (!ok) {
+            if (lane == 0) {   // (`failed` is read by one lane, for all of them)
+                ok = !*(volatile int*)&failed;
+                if (ok && i >= 2 && !tc_mbar_wait(pt_smem_u32(which ? &bars.v_empty[b] : &bars.k_empty[b]), (unsigned)(((i >> 1) - 1) & 1))) {
+                    ok = false;
                     failed = 1;
                     atomicExch(error, 11);
-                } else {
-                    pt_mbar_expect_tx(full, PT_TILE_BYTES);
                 }
+                if (ok) pt_mbar_expect_tx(full, PT_TILE_BYTES);
             }
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) break;
@@ -414,11 +401,11 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
             };
             bool ok = true;
             // the first key tile's scores
-            ok = pt_mbar_wait(pt_smem_u32(&bars.k_full[0]), 0);
+            ok = tc_warp_wait(pt_smem_u32(&bars.k_full[0]), 0);
 #pragma unroll
             for (int q = 0; q < PT_QTILES; ++q) {
                 if (tile_b[q] > tile_a[q]) {
-                    ok = ok && pt_mbar_wait(pt_smem_u32(&bars.q_full[q]), 0);   // (once: the queries stay)
+                    ok = ok && tc_warp_wait(pt_smem_u32(&bars.q_full[q]), 0);   // (once: the queries stay)
                     if (ok && tile_a[q] == lo) {
                         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                         issue_s(q, lo);
@@ -433,9 +420,9 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                 for (int q = 0; q < PT_QTILES; ++q) {
                     if (t >= tile_a[q] && t < tile_b[q]) {
                         // O_q += P_q V: the probabilities of this tile, the values
-                        if (!have_v) { ok = ok && pt_mbar_wait(pt_smem_u32(&bars.v_full[b]), (unsigned)((u >> 1) & 1)); have_v = true; }
+                        if (!have_v) { ok = ok && tc_warp_wait(pt_smem_u32(&bars.v_full[b]), (unsigned)((u >> 1) & 1)); have_v = true; }
                         const int n = t - tile_a[q];
-                        ok = ok && pt_mbar_wait(pt_smem_u32(&bars.p_ready[q]), (unsigned)(n & 1));
+                        ok = ok && tc_warp_wait(pt_smem_u32(&bars.p_ready[q]), (unsigned)(n & 1));
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                         const unsigned vd = pt_mnmajor(pt_smem_u32(v_s + b * PT_TILE_BYTES));
@@ -456,7 +443,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                     if (t + 1 >= tile_a[q] && t + 1 < tile_b[q]) {
                         // the next scores of this query tile go where its probabilities were: the tensor core
                         // takes its instructions in order, so P V above has read them before
-                        if (!have_k) { ok = ok && pt_mbar_wait(pt_smem_u32(&bars.k_full[b ^ 1]), (unsigned)(((u + 1) >> 1) & 1)); have_k = true; }
+                        if (!have_k) { ok = ok && tc_warp_wait(pt_smem_u32(&bars.k_full[b ^ 1]), (unsigned)(((u + 1) >> 1) & 1)); have_k = true; }
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                         issue_s(q, t + 1);
@@ -495,8 +482,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
         for (int n = 0; n < my_tiles; ++n) {
             const int t = my_a + n;
             const int key_base = t * PT_KEYS;
-            ok = pt_mbar_wait(pt_smem_u32(&bars.s_full[q]), (unsigned)(n & 1));
-            ok = __all_sync(0xffffffffu, ok);
+            ok = tc_warp_wait(pt_smem_u32(&bars.s_full[q]), (unsigned)(n & 1));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             // the row's 128 scores are read once and stay in registers for both passes
@@ -542,8 +528,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                     }
                     if (n > 0 && __any_sync(0xffffffffu, move)) {
                         // O is rescaled in the rows that moved; P V of the previous tile must be complete
-                        ok = pt_mbar_wait(pt_smem_u32(&bars.pv_done[q]), (unsigned)((n - 1) & 1));
-                        ok = __all_sync(0xffffffffu, ok);
+                        ok = tc_warp_wait(pt_smem_u32(&bars.pv_done[q]), (unsigned)((n - 1) & 1));
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll 1
@@ -613,8 +598,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                 // the tile reaches past the request's last key: the lowest query tile that works on it clears
                 // those value rows (both halves); the tensor core takes the tiles' products in this order
                 const int u = t - lo, b = u & 1;
-                ok = pt_mbar_wait(pt_smem_u32(&bars.v_full[b]), (unsigned)((u >> 1) & 1));
-                ok = __all_sync(0xffffffffu, ok);
+                ok = tc_warp_wait(pt_smem_u32(&bars.v_full[b]), (unsigned)((u >> 1) & 1));
                 if (!ok) break;
                 unsigned char* vt = v_s + b * PT_TILE_BYTES;
                 const int first = max(kv_total - t * PT_KEYS, 0);
@@ -644,8 +628,7 @@ paged_prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
             if (lane == 0) pt_mbar_arrive(pt_smem_u32(&bars.p_ready[q]));
         }
         if (ok && my_tiles > 0) {
-            ok = pt_mbar_wait(pt_smem_u32(&bars.pv_done[q]), (unsigned)((my_tiles - 1) & 1));
-            ok = __all_sync(0xffffffffu, ok);
+            ok = tc_warp_wait(pt_smem_u32(&bars.pv_done[q]), (unsigned)((my_tiles - 1) & 1));
         }
         if (!ok) {
             if (lane == 0) { failed = 1; atomicExch(error, 13); }

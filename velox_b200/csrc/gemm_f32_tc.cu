@@ -231,7 +231,7 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     bool ok = true;
     // adds chunk c's accumulators
     auto drain = [&](int c) {
-        ok = tc_mbar_wait(tc_smem_u32(&done[c & 1]), (unsigned)((c >> 1) & 1)) && ok;
+        ok = ok && tc_warp_wait(tc_smem_u32(&done[c & 1]), (unsigned)((c >> 1) & 1));   // (once one has run out no further one is waited for)
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         if (col0 < bm) {   // (uniform)
 #pragma unroll
@@ -303,7 +303,7 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     }
     drain(chunks - 1);
     if (AHEAD) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    if (!ok) {
+    if (!ok && lane == 0) {
         failed = 1;
         if (g.error) atomicExch(g.error, TC_ERR_EPILOGUE);
     }

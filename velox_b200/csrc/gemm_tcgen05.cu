@@ -54,7 +54,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     extern __shared__ unsigned char tc_smem_raw[];
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_s;
-    __shared__ int failed;
     constexpr unsigned A_BYTES = TC_BM * TC_BK * 2, W_BYTES = BN * TC_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
     // the swizzled tiles must start on 1024-byte boundaries
     unsigned char* tiles = (unsigned char*)(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -78,7 +77,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             tc_mbar_init(tc_smem_u32(&acc_full[i]), 1);
             tc_mbar_init(tc_smem_u32(&acc_empty[i]), 4);   // one arrival per epilogue warp
         }
-        failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {  // tensor memory: two accumulators of BN columns x 128 lanes
@@ -101,8 +99,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const int m0 = row_tiles ? row_tiles[3 * rt + 1] : rt * TC_BM;
             const int n0 = (tile / mtiles) * bn + (row_tiles ? row_tiles[3 * rt] * N : 0);   // (row of W)
             for (int kb = 0; kb < nkb; ++kb) {
-                if (!tc_mbar_wait(tc_smem_u32(&empty_bar[s]), phase)) {
-                    if (lane == 0) { failed = 1; atomicExch(error, TC_ERR_PRODUCER); }
+                if (!tc_warp_wait(tc_smem_u32(&empty_bar[s]), phase)) {
+                    if (lane == 0) atomicExch(error, TC_ERR_PRODUCER);
                     ti = my_tiles;
                     break;
                 }
@@ -125,11 +123,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int ti = 0; ok && ti < my_tiles; ++ti) {
             const int buf = ti & 1;
             // the epilogue must have emptied this buffer (it last held tile ti - 2)
-            ok = ti < 2 || tc_mbar_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1));
+            ok = ti < 2 || tc_warp_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1));
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned tmem_d = tmem_base + (unsigned)(buf * BN);
             for (int kb = 0; ok && kb < nkb; ++kb) {
-                ok = tc_mbar_wait(tc_smem_u32(&full_bar[s]), phase);
+                ok = tc_warp_wait(tc_smem_u32(&full_bar[s]), phase);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const unsigned a_lo = tc_desc_lo(tc_smem_u32(tiles) + s * STAGE_BYTES);
@@ -141,7 +139,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
             if (ok && tc_elect()) tc_commit(tc_smem_u32(&acc_full[buf]));   // the accumulator is complete once all have finished
         }
-        if (!ok && lane == 0) { failed = 1; atomicExch(error, TC_ERR_MMA); }
+        if (!ok && lane == 0) atomicExch(error, TC_ERR_MMA);
     } else {
         // ---- epilogue: warp w reads lanes 32 * (w % 4) .. + 31 of tensor memory ----
         const int quarter = warp & 3;
@@ -154,10 +152,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             // (a grouped tile stores only its own rows: those after them belong to the next group)
             const int row = (row_tiles && quarter * 32 + lane >= row_tiles[3 * rt + 2]) ? M : m0 + quarter * 32 + lane;
             const float rs = EPI != TC_PLAIN && row_scale && row < M ? row_scale[src_of_row[row]] : 1.f;
-            bool ok = tc_mbar_wait(tc_smem_u32(&acc_full[buf]), (unsigned)((ti >> 1) & 1));
-            if (!ok && lane == 0) { failed = 1; atomicExch(error, TC_ERR_EPILOGUE); }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+            if (!tc_warp_wait(tc_smem_u32(&acc_full[buf]), (unsigned)((ti >> 1) & 1))) {
+                if (lane == 0) atomicExch(error, TC_ERR_EPILOGUE);
+                break;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned tmem_acc = tmem_base + (unsigned)(buf * BN) + ((unsigned)(quarter * 32) << 16);
 #pragma unroll 1

@@ -46,7 +46,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     extern __shared__ unsigned char tp_smem_raw[];
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_s;
-    __shared__ int failed;
     constexpr unsigned A_BYTES = TC_BM * TC_BK * 2, W_BYTES = TP_HALF * TC_BK * 2, STAGE_BYTES = A_BYTES + W_BYTES;
     unsigned char* tiles = (unsigned char*)(((uintptr_t)tp_smem_raw + 1023) & ~(uintptr_t)1023);
     pdl_wait();
@@ -68,7 +67,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             tc_mbar_init(tc_smem_u32(&acc_full[i]), 1);
             tc_mbar_init(tc_smem_u32(&acc_empty[i]), 8);   // one arrival per epilogue warp of both blocks
         }
-        failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {  // tensor memory: two accumulators of 256 columns x 128 lanes in each block
@@ -90,8 +88,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             const int m0 = (tile % mtiles) * (2 * TC_BM) + (int)rank * TC_BM;
             const int n0 = (tile / mtiles) * TP_BN + (int)rank * TP_HALF;
             for (int kb = 0; kb < nkb; ++kb) {
-                if (!tc_mbar_wait(tc_smem_u32(&empty_bar[s]), phase)) {
-                    if (lane == 0) { failed = 1; atomicExch(error, TP_ERR_PRODUCER); }
+                if (!tc_warp_wait(tc_smem_u32(&empty_bar[s]), phase)) {
+                    if (lane == 0) atomicExch(error, TP_ERR_PRODUCER);
                     ti = my_tiles;
                     break;
                 }
@@ -115,11 +113,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             bool ok = true;
             for (int ti = 0; ok && ti < my_tiles; ++ti) {
                 const int buf = ti & 1;
-                ok = ti < 2 || tc_mbar_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1));
+                ok = ti < 2 || tc_warp_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)(((ti >> 1) - 1) & 1));
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const unsigned tmem_d = tmem_base + (unsigned)(buf * TP_BN);
                 for (int kb = 0; ok && kb < nkb; ++kb) {
-                    ok = tc_mbar_wait(tc_smem_u32(&full_bar[s]), phase);
+                    ok = tc_warp_wait(tc_smem_u32(&full_bar[s]), phase);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     const unsigned a_lo = tc_desc_lo(tc_smem_u32(tiles) + s * STAGE_BYTES);
@@ -131,7 +129,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 }
                 if (ok && tc_elect()) tp_commit_mask(tc_smem_u32(&acc_full[buf]), 3);
             }
-            if (!ok && lane == 0) { failed = 1; atomicExch(error, TP_ERR_MMA); }
+            if (!ok && lane == 0) atomicExch(error, TP_ERR_MMA);
         }
     } else {
         // ---- epilogue (both blocks): warp w reads lanes 32 * (w % 4) .. + 31 of its block's tensor memory ----
@@ -143,10 +141,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             const int tile = pair + ti * pairs;
             const int m0 = (tile % mtiles) * (2 * TC_BM) + (int)rank * TC_BM, n0 = (tile / mtiles) * TP_BN;
             const int row = m0 + quarter * 32 + lane;
-            bool ok = tc_mbar_wait(tc_smem_u32(&acc_full[buf]), (unsigned)((ti >> 1) & 1));
-            if (!ok && lane == 0) { failed = 1; atomicExch(error, TP_ERR_EPILOGUE); }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
+            if (!tc_warp_wait(tc_smem_u32(&acc_full[buf]), (unsigned)((ti >> 1) & 1))) {
+                if (lane == 0) atomicExch(error, TP_ERR_EPILOGUE);
+                break;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned tmem_acc = tmem_base + (unsigned)(buf * TP_BN) + ((unsigned)(quarter * 32) << 16);
 #pragma unroll 1

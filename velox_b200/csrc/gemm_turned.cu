@@ -157,7 +157,7 @@ gemm_turned_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int ti = 0; ti < my_tiles; ++ti) {
             const Tile t = tile_of(ti);
             for (int kb = ti ? 0 : ahead; kb < nkb; ++kb) {
-                if (!tc_mbar_wait(tc_smem_u32(&empty_bar[s]), phase)) {
+                if (!tc_warp_wait(tc_smem_u32(&empty_bar[s]), phase)) {
                     if (lane == 0) atomicExch(error, GU_ERR_PRODUCER);
                     ti = my_tiles;
                     break;
@@ -178,10 +178,10 @@ gemm_turned_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 const int buf = ti & 1, use = ti >> 1;
                 const unsigned d = tmem + (unsigned)(buf * sh.n);
                 // the epilogue must have emptied this accumulator
-                ok = !use || tc_mbar_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)((use - 1) & 1));
+                ok = !use || tc_warp_wait(tc_smem_u32(&acc_empty[buf]), (unsigned)((use - 1) & 1));
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 for (int kb = 0; ok && kb < nkb; ++kb) {
-                    ok = tc_mbar_wait(tc_smem_u32(&full_bar[s]), phase);
+                    ok = tc_warp_wait(tc_smem_u32(&full_bar[s]), phase);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                     const unsigned wd = tc_desc_lo(tc_smem_u32(tiles) + (unsigned)s * stage_bytes);
@@ -207,9 +207,8 @@ gemm_turned_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             const Tile t = tile_of(ti);
             const int buf = ti & 1, use = ti >> 1;
             if (ok) {
-                ok = tc_mbar_wait(tc_smem_u32(&acc_full[buf]), (unsigned)(use & 1));
+                ok = tc_warp_wait(tc_smem_u32(&acc_full[buf]), (unsigned)(use & 1));
                 if (!ok && lane == 0) atomicExch(error, GU_ERR_EPILOGUE);
-                ok = __all_sync(0xffffffffu, ok);
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned acc = tmem + (unsigned)(buf * sh.n) + ((unsigned)(quarter * 32) << 16);

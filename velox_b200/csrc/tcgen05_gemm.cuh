@@ -21,14 +21,25 @@ __device__ __forceinline__ void tc_mbar_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void tc_mbar_expect_tx(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ bool tc_mbar_try(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// A bounded wait of one thread.
 __device__ __forceinline__ bool tc_mbar_wait(unsigned bar, unsigned parity) {
-    for (int i = 0; i < TC_SPIN_LIMIT; ++i) {
-        unsigned ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
+    for (int i = 0; i < TC_SPIN_LIMIT; ++i)
+        if (tc_mbar_try(bar, parity)) return true;
+    return false;
+}
+// A bounded wait of a whole warp, with one answer for all its lanes.  A role that goes on as a warp (tc_elect, tcgen05.ld) waits this
+// way: if lanes counted by themselves, a phase that ends as the limit does could let some of them through and send others away, and an
+// elect.sync that names lanes which have left is undefined.
+__device__ __forceinline__ bool tc_warp_wait(unsigned bar, unsigned parity) {
+    for (int i = 0; i < TC_SPIN_LIMIT; ++i)
+        if (__all_sync(0xffffffffu, tc_mbar_try(bar, parity))) return true;
     return false;
 }
 __device__ __forceinline__ void tc_tma_load_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
