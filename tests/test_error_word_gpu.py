@@ -1,0 +1,94 @@
+"""A wait that ran out is raised before the results it concerns are handed out.  Nothing fails here: the error word is set
+from the host, as a kernel that gives up would set it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from velox_b200.csrc import ops as o
+    return o
+
+
+@pytest.fixture(autouse=True)
+def clean():
+    ops().check_device_errors()
+    yield
+    word = ops()._error_word(torch.device(DEV))
+    torch.cuda.synchronize()
+    word.zero_()
+    ops().check_device_errors()
+
+
+def set_word():
+    ops()._error_word(torch.device(DEV)).fill_(8)
+
+
+def products():
+    a, w = torch.randn(24, 512, device=DEV), torch.randn(256, 512, device=DEV)
+    ab, wb = a.bfloat16(), w.bfloat16()
+    return {"turned": lambda: ops().gemm_turned(ab, wb),
+            "turned gated": lambda: ops().gemm_turned(ab, wb, gated_activation="silu"),
+            "float32": lambda: ops().gemm_nt_simt(a, w),
+            "float32 heads": lambda: ops().gemm_heads(a.view(24, 1, 512), w.view(1, 256, 512), torch.empty(24, 1, 256, device=DEV)),
+            "float32 members": lambda: ops().gemm_members(a.view(1, 24, 512), w.view(1, 256, 512)),
+            "tcgen05": lambda: ops().gemm_tcgen05(ab, wb)}
+
+
+@pytest.mark.parametrize("name", ["turned", "turned gated", "float32", "float32 heads", "float32 members", "tcgen05"])
+def test_products_with_bounded_waits_are_checked(name):
+    o = ops()
+    call = products()[name]
+    call()
+    assert o.bounded_wait_pending()
+    o.check_pending_device_errors()
+    assert not o.bounded_wait_pending()
+    call()
+    set_word()
+    with pytest.raises(o.KernelError, match="gave up a wait"):
+        o.check_pending_device_errors()
+    o.check_pending_device_errors()   # (reported once)
+
+
+def engine(dtype):
+    from velox_b200 import Engine, EngineConfig
+    from velox_b200.config import Qwen3Config
+    raw = dict(vocab_size=512, hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, head_dim=128,
+               attention_bias=False, num_key_value_heads=2, max_position_embeddings=256, tie_word_embeddings=False, rope_theta=10000.0,
+               rms_norm_eps=1e-6, hidden_act="silu", architectures=["Qwen3ForCausalLM"], model_type="qwen3")
+    return Engine(model_config=Qwen3Config.from_dict(raw), random_seed=1,
+                  config=EngineConfig(dtype=dtype, page_size=16, num_pages=64, max_running_requests=16, max_model_len=64))
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_a_decode_step_hands_out_no_token_of_a_failed_wait(dtype):
+    """Twelve requests decode; then the word is set while a step's results are under way: that very step raises, the last one of a
+    request (after which nothing would look again) as well."""
+    from velox_b200 import SamplingParams
+    e = engine(dtype)
+    for i in range(12):
+        e.add_request([1 + i, 7, 9], SamplingParams(max_tokens=4))
+    for _ in range(3):
+        e.step()
+    e.on_logits = lambda ids, logits: set_word()
+    with pytest.raises(ops().KernelError, match="gave up a wait"):
+        e.step()
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_run_step_hands_out_no_logits_of_a_failed_wait(dtype):
+    from velox_b200.engine import StepEntry
+    e = engine(dtype)
+    for i in range(12):
+        e.cache.add_request(i)
+    entries = [StepEntry(i, [3 + i], [0]) for i in range(12)]
+    for _ in range(2):
+        e.run_step(entries)
+    logits = e.runner.step(entries)
+    assert e.runner.pending_error_check and logits is not None
+    set_word()
+    with pytest.raises(ops().KernelError, match="gave up a wait"):
+        e.runner.check_errors()
+    assert not e.runner.pending_error_check

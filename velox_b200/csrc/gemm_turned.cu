@@ -219,7 +219,7 @@ gemm_turned_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 unsigned r[16];
                 if (ok) {
                     gu_ld16(acc + (unsigned)c0, r);
-                } else {   // (a wait ran out: NaN, which nothing takes for a result)
+                } else {   // (a wait ran out, and the error word says so: NaN rather than what the memory held)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) r[j] = 0x7fc00000u;
                 }

@@ -1040,7 +1040,7 @@ def _simt(a, w, bias, out, m, n, k, lda, ldw, ldc, batch, sa, sw, sc, w_ready, w
                                              dtype_code(a.dtype), dtype_code(out.dtype), 1 if w_ready else 0,
                                              _ptr(_error_word(a.device)) if exact else None, _stream()), what)
     if exact:
-        note_marked_wait()
+        note_bounded_wait()
 
 
 def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None,
@@ -1638,41 +1638,6 @@ _BOUNDED_WAIT_LAUNCHES = 0   # launches of kernels with bounded waits, ever
 _BOUNDED_WAIT_CHECKED = 0    # ... at the last check of the error word
 
 
-_MARKED_WAIT_LAUNCHES = 0    # launches of kernels that write NaN where a wait runs out, ever
-_MARKED_WAIT_CHECKED = 0     # ... at the last look at the error word
-_LOOKS = {}                  # device: (host copy of its error word, the copy's event)
-
-
-def marked_wait_launches() -> int:
-    return _MARKED_WAIT_LAUNCHES
-
-
-def note_marked_wait(n: int = 1) -> None:
-    """A kernel was launched whose waits are bounded and whose results are NaN if one runs out: they cannot pass for results, so
-    the error word is looked at without waiting for the kernel (see `check_pending_device_errors`)."""
-    global _MARKED_WAIT_LAUNCHES
-    _MARKED_WAIT_LAUNCHES += n
-
-
-def _look_at_error_words() -> None:
-    """What the error words held when they were last copied to the host, if that copy has arrived; and the next copy.  A decode step that waited
-    for its own word instead would keep the next one from being launched behind it (130 us of an idle GPU a step)."""
-    global _MARKED_WAIT_CHECKED
-    _MARKED_WAIT_CHECKED = _MARKED_WAIT_LAUNCHES
-    for key, word in _ERROR_WORDS.items():
-        with torch.cuda.device(word.device):
-            if key in _LOOKS:
-                copy, event = _LOOKS[key]
-                if not event.query():
-                    continue
-                if int(copy[0]):
-                    check_device_errors()
-            else:
-                copy, event = _LOOKS[key] = (torch.zeros(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event())
-            copy.copy_(word, non_blocking=True)
-            event.record()
-
-
 def bounded_wait_launches() -> int:
     return _BOUNDED_WAIT_LAUNCHES
 
@@ -1691,21 +1656,20 @@ def bounded_wait_pending() -> bool:
 
 
 def check_pending_device_errors() -> None:
-    """`check_device_errors()` if a kernel with bounded waits ran since the last check;
-    without a synchronisation, a look at the word as it was a step or so ago, if only
-    kernels ran that write NaN where a wait runs out; else nothing.  What steps a model calls this before it
-    hands out a step's results; it does not have to know which kernels a part chose."""
+    """`check_device_errors()` if a kernel with bounded waits ran since the last check,
+    else nothing (and no synchronisation).  What steps a model calls this before it
+    hands out a step's results; it does not have to know which kernels a part chose.
+    (Some kernels write NaN where a wait runs out.  That replaces no check: a maximum drops NaN, and the sampler
+    hands out a token id for a row of it.)"""
     if bounded_wait_pending():
         check_device_errors()
-    elif _MARKED_WAIT_LAUNCHES != _MARKED_WAIT_CHECKED:
-        _look_at_error_words()
 
 
 def check_device_errors() -> None:
     """Raises if a kernel has reported that one of its bounded waits ran out since
     the last check (its results are then missing).  Synchronises the device."""
-    global _BOUNDED_WAIT_CHECKED, _MARKED_WAIT_CHECKED
-    _BOUNDED_WAIT_CHECKED, _MARKED_WAIT_CHECKED = _BOUNDED_WAIT_LAUNCHES, _MARKED_WAIT_LAUNCHES
+    global _BOUNDED_WAIT_CHECKED
+    _BOUNDED_WAIT_CHECKED = _BOUNDED_WAIT_LAUNCHES
     for key, word in _ERROR_WORDS.items():
         code = int(word.item())
         if code:
@@ -1839,7 +1803,7 @@ def gemm_turned(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtyp
         out = torch.empty((m, n // 2 if gated else n), dtype=out_dtype, device=a.device)
         _check(library().vx_gemm_turned(_ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), w.stride(0), out.shape[1], gated, act,
                                         dtype_code(out_dtype), 1 if w_ready else 0, _ptr(_error_word(a.device)), _stream()), "gemm_turned")
-    note_marked_wait()
+    note_bounded_wait()
     return out
 
 

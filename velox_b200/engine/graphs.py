@@ -109,7 +109,6 @@ class _Graph:
         self.logits = self.ids = None
         self.launches = 0
         self.bounded_wait_launches = 0  # of those, kernels whose waits are bounded
-        self.marked_wait_launches = 0   # ... and that write NaN where one runs out
         self.copied: Optional[torch.cuda.Event] = None  # the last copy out of the pinned buffer
 
     def fill(self, entries: Sequence[StepEntry], rids, cache, sampling, vocab_size: int = -1) -> None:
@@ -168,7 +167,7 @@ class _MixedGraph:
                                max_short=max_short, **dict(zip(SECTION_NAMES, v[:F])))
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.logits = self.ids = None
-        self.launches = self.bounded_wait_launches = self.marked_wait_launches = 0
+        self.launches = self.bounded_wait_launches = 0
         self.copied: Optional[torch.cuda.Event] = None
 
     def fill(self, entries, cache, vocab_size, short_max) -> List[int]:
@@ -246,7 +245,8 @@ class DecodeGraphs:
             return g.logits, g.ids
         g.graph.replay()
         ops.add_launches(g.launches)
-        self._note(g)
+        if g.bounded_wait_launches:
+            ops.note_bounded_wait(g.bounded_wait_launches)
         return g.logits, g.ids
 
     # -- small mixed steps ---------------------------------------------------------
@@ -288,15 +288,9 @@ class DecodeGraphs:
         else:
             g.graph.replay()
             ops.add_launches(g.launches)
-            self._note(g)
+            if g.bounded_wait_launches:
+                ops.note_bounded_wait(g.bounded_wait_launches)
         return g.logits if sig[2] else None
-
-    @staticmethod
-    def _note(g) -> None:
-        if g.bounded_wait_launches:
-            ops.note_bounded_wait(g.bounded_wait_launches)
-        if g.marked_wait_launches:
-            ops.note_marked_wait(g.marked_wait_launches)
 
     def _capture(self, g) -> None:
         # once eagerly (first-use set-up of kernels and libraries happens outside the capture) ...
@@ -315,7 +309,7 @@ class DecodeGraphs:
         # recording only: what was garbage before the engine's time is gone then, and
         # engines themselves are freed by their reference counts, without the collector.
         graph = torch.cuda.CUDAGraph()
-        n0, b0, m0 = ops.launch_count(), ops.bounded_wait_launches(), ops.marked_wait_launches()
+        n0, b0 = ops.launch_count(), ops.bounded_wait_launches()
         if not self._collected:
             gc.collect()
             self._collected = True
@@ -330,7 +324,6 @@ class DecodeGraphs:
         g.launches = ops.launch_count() - n0
         ops.add_launches(-g.launches)  # (recorded, not run)
         g.bounded_wait_launches = ops.bounded_wait_launches() - b0
-        g.marked_wait_launches = ops.marked_wait_launches() - m0
         if self.pool is None:
             self.pool = graph.pool()
         g.graph = graph
