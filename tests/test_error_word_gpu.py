@@ -24,6 +24,7 @@ def clean():
 
 def set_word():
     ops()._error_word(torch.device(DEV)).fill_(8)
+    torch.cuda.synchronize()   # (a kernel's own report is there when the kernel has ended)
 
 
 def products():
@@ -52,10 +53,10 @@ def test_products_with_bounded_waits_are_checked(name):
     o.check_pending_device_errors()   # (reported once)
 
 
-def engine(dtype):
+def engine(dtype, vocab=512):
     from velox_b200 import Engine, EngineConfig
     from velox_b200.config import Qwen3Config
-    raw = dict(vocab_size=512, hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, head_dim=128,
+    raw = dict(vocab_size=vocab, hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, head_dim=128,
                attention_bias=False, num_key_value_heads=2, max_position_embeddings=256, tie_word_embeddings=False, rope_theta=10000.0,
                rms_norm_eps=1e-6, hidden_act="silu", architectures=["Qwen3ForCausalLM"], model_type="qwen3")
     return Engine(model_config=Qwen3Config.from_dict(raw), random_seed=1,
@@ -92,3 +93,53 @@ def test_run_step_hands_out_no_logits_of_a_failed_wait(dtype):
     with pytest.raises(ops().KernelError, match="gave up a wait"):
         e.runner.check_errors()
     assert not e.runner.pending_error_check
+
+
+def test_the_end_of_waits_of_a_graph_is_that_of_its_latest_replay():
+    """The host waits for the event that a replay records behind its last kernel with bounded waits: what comes before it has then run,
+    in that very replay, though the stream is still busy with what comes after."""
+    o = ops()
+    x, big = torch.zeros(1, dtype=torch.int32, device=DEV), torch.randn(4096, 4096, device=DEV).bfloat16()
+    end = o.EndOfWaits(captured=True)
+
+    def work():
+        for _ in range(20):
+            torch.mm(big, big)
+        x.add_(1)
+        end.record()
+        for _ in range(20):
+            torch.mm(big, big)
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        work()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        work()
+    x.zero_()
+    torch.cuda.synchronize()
+    busy = 0
+    for i in range(1, 21):
+        graph.replay()
+        end.event.synchronize()
+        busy += not torch.cuda.current_stream().query()
+        with torch.cuda.stream(side):
+            assert int(x.item()) == i
+    assert busy > 0
+
+
+def test_a_captured_step_is_checked_at_its_end_of_waits():
+    """Decode steps from a graph: the end noted last is the graph's own, and covers all that it launched."""
+    from velox_b200.engine import StepEntry
+    o, e = ops(), engine("bfloat16", vocab=32784)   # (the head is the library's: no waits)
+    for i in range(12):
+        e.cache.add_request(i)
+    for k in range(3):
+        e.runner.step([StepEntry(i, [3 + i], [0]) for i in range(12)])
+        if k:
+            assert o._END_OF_WAITS[0] == o.bounded_wait_launches()
+            g = next(iter(e.runner.graphs.graphs.values()))
+            assert o._END_OF_WAITS[1] is g.end_of_waits.event
+        e.runner.check_errors()
+        assert not e.runner.pending_error_check

@@ -1655,23 +1655,65 @@ def bounded_wait_pending() -> bool:
     return _BOUNDED_WAIT_LAUNCHES != _BOUNDED_WAIT_CHECKED
 
 
+class EndOfWaits:
+    """A place in a stream with no kernel with bounded waits behind it: once it is reached the error word is final.  A step's head and
+    its sampling lie behind its last such kernel, and while they run the host can prepare the next step (waiting for them as well
+    left the GPU idle for 80 to 130 us a step).  `captured`: recorded inside a graph, and by each of its replays."""
+
+    def __init__(self, captured: bool = False):
+        self.event = torch.cuda.Event(external=captured)
+        self.launches = -1   # with bounded waits, ever, where it was recorded
+
+    def record(self) -> None:
+        self.event.record()
+        self.launches = _BOUNDED_WAIT_LAUNCHES
+
+
+_END_OF_WAITS = (-1, None)   # the latest end: (launches with bounded waits before it, its event)
+_READERS = {}                # device: the stream on which the error word is read without waiting for what runs
+
+
+def note_end_of_waits(end: EndOfWaits) -> None:
+    """All kernels with bounded waits launched so far come before `end`."""
+    global _END_OF_WAITS
+    _END_OF_WAITS = (_BOUNDED_WAIT_LAUNCHES, end.event)
+
+
 def check_pending_device_errors() -> None:
     """`check_device_errors()` if a kernel with bounded waits ran since the last check,
     else nothing (and no synchronisation).  What steps a model calls this before it
     hands out a step's results; it does not have to know which kernels a part chose.
+    If an end of waits was noted after the last of them, the host waits for that only.
     (Some kernels write NaN where a wait runs out.  That replaces no check: a maximum drops NaN, and the sampler
     hands out a token id for a row of it.)"""
     if bounded_wait_pending():
-        check_device_errors()
+        launches, event = _END_OF_WAITS
+        if launches == _BOUNDED_WAIT_LAUNCHES:
+            event.synchronize()
+            _read_error_words(True)
+        else:
+            check_device_errors()
 
 
 def check_device_errors() -> None:
     """Raises if a kernel has reported that one of its bounded waits ran out since
     the last check (its results are then missing).  Synchronises the device."""
+    _read_error_words(False)
+
+
+def _read_error_words(reached: bool) -> None:
+    """`reached`: the kernels in question have ended; the words are read beside what runs now, else behind it."""
     global _BOUNDED_WAIT_CHECKED
     _BOUNDED_WAIT_CHECKED = _BOUNDED_WAIT_LAUNCHES
     for key, word in _ERROR_WORDS.items():
-        code = int(word.item())
+        if reached:
+            reader = _READERS.get(key)
+            if reader is None:
+                reader = _READERS[key] = torch.cuda.Stream(word.device)
+            with torch.cuda.stream(reader):
+                code = int(word.item())
+        else:
+            code = int(word.item())
         if code:
             word.zero_()
             raise KernelError("a kernel on %s gave up a wait on its asynchronous copies or tensor-core work "

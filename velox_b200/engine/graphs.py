@@ -109,6 +109,7 @@ class _Graph:
         self.logits = self.ids = None
         self.launches = 0
         self.bounded_wait_launches = 0  # of those, kernels whose waits are bounded
+        self.end_of_waits = ops.EndOfWaits(captured=True)   # behind the last of them
         self.copied: Optional[torch.cuda.Event] = None  # the last copy out of the pinned buffer
 
     def fill(self, entries: Sequence[StepEntry], rids, cache, sampling, vocab_size: int = -1) -> None:
@@ -132,8 +133,7 @@ class _Graph:
         self.copied.record()
 
     def run_model(self, runner) -> None:
-        residual, delta = runner.model.forward_hidden(self.ctx, runner.cache)
-        self.logits = runner.model.logits(residual, delta, self.ctx.wanted_rows)
+        self.logits = runner.run(self.ctx, self.end_of_waits)
         self.ids = ops.sample(self.logits, self.d_temp, self.d_top_p, self.d_uniform)
 
 
@@ -168,6 +168,7 @@ class _MixedGraph:
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.logits = self.ids = None
         self.launches = self.bounded_wait_launches = 0
+        self.end_of_waits = ops.EndOfWaits(captured=True)
         self.copied: Optional[torch.cuda.Event] = None
 
     def fill(self, entries, cache, vocab_size, short_max) -> List[int]:
@@ -181,7 +182,7 @@ class _MixedGraph:
         return summary
 
     def run_model(self, runner) -> None:
-        self.logits = runner.run(self.ctx)
+        self.logits = runner.run(self.ctx, self.end_of_waits)
         if self.logits is None:   # (nothing wanted: the capture still needs a tensor to hand around)
             self.logits = torch.empty((0, runner.vocab_size), dtype=torch.float32, device=runner.device)
         self.ids = self.logits   # (no sampling inside; `_capture` copies both)
@@ -245,8 +246,7 @@ class DecodeGraphs:
             return g.logits, g.ids
         g.graph.replay()
         ops.add_launches(g.launches)
-        if g.bounded_wait_launches:
-            ops.note_bounded_wait(g.bounded_wait_launches)
+        self._note_waits(g)
         return g.logits, g.ids
 
     # -- small mixed steps ---------------------------------------------------------
@@ -288,9 +288,16 @@ class DecodeGraphs:
         else:
             g.graph.replay()
             ops.add_launches(g.launches)
-            if g.bounded_wait_launches:
-                ops.note_bounded_wait(g.bounded_wait_launches)
+            self._note_waits(g)
         return g.logits if sig[2] else None
+
+    @staticmethod
+    def _note_waits(g) -> None:
+        """What a replay of `g` launched."""
+        if g.bounded_wait_launches:
+            ops.note_bounded_wait(g.bounded_wait_launches)
+            if g.end_is_last:
+                ops.note_end_of_waits(g.end_of_waits)
 
     def _capture(self, g) -> None:
         # once eagerly (first-use set-up of kernels and libraries happens outside the capture) ...
@@ -324,6 +331,7 @@ class DecodeGraphs:
         g.launches = ops.launch_count() - n0
         ops.add_launches(-g.launches)  # (recorded, not run)
         g.bounded_wait_launches = ops.bounded_wait_launches() - b0
+        g.end_is_last = g.end_of_waits.launches == ops.bounded_wait_launches()
         if self.pool is None:
             self.pool = graph.pool()
         g.graph = graph

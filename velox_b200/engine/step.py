@@ -30,6 +30,7 @@ class ModelRunner:
         # requests that bring at most so many tokens are listed token by token for the mixers (a mixer
         # may then treat each token as a decoded one): the largest wish among the model's parts
         self.short_max = max([1] + [int(getattr(p, "short_rows_up_to", 1)) for p in model.parts()])
+        self.end_of_waits = ops.EndOfWaits()
         self.graphs = None
         if cuda_graphs:
             from .graphs import DecodeGraphs
@@ -131,8 +132,14 @@ class ModelRunner:
     def check_errors(self) -> None:
         ops.check_pending_device_errors()
 
-    def run(self, ctx: StepContext) -> Optional[torch.Tensor]:
+    def run(self, ctx: StepContext, end_of_waits=None) -> Optional[torch.Tensor]:
+        """`end_of_waits`: a captured step's own (`ops.EndOfWaits`)."""
         residual, delta = self.model.forward_hidden(ctx, self.cache)
+        if end_of_waits is not None:
+            end_of_waits.record()
+        elif ops.bounded_wait_pending():
+            self.end_of_waits.record()
+            ops.note_end_of_waits(self.end_of_waits)
         if ctx.wanted_rows.numel() == 0:
             return None
         return self.model.logits(residual, delta, ctx.wanted_rows)
