@@ -376,6 +376,33 @@ def test_gemm_float32_infinities_nan_and_tiny_sums():
     assert (abs(got[finite] - want[finite]) <= (K * 2.0 ** -24 * size + K * 2.0 ** -149)[finite]).all()
 
 
+@pytest.mark.parametrize("K", [512, 1024, 1100, 3072])
+@pytest.mark.parametrize("M", [1, 37, 130])
+def test_gemm_float32_tiny_operands_against_large_ones(M, K):
+    """Operands below what bfloat16 parts hold against ones so large that their sums are ordinary numbers (or would be: all parts of the
+    smallest are 0), beside ordinary rows: every sum within K roundings of 2^-24 of the sum of the products' magnitudes.  A row of zeros gives
+    zeros; the ordinary rows have the bits that they have without the others."""
+    a, w = rnd((M, K), torch.float32, 1), rnd((200, K), torch.float32, 2)
+    plain = ops().gemm_nt_simt(a, w)
+    w2 = w.clone()
+    for n, size in enumerate([1e20, 1e25, 1e30, 1e12, 2.0 ** 29, 1e-20]):
+        w2[3 + 20 * n] = (0.5 + rnd((K,), torch.float32, 5 + n).abs()) * size
+    w2[7] = 0
+    x = a.clone()
+    small = [3e-38, 1e-40, 1e-42, 1e-36, 1e-33, 1e-25]
+    for i, size in enumerate(small[:M]):
+        x[i * (M // len(small))] = (0.5 + rnd((K,), torch.float32, 20 + i).abs()) * size
+    got = ops().gemm_nt_simt(x, w2)
+    X, W = f64(x), f64(w2)
+    want, size = X @ W.T, abs(X) @ abs(W).T
+    assert (size < 3e38).all()
+    assert (abs(f64(got) - want) <= K * 2.0 ** -24 * size + K * 2.0 ** -149).all()
+    assert (got[:, 7] == 0).all()
+    rows = [m for m in range(M) if torch.equal(x[m], a[m])]
+    cols = [n for n in range(200) if torch.equal(w2[n], w[n])]
+    assert torch.equal(got[rows][:, cols], plain[rows][:, cols])
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (12, 1000, 777), (99, 4096, 1024), (3, 40000, 300)])
 def test_gemm_float32_waits_for_a_w_that_was_just_written(M, N, K):
     """W written by the kernel launched just before, in memory that holds NaN until then: the products (plain, per head, of a batch)

@@ -1,7 +1,7 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) in float32 on the fifth-generation tensor cores: the matrix product of the 32-bit path.
 //
-// A 32-bit number is the sum of three bfloat16 ones, exactly: its value rounded to 8 bits, what is left rounded to 8 bits, and
-// the rest (24 bits in all; Dekker's splitting, with three parts).  Of the nine products of two such numbers the six that
+// A 32-bit number of 2^-109 or more is the sum of three bfloat16 ones, exactly: its value rounded to 8 bits, what is left rounded
+// to 8 bits, and the rest (24 bits in all; Dekker's splitting, with three parts).  Of the nine products of two such numbers the six that
 // matter are formed by tcgen05.mma (hi hi, hi mid, mid hi, mid mid, hi lo, lo hi; the others are 2^-24 of the result and
 // below), each exact before it is added, the small ones first.  The tensor core cuts off what does not fit into an accumulator where
 // a multiply-add rounds, so an accumulator takes 32 k only and is then added, rounded, to a sum in a register.  Error against 64
@@ -22,8 +22,13 @@
 // splitting's stores, the copies), above that the splitting and the products about alike.  (With 256 threads two warps a scheduler waited on each
 // other: 40 % of the issue slots used, 1.4 to 2.9 us a chunk.)  Measurements: at vx_gemm_f32_tc below.
 //
-// Where the sum is no ordinary number (an infinity or NaN among the operands, a sum that overflows, parts below what bfloat16
-// holds: a sum under 2^-80), it is formed again by multiply-adds in ascending k, so that infinities and NaN come out as they do there.
+// What three parts cannot hold is formed again by multiply-adds in ascending k: sums that are no ordinary numbers (an infinity or
+// NaN among the operands, a sum that overflows), so that infinities and NaN come out as they do there; and those to which what
+// bfloat16 loses below 2^-126 may matter.  An operand loses less than 2^-125, so a sum of K products loses less than
+// K 2^-94 while all operands are below 2^30: nothing, to a sum of 2^-50 or more (K up to 2^20).  Hence: sums below 2^-50 (0 included, unless
+// a row is all zeros) and sums with an operand of 2^30 or more.  Both follow from the sum's own two rows.  (Rows are only searched where the
+// squares of what a thread has split add up to 2^60.  A maximum instead, on the pipe that the splitting's conversions fill: 99 x 4096 x 1024
+// 17.5 us, 14.3 without.)
 #include <cooperative_groups.h>
 
 #include "gemm_f32.cuh"
@@ -109,9 +114,28 @@ struct GtCall {
     int* error;
 };
 
-// The sum by multiply-adds one after another, for the sums that the tensor cores cannot form.
-__device__ __noinline__ float gt_plain(const float* a, const float* b, int K) {
-    float v = 0.f;
+// The squares of four numbers, added to a thread's two sums (on the pipe that the splitting uses least).
+__device__ __forceinline__ void gt_squares(float2& sum, const float4& v) {
+    sum = __ffma2_rn(make_float2(v.x, v.y), make_float2(v.x, v.y), sum);
+    sum = __ffma2_rn(make_float2(v.z, v.w), make_float2(v.z, v.w), sum);
+}
+__device__ __forceinline__ bool gt_any(const float* a, int K, float least) {   // (whether a magnitude is `least` or more)
+    for (int k = 0; k < K; ++k)
+        if (fabsf(a[k]) >= least) return true;
+    return false;
+}
+// The tensor cores' sum `v` of two rows if they could form it, else the sum by multiply-adds one after another.  `huge`: an operand
+// of GT_HUGE or more may be somewhere in the tile.
+#define GT_HUGE 1.073741824e9f   // 2^30
+#define GT_TINY 8.8817842e-16f   // 2^-50
+__device__ __noinline__ float gt_careful(const float* a, const float* b, int K, float v, bool huge) {
+    const float size = fabsf(v);
+    bool again = !(size < INFINITY);
+    if (!again && size < GT_TINY) again = size > 0.f || (gt_any(a, K, 1.4e-45f) && gt_any(b, K, 1.4e-45f));
+    if (!again && huge) again = gt_any(a, K, GT_HUGE) || gt_any(b, K, GT_HUGE);
+    if (!again) return v;
+    v = 0.f;
+#pragma unroll 8
     for (int k = 0; k < K; ++k) v = fmaf(a[k], b[k], v);
     return v;
 }
@@ -134,7 +158,7 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     extern __shared__ unsigned char gt_raw[];
     __shared__ __align__(8) unsigned long long done[2];
     __shared__ unsigned tmem_s;
-    __shared__ int failed;
+    __shared__ int failed, huge_s;
     unsigned char* tiles = (unsigned char*)(((uintptr_t)gt_raw + 1023) & ~(uintptr_t)1023);
     const float* A = g.A + (size_t)blockIdx.z * g.sa;
     const float* W = g.W + (size_t)blockIdx.z * g.sw;
@@ -219,6 +243,7 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     const unsigned tmem = tmem_s;
 
     float acc[COLS], total[SPLIT ? 1 : COLS];
+    float2 squares = make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
     if (!SPLIT) {
@@ -271,10 +296,15 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
             for (int i = 0; i < XSTEPS; ++i) x[i] = *reinterpret_cast<const float4*>(slot + (WSTEPS + i) * STEP);
         }
 #pragma unroll
-        for (int i = 0; i < WSTEPS; ++i) gt_store(st + place + i * GT_STEP * 128, GT_W_BYTES, w[i]);
+        for (int i = 0; i < WSTEPS; ++i) {
+            gt_squares(squares, w[i]);
+            gt_store(st + place + i * GT_STEP * 128, GT_W_BYTES, w[i]);
+        }
 #pragma unroll
-        for (int i = 0; i < XSTEPS; ++i)
+        for (int i = 0; i < XSTEPS; ++i) {
+            gt_squares(squares, x[i]);
             if (GT_STEP * i + fr < bm) gt_store(sx + place + i * GT_STEP * 128, BM * 128, x[i]);
+        }
         if (c + (AHEAD ? AHEAD : 1) < chunks) {
             fetch_w(c + (AHEAD ? AHEAD : 1));
             fetch_x(c + (AHEAD ? AHEAD : 1));
@@ -308,7 +338,7 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
         if (g.error) atomicExch(g.error, TC_ERR_EPILOGUE);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();   // (everyone has read the tensor memory, and the tensor core the stages)
+    bool huge = __syncthreads_or(!(squares.x < GT_HUGE * GT_HUGE && squares.y < GT_HUGE * GT_HUGE));   // (everyone has read the tensor memory, and the tensor core the stages)
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((unsigned)TMEM) : "memory");
@@ -318,7 +348,7 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     auto finish = [&](float v, int m, int n) {
         const float size = fabsf(v);
         if (bad) v = __int_as_float(0x7fc00000);
-        else if (!(size < INFINITY) || (size < 8.3e-25f && size > 0.f)) v = gt_plain(A + (size_t)m * g.lda, W + (size_t)n * g.ldw, g.K);
+        else if (huge || !(size < INFINITY && size >= GT_TINY)) v = gt_careful(A + (size_t)m * g.lda, W + (size_t)n * g.ldw, g.K, v, huge);
         C[(size_t)m * g.ldc + n] = v + (g.bias ? g.bias[n] : 0.f);
     };
     const int row = (warp & 3) * 32 + lane;
@@ -334,8 +364,10 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
 #pragma unroll
     for (int j = 0; j < COLS; ++j)
         if (col0 + j < bm) sums[(col0 + j) * GT_BN + row] = bad ? __int_as_float(0x7fc00000) : acc[j];
+    if (threadIdx.x == 0) huge_s = huge;
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
+    for (int p = 0; p < parts; ++p) huge = huge || *cluster.map_shared_rank(&huge_s, p);
     const int used = min(bm, g.M - m0) * GT_BN;
     for (int e = rank * GT_THREADS + threadIdx.x; e < used; e += parts * GT_THREADS) {
         const int n = n0 + e % GT_BN;
