@@ -43,13 +43,17 @@ __device__ __forceinline__ float4 att_load4(const bf16* p) {
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// FOUR: the sizes of keys and values, the stride of a value row and the pools' addresses are multiples of four elements.  What
-// bounds this kernel is the latency of its loads: eight lanes fetch a key, four keys at a time, and a value row comes as four neighbouring
-// channels a lane, both in batches that are all asked for before the first is used (a lane a key, which touched 32 rows with every load: one token
-// on 400 keys, 16 heads of 128, float32, 42 us, 25 so).  SMALL: heads up to 128, with more keys and values ahead.
+// PARTS > 0: the sizes of keys and values, the stride of a value row and the pools' addresses are multiples of four elements.  What
+// bounds this kernel is the latency of its loads and how many blocks are there to hide it: eight lanes fetch a key, four keys at a time
+// (PARTS times 32 elements), and a value row comes as four neighbouring channels a lane.  Heads up to 128: one such batch of keys and
+// four values ahead, in 64 registers, eight blocks an SM; larger heads two and four, four blocks.  (Four batches and sixteen values in 124 registers
+// were slower wherever blocks are many.  us, a lane a key, which touches 32 rows with every load, that, and so: one float32 token on 400
+// keys, 16 heads of 128, 42, 25, 22; 64 of them 125, 110, 52; 1,000 tokens in a window of 1,024 2490, 1334, 1158; bfloat16, 1,000 tokens,
+// heads of 80 640, 905, 572, of 256 1258, 976, 557; 64 decoded on 600 keys, heads of 192, 136, 196, 83.  Slower than a lane a key: bfloat16 heads of 36,
+// 1,000 tokens, 485, 510.)  PARTS 0: any sizes, a lane a key.
 // Which form runs follows from the layer's sizes, so a position's sums have one order.
-template <typename T, bool FOUR, bool SMALL>
-__global__ void __launch_bounds__(ATT_WARPS * 32, SMALL ? 4 : (FOUR ? 2 : 9)) paged_attention_generic_kernel(
+template <typename T, int PARTS>
+__global__ void __launch_bounds__(ATT_WARPS * 32, PARTS == 0 ? 9 : (PARTS <= 4 ? 8 : 4)) paged_attention_generic_kernel(
     const T* __restrict__ q, int q_row_stride, const T* __restrict__ k_pool,
     const T* __restrict__ v_pool, const int* __restrict__ block_table, int max_blocks,
     const int* __restrict__ seq_of_token, const int* __restrict__ positions, T* __restrict__ out,
@@ -58,6 +62,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, SMALL ? 4 : (FOUR ? 2 : 9)) pa
     int chunk) {
     pdl_wait();
     pdl_trigger();
+    constexpr bool FOUR = PARTS > 0, SMALL = FOUR && PARTS <= 4;   // (SMALL: values up to 128 as well)
     __shared__ __align__(FOUR ? 16 : 4) float q_s[ATT_MAX_D];   // (aligned for the other form, its loop over d is half as fast)
     __shared__ float acc_s[ATT_WARPS][ATT_MAX_D];
     __shared__ float m_s[ATT_WARPS], l_s[ATT_WARPS];
@@ -105,11 +110,11 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, SMALL ? 4 : (FOUR ? 2 : 9)) pa
         }
         const int nvalid = min(32, nkeys - c * 32);
         if (FOUR) {
-            // eight lanes a key, four keys at a time (key 4 i + lane / 8 of the chunk), four such loads in flight
-            constexpr int AHEAD = SMALL ? 4 : 2, PARTS = SMALL ? 4 : 8;
+            // eight lanes a key, four keys at a time: key 4 i + lane / 8 of the chunk
+            constexpr int AHEAD = SMALL ? 1 : 2;
 #pragma unroll 1
             for (int i0 = 0; i0 < 8; i0 += AHEAD) {
-                float4 b[AHEAD][PARTS];
+                float4 b[AHEAD][FOUR ? PARTS : 1];
 #pragma unroll
                 for (int u = 0; u < AHEAD; ++u) {
                     const int jj = 4 * (i0 + u) + (lane >> 3);
@@ -151,22 +156,22 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, SMALL ? 4 : (FOUR ? 2 : 9)) pa
 #pragma unroll
         for (int i = 0; i < NR; ++i) acc[i] *= alpha;
         if (FOUR) {
-            constexpr int AHEAD = SMALL ? 16 : 8, PARTS = SMALL ? 1 : 2;
+            constexpr int AHEAD = 4, VPARTS = SMALL ? 1 : 2;
 #pragma unroll 1
             for (int j0 = 0; j0 < nvalid; j0 += AHEAD) {
-                float4 v[AHEAD][PARTS];
+                float4 v[AHEAD][VPARTS];
 #pragma unroll
                 for (int u = 0; u < AHEAD; ++u) {
                     const T* vp = v_pool + (size_t)__shfl_sync(0xffffffffu, (unsigned long long)base, j0 + u) * v_stride + lane * 4;
 #pragma unroll
-                    for (int r = 0; r < PARTS; ++r)
+                    for (int r = 0; r < VPARTS; ++r)
                         v[u][r] = j0 + u < nvalid && lane * 4 + 128 * r < Dv ? att_load4(vp + 128 * r) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
                 for (int u = 0; u < AHEAD; ++u) {
                     const float pj = __shfl_sync(0xffffffffu, p, j0 + u);   // (0 beyond the last key)
 #pragma unroll
-                    for (int r = 0; r < PARTS; ++r) {
+                    for (int r = 0; r < VPARTS; ++r) {
                         acc[4 * r] = fmaf(pj, v[u][r].x, acc[4 * r]);
                         acc[4 * r + 1] = fmaf(pj, v[u][r].y, acc[4 * r + 1]);
                         acc[4 * r + 2] = fmaf(pj, v[u][r].z, acc[4 * r + 2]);
@@ -532,19 +537,22 @@ extern "C" int vx_paged_attention_generic_requests(const void* q, int q_row_stri
         VX_LAUNCH_CHECK();
         return VX_OK;
     }
-#define ATT_GO(T, F, S_)                                                                                                                 \
-    VX_LAUNCH_K(VX_K_ATTENTION, (paged_attention_generic_kernel<T, F, S_>), grid, ATT_WARPS * 32, 0, stream, (const T*)q, q_row_stride,  \
+    const int parts = !four ? 0 : (!small ? 8 : (D <= 64 ? 2 : (D + 31) / 32));
+#define ATT_GO(T, P_)                                                                                                                    \
+    VX_LAUNCH_K(VX_K_ATTENTION, (paged_attention_generic_kernel<T, P_>), grid, ATT_WARPS * 32, 0, stream, (const T*)q, q_row_stride,     \
                 (const T*)k_pool, (const T*)v_pool, block_table, max_blocks, seq_of_token, positions, (T*)out, out_row_stride, scale, \
                 window, H, Hk, D, S, Dv, keep_first, bias_exp, sinks, gate_col, softcap, v_stride, v_share, out_f32, chunk)
-    if (dtype == VX_F32) {
-        if (four && small) ATT_GO(float, true, true);
-        else if (four) ATT_GO(float, true, false);
-        else ATT_GO(float, false, false);
-    } else {
-        if (four && small) ATT_GO(bf16, true, true);
-        else if (four) ATT_GO(bf16, true, false);
-        else ATT_GO(bf16, false, false);
-    }
+#define ATT_OF(T)                          \
+    do {                                   \
+        if (parts == 0) ATT_GO(T, 0);      \
+        else if (parts == 2) ATT_GO(T, 2); \
+        else if (parts == 3) ATT_GO(T, 3); \
+        else if (parts == 4) ATT_GO(T, 4); \
+        else ATT_GO(T, 8);                 \
+    } while (0)
+    if (dtype == VX_F32) ATT_OF(float);
+    else ATT_OF(bf16);
+#undef ATT_OF
 #undef ATT_GO
     VX_LAUNCH_CHECK();
     return VX_OK;
