@@ -291,6 +291,31 @@ def test_float32_attention_whatever_tokens_a_block_has(H, Hk, D, Dv):
             assert torch.equal(run(q[t:t + 1], seq[t:t + 1], pos[t:t + 1], 0, **kw)[0], whole[t]), t
 
 
+@pytest.mark.parametrize("H,Hk,D,Dv", [(16, 16, 128, 128), (16, 8, 64, 128), (8, 2, 96, 36), (12, 12, 36, 20)])
+def test_float32_attention_of_many_decoded_tokens(H, Hk, D, Dv):
+    """So many requests with a token each that their blocks would take turns: the form without sharing, with the bits that the shared one gives a few
+    of them, with a soft cap, a bias by distance, sinks and a gate as well."""
+    S, lens = 16, [1 + 37 * i % 611 for i in range(90)]
+    need = [-(-n // S) for n in lens]
+    bt = torch.zeros((len(lens), max(need)), dtype=torch.int32)
+    order, at = torch.randperm(sum(need), generator=torch.Generator().manual_seed(0)).to(torch.int32), 0
+    for i, n in enumerate(need):
+        bt[i, :n], at = order[at:at + n], at + n
+    bt = bt.to(DEV)
+    k, v = rnd((sum(need), Hk, S, D), torch.float32, 1), rnd((sum(need), Hk, S, Dv), torch.float32, 2)
+    q = rnd((len(lens), H * D + H), torch.float32, 3)
+    seq, pos = torch.arange(len(lens), dtype=torch.int32, device=DEV), torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+
+    def run(lo, hi, **kw):   # (the block table of the tokens' own requests: a call knows how many there are)
+        return ops().paged_attention_generic(q[lo:hi], q.shape[1], k, v, bt[lo:hi], seq[lo:hi] - lo, pos[lo:hi], D ** -0.5, 0, H, Hk, D, hi - lo,
+                                             v_head_dim=Dv, **kw)
+
+    for kw in (dict(), dict(softcap=20.0, bias_exponent=8.0, sinks=rnd((H,), torch.float32, 4), gate_col=H * D)):
+        whole = run(0, len(lens), **kw)
+        for lo in range(0, len(lens), 6):
+            assert torch.equal(run(lo, lo + 6, **kw), whole[lo:lo + 6]), lo
+
+
 # ----------------------------------------------------------------------------
 @pytest.mark.parametrize("M,N,K", [(1, 53, 71), (37, 64, 16), (130, 129, 100), (5, 384, 96)])
 def test_gemm_simt_fp32(M, N, K):

@@ -526,14 +526,20 @@ extern "C" int vx_paged_attention_generic_requests(const void* q, int q_row_stri
     if (dtype != VX_F32 && dtype != VX_BF16) return VX_ERR_DTYPE;
     const bool four = !((D | Dv | v_stride) & 3) && !((((uintptr_t)k_pool) | ((uintptr_t)v_pool)) & (dtype == VX_F32 ? 15 : 7));
     const bool small = D <= 128 && Dv <= 128;
-    if (dtype == VX_F32 && four && small && window == 0 && chunk == 0) {
+    // Tokens that share their keys and values: not where most requests bring a token of their own and the blocks, which fill an SM each, would take
+    // turns (the form below has the same bits.  Decoded tokens, us, shared and not: 64 on 100 keys, 16 heads on 8, 33, 14; on 1,500 277, 160;
+    // 16 heads on 16, 32 on 100 34, 9; on 400 95, 49; 8 heads on 2, 64 on 1,500 125, 130.  In one turn: 8 on 400 keys 24, 22; on 1,500 70, 117).
+    static int sms_cache[VX_MAX_DEVICES];
+    const int groups = Hk * ((H / Hk + ATS_HEADS - 1) / ATS_HEADS);
+    const bool shared = requests <= 0 || tokens >= 4ll * requests || (long long)tokens * groups <= vx_sm_count(sms_cache);
+    if (dtype == VX_F32 && four && small && window == 0 && chunk == 0 && shared) {
         static bool configured[VX_MAX_DEVICES];
         if (int rc = vx_configure_smem(paged_attention_shared_kernel, ATS_SMEM, configured)) return rc;
         // (runs of tokens: a request's neighbouring ones have one for every eight positions, and two that are not whole)
-        const int group = H / Hk, runs = requests > 0 && requests < tokens ? (int)min((long long)tokens, tokens / ATS_TOKENS + 2ll * requests) : tokens;
+        const int runs = requests > 0 && requests < tokens ? (int)min((long long)tokens, tokens / ATS_TOKENS + 2ll * requests) : tokens;
         const AtsCall g = {(const float*)q, (const float*)k_pool, (const float*)v_pool, block_table, seq_of_token, positions, (float*)out, sinks, scale,
                            bias_exp, softcap, q_row_stride, max_blocks, out_row_stride, tokens, H, Hk, D, S, Dv, gate_col, v_stride, v_share};
-        VX_LAUNCH_K(VX_K_ATTENTION, paged_attention_shared_kernel, dim3(runs, Hk * ((group + ATS_HEADS - 1) / ATS_HEADS)), ATS_THREADS, ATS_SMEM, stream, g);
+        VX_LAUNCH_K(VX_K_ATTENTION, paged_attention_shared_kernel, dim3(runs, groups), ATS_THREADS, ATS_SMEM, stream, g);
         VX_LAUNCH_CHECK();
         return VX_OK;
     }
