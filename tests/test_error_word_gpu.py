@@ -28,13 +28,13 @@ def set_word():
 
 
 def products():
-    a, w = torch.randn(24, 512, device=DEV), torch.randn(256, 512, device=DEV)
+    a, w = torch.randn(24, 1024, device=DEV), torch.randn(256, 1024, device=DEV)
     ab, wb = a.bfloat16(), w.bfloat16()
     return {"turned": lambda: ops().gemm_turned(ab, wb),
             "turned gated": lambda: ops().gemm_turned(ab, wb, gated_activation="silu"),
             "float32": lambda: ops().gemm_nt_simt(a, w),
-            "float32 heads": lambda: ops().gemm_heads(a.view(24, 1, 512), w.view(1, 256, 512), torch.empty(24, 1, 256, device=DEV)),
-            "float32 members": lambda: ops().gemm_members(a.view(1, 24, 512), w.view(1, 256, 512)),
+            "float32 heads": lambda: ops().gemm_heads(a.view(24, 1, 1024), w.view(1, 256, 1024), torch.empty(24, 1, 256, device=DEV)),
+            "float32 members": lambda: ops().gemm_members(a.view(1, 24, 1024), w.view(1, 256, 1024)),
             "tcgen05": lambda: ops().gemm_tcgen05(ab, wb)}
 
 
@@ -56,7 +56,7 @@ def test_products_with_bounded_waits_are_checked(name):
 def engine(dtype, vocab=512):
     from velox_b200 import Engine, EngineConfig
     from velox_b200.config import Qwen3Config
-    raw = dict(vocab_size=vocab, hidden_size=512, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, head_dim=128,
+    raw = dict(vocab_size=vocab, hidden_size=1024, intermediate_size=1024, num_hidden_layers=2, num_attention_heads=4, head_dim=128,
                attention_bias=False, num_key_value_heads=2, max_position_embeddings=256, tie_word_embeddings=False, rope_theta=10000.0,
                rms_norm_eps=1e-6, hidden_act="silu", architectures=["Qwen3ForCausalLM"], model_type="qwen3")
     return Engine(model_config=Qwen3Config.from_dict(raw), random_seed=1,

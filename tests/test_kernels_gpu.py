@@ -366,11 +366,13 @@ def test_gemm_float32_error_follows_the_parts(K):
     assert err <= 0.6 * 2.0 ** -24 * math.sqrt(length / 4 + 1 + (parts + 1) / 2), err
 
 
-@pytest.mark.parametrize("N,K,pad", [(1, 257, 0), (127, 320, 4), (129, 1025, 3), (1024, 2049, 3), (32768, 264, 0), (256, 4096, 0)])
+@pytest.mark.parametrize("N,K,pad", [(1, 1024, 0), (127, 1056, 4), (129, 1025, 3), (1024, 2049, 3), (32768, 1032, 0), (256, 4096, 0),
+                                     (6144, 1024, 0), (6144, 2560, 0), (4000, 1792, 0)])
 def test_gemm_float32_by_three_parts(N, K, pad):
-    """The 32-bit product on the tensor cores (k above 256) at the edges of its tiles (16, 32, 64, 128 rows, 128 columns), runs (32 k),
-    chunks (64) and parts.  A term passes at most ten additions in its accumulator, each cut off below 2^-23 of the sum of the terms' sizes, the
+    """The 32-bit product on the tensor cores at the edges of its tiles (16, 32, 64, 128 rows, 128 columns), runs (32 k),
+    chunks (64) and parts, which are dealt one, two or four to a block of a cluster or not at all (7 by twos leave one).  A term passes at most ten additions in its accumulator, each cut off below 2^-23 of the sum of the terms' sizes, the
     run's among those of its part and the part's, rounded to 2^-24; the products left out are below 3 x 2^-24."""
+    assert ops()._f32_takes_tc(N, K)
     parts = min(8, max(1, K // 256))
     steps = 2 * 10 + -(-K // (32 * parts)) + 2 + parts + 3
     w = rnd((N, K + pad), torch.float32, 7)[:, :K]
@@ -381,9 +383,10 @@ def test_gemm_float32_by_three_parts(N, K, pad):
         assert torch.equal(ops().gemm_nt_simt(a[257 - M:], w), whole[257 - M:]), M
 
 
-def test_gemm_float32_infinities_nan_and_tiny_sums():
-    """Infinities, NaN, sums that overflow and operands so small that their parts vanish in bfloat16: what multiply-adds give."""
-    K = 512
+@pytest.mark.parametrize("K", [512, 1024, 2560])
+def test_gemm_float32_infinities_nan_and_tiny_sums(K):
+    """Infinities, NaN, sums that overflow and operands so small that their parts vanish in bfloat16: what multiply-adds give (at 512
+    they form the product)."""
     a, w = rnd((5, K), torch.float32, 1), rnd((70, K), torch.float32, 2)
     a[1, 7], w[3, 9], w[4, 10], w[6], w[8] = math.inf, -math.inf, math.nan, 0.0, 1.0
     a[2] = 3e38
@@ -399,6 +402,21 @@ def test_gemm_float32_infinities_nan_and_tiny_sums():
     infinite, finite = np.isinf(want), np.isfinite(want)
     assert infinite.any() and np.array_equal(got[infinite], want[infinite])
     assert (abs(got[finite] - want[finite]) <= (K * 2.0 ** -24 * size + K * 2.0 ** -149)[finite]).all()
+
+
+def test_gemm_float32_takes_the_tensor_cores_where_few_rows_are_no_slower():
+    """The choice by N and K, on both sides of what was measured; only products that take them are noted as ones with bounded waits."""
+    o = ops()
+    for n, k in [(4096, 1024), (6144, 1024), (1024, 2048), (1024, 3072), (4096, 4096), (4096, 12288), (16384, 1024), (512, 1024)]:
+        assert o._f32_takes_tc(n, k), (n, k)
+    for n, k in [(512, 512), (3072, 512), (8192, 768), (1024, 1023), (2048, 2048), (19456, 2560), (32769, 1024), (151936, 1024)]:
+        assert not o._f32_takes_tc(n, k), (n, k)
+    o.check_device_errors()
+    o.gemm_nt_simt(rnd((3, 512), torch.float32, 1), rnd((64, 512), torch.float32, 2))
+    assert not o.bounded_wait_pending()
+    o.gemm_nt_simt(rnd((3, 1024), torch.float32, 1), rnd((64, 1024), torch.float32, 2))
+    assert o.bounded_wait_pending()
+    o.check_device_errors()
 
 
 @pytest.mark.parametrize("K", [512, 1024, 1100, 3072])
@@ -428,7 +446,7 @@ def test_gemm_float32_tiny_operands_against_large_ones(M, K):
     assert torch.equal(got[rows][:, cols], plain[rows][:, cols])
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (12, 1000, 777), (99, 4096, 1024), (3, 40000, 300)])
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (12, 1000, 777), (12, 1000, 1100), (40, 6144, 1024), (99, 4096, 1024), (3, 40000, 300)])
 def test_gemm_float32_waits_for_a_w_that_was_just_written(M, N, K):
     """W written by the kernel launched just before, in memory that holds NaN until then: the products (plain, per head, of a batch)
     see it whole, as they do when the GPU was waited for in between; with `w_ready` and a W that is, the same bits."""

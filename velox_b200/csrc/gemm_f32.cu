@@ -1,5 +1,5 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) in float32 on the CUDA cores: the matrix product of the 32-bit path
-// where the tensor cores (gemm_f32_tc.cu) are slower: a short k, a vocabulary's head.
+// where the tensor cores (gemm_f32_tc.cu) are slower for a few rows: a short k, a vocabulary's head, some sizes between.
 //
 // Order of a sum: k is cut into at most eight parts of equal length, by K alone (gf_parts); within a part the even and the
 // odd k are summed apart, each in ascending order (two lanes of one packed multiply-add), then added; the parts' sums are

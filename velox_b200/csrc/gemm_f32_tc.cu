@@ -16,11 +16,11 @@
 // fetch 64 k of both as float32 (16 bytes a load, ahead of their use), split them and store the three parts into shared memory in the
 // layout that the tensor core reads (128-byte swizzle); one elected lane issues the products; while they run all threads add the
 // accumulators of the chunk before and split the next one.  Two stages, two sets of accumulators.  Few tiles: the parts of k go
-// to the blocks of a cluster, which add them through distributed shared memory.
+// to the blocks of a cluster, one, two or four to a block, which add them through distributed shared memory.
 //
 // What bounds it: up to some 64 rows the traffic in shared memory (1.2 us a chunk: six reads of W's tile by the tensor core, the
 // splitting's stores, the copies), above that the splitting and the products about alike.  (With 256 threads two warps a scheduler waited on each
-// other: 40 % of the issue slots used, 1.4 to 2.9 us a chunk.)  Measurements: at vx_gemm_f32_tc below.
+// other: 40 % of the issue slots used, 1.4 to 2.9 us a chunk.)  Measurements: at vx_gemm_f32_takes_tc below.
 //
 // What three parts cannot hold is formed again by multiply-adds in ascending k: sums that are no ordinary numbers (an infinity or
 // NaN among the operands, a sum that overflows), so that infinities and NaN come out as they do there; and those to which what
@@ -147,10 +147,12 @@ __host__ __device__ constexpr int gt_smem(int bm) {
     return gt_stages_bytes(bm) + gt_ahead(bm) * (GT_BN / GT_STEP + gt_xsteps(bm)) * GT_THREADS * 16;
 }
 
-// BM: rows of A a tile has room for; `bm` of them (a multiple of 16) are used.
-template <int BM, bool VEC, bool SPLIT>
+// BM: rows of A a tile has room for; `bm` of them (a multiple of 16) are used.  PER: parts of k that a block of the cluster sums up,
+// each by itself (0: no cluster, the block adds all parts).
+template <int BM, bool VEC, int PER>
 __global__ void __launch_bounds__(GT_THREADS, 1)
 gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
+    constexpr bool SPLIT = PER > 0;
     constexpr int STAGE = 3 * GT_W_BYTES + 3 * BM * 128, AHEAD = gt_ahead(BM);
     constexpr int COLS = BM / 4, LDN = COLS < 16 ? COLS : 16;      // columns of a warp, of a load from tensor memory
     constexpr int RUNS = GT_BK / GT_RUN, TMEM = 2 * RUNS * BM;
@@ -164,9 +166,10 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     const float* W = g.W + (size_t)blockIdx.z * g.sw;
     float* C = g.C + (size_t)blockIdx.z * g.sc;
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int rank = SPLIT ? (int)blockIdx.x % parts : 0;
-    const int n0 = (SPLIT ? (int)blockIdx.x / parts : (int)blockIdx.x) * GT_BN, m0 = blockIdx.y * bm;
-    const int kbeg = SPLIT ? rank * part_len : 0, kend = SPLIT ? min(g.K, kbeg + part_len) : g.K;
+    const int blocks = SPLIT ? (parts + PER - 1) / (SPLIT ? PER : 1) : 1;   // of the cluster
+    const int rank = SPLIT ? (int)blockIdx.x % blocks : 0;
+    const int n0 = (SPLIT ? (int)blockIdx.x / blocks : (int)blockIdx.x) * GT_BN, m0 = blockIdx.y * bm;
+    const int kbeg = SPLIT ? rank * PER * part_len : 0, kend = SPLIT ? min(g.K, kbeg + PER * part_len) : g.K;
     const int chunks = (kend - kbeg + GT_BK - 1) / GT_BK;
     // a warp's 32 lanes fetch 64 k of two rows at a time: row GT_STEP i + fr, columns 4 c4
     const int fr = warp * 2 + (lane >> 4), c4 = lane & 15;
@@ -242,17 +245,18 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
     pdl_trigger();
     const unsigned tmem = tmem_s;
 
-    float acc[COLS], total[SPLIT ? 1 : COLS];
+    constexpr int KEPT = SPLIT ? PER - 1 : 1;   // the sum of the parts so far; in a cluster each part before the block's last
+    float acc[COLS], total[KEPT ? KEPT : 1][KEPT ? COLS : 1];
     float2 squares = make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
-    if (!SPLIT) {
 #pragma unroll
-        for (int j = 0; j < COLS; ++j) total[SPLIT ? 0 : j] = 0.f;
-    }
+    for (int p = 0; p < KEPT; ++p)
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) total[p][j] = 0.f;
     const int col0 = (warp >> 2) * COLS;   // this warp's columns (rows of A), its lanes (rows of W) are 32 (warp % 4) ..
     const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bm >> 3) << 17) | ((unsigned)(GT_BN >> 4) << 24);
-    int ended = SPLIT ? chunks : part_len / GT_BK, left = ended;   // chunks until the part ends
+    int left = part_len / GT_BK, kept = 0;   // chunks until the part ends; parts that have
     bool ok = true;
     // adds chunk c's accumulators
     auto drain = [&](int c) {
@@ -272,13 +276,17 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
                 }
             }
         }
-        if (!SPLIT && (--left == 0 || c + 1 == chunks)) {
-            left = ended;
+        if (KEPT && (--left == 0 || c + 1 == chunks) && !(SPLIT && c + 1 == chunks)) {   // (a cluster's block keeps its last part in acc)
+            left = part_len / GT_BK;
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) {
-                total[SPLIT ? 0 : j] += acc[j];
-                acc[j] = 0.f;
-            }
+            for (int p = 0; p < KEPT; ++p)
+                if (!SPLIT || p == kept) {
+#pragma unroll
+                    for (int j = 0; j < COLS; ++j) total[p][j] += acc[j];
+                }
+            ++kept;
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
         }
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     };
@@ -356,24 +364,28 @@ gemm_f32_tc_kernel(GtCall g, int bm, int parts, int part_len) {
         if (n0 + row < g.N) {
 #pragma unroll
             for (int j = 0; j < COLS; ++j)
-                if (col0 + j < bm && m0 + col0 + j < g.M) finish(total[SPLIT ? 0 : j], m0 + col0 + j, n0 + row);
+                if (col0 + j < bm && m0 + col0 + j < g.M) finish(total[0][KEPT ? j : 0], m0 + col0 + j, n0 + row);
         }
         return;
     }
-    float* sums = reinterpret_cast<float*>(tiles);   // [bm][128]: this part's sums, in place of the stages
+    float* sums = reinterpret_cast<float*>(tiles);   // [part][bm][128]: this block's parts' sums, in place of the stages
 #pragma unroll
-    for (int j = 0; j < COLS; ++j)
-        if (col0 + j < bm) sums[(col0 + j) * GT_BN + row] = bad ? __int_as_float(0x7fc00000) : acc[j];
+    for (int p = 0; p < (SPLIT ? PER : 1); ++p)
+        if (p <= kept) {
+#pragma unroll
+            for (int j = 0; j < COLS; ++j)
+                if (col0 + j < bm) sums[(p * bm + col0 + j) * GT_BN + row] = bad ? __int_as_float(0x7fc00000) : (p == kept || !KEPT ? acc[j] : total[p < KEPT ? p : 0][KEPT ? j : 0]);
+        }
     if (threadIdx.x == 0) huge_s = huge;
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
-    for (int p = 0; p < parts; ++p) huge = huge || *cluster.map_shared_rank(&huge_s, p);
+    for (int p = 0; p < blocks; ++p) huge = huge || *cluster.map_shared_rank(&huge_s, p);
     const int used = min(bm, g.M - m0) * GT_BN;
-    for (int e = rank * GT_THREADS + threadIdx.x; e < used; e += parts * GT_THREADS) {
+    for (int e = rank * GT_THREADS + threadIdx.x; e < used; e += blocks * GT_THREADS) {
         const int n = n0 + e % GT_BN;
         if (n >= g.N) continue;
         float v = 0.f;
-        for (int p = 0; p < parts; ++p) v += cluster.map_shared_rank(sums, p)[e];
+        for (int p = 0; p < parts; ++p) v += cluster.map_shared_rank(sums, p / (SPLIT ? PER : 1))[p % (SPLIT ? PER : 1) * bm * GT_BN + e];
         finish(v, m0 + e / GT_BN, n);
     }
     cluster.sync();   // (a block's sums are read until here)
@@ -387,17 +399,18 @@ static void gt_parts(int K, int* parts, int* len) {
     *parts = (K + *len - 1) / *len;
 }
 
-template <int BM, bool VEC, bool SPLIT>
-static cudaLaunchConfig_t gt_config(const GtCall& g, int bm, int parts, cudaLaunchAttribute (&attr)[2], cudaStream_t stream) {
+// `blocks`: of a cluster (1: none).
+template <int BM>
+static cudaLaunchConfig_t gt_config(const GtCall& g, int bm, int blocks, cudaLaunchAttribute (&attr)[2], cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((g.N + GT_BN - 1) / GT_BN * (SPLIT ? parts : 1)), (unsigned)((g.M + bm - 1) / bm), (unsigned)g.batch);
+    cfg.gridDim = dim3((unsigned)((g.N + GT_BN - 1) / GT_BN * blocks), (unsigned)((g.M + bm - 1) / bm), (unsigned)g.batch);
     cfg.blockDim = dim3(GT_THREADS);
     cfg.dynamicSmemBytes = gt_smem(BM) + 1024;
     cfg.stream = stream;
     int n = 0;
-    if (SPLIT) {
+    if (blocks > 1) {
         attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = parts;
+        attr[n].val.clusterDim.x = blocks;
         attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
         ++n;
     }
@@ -410,83 +423,106 @@ static cudaLaunchConfig_t gt_config(const GtCall& g, int bm, int parts, cudaLaun
     return cfg;
 }
 
-template <int BM, bool VEC, bool SPLIT>
+template <int BM, bool VEC, int PER>
 static int gt_launch(const GtCall& g, int bm, int parts, int len, cudaStream_t stream) {
-    auto kernel = gemm_f32_tc_kernel<BM, VEC, SPLIT>;
-    static_assert(gt_stages_bytes(BM) >= BM * GT_BN * 4, "a part's sums fit into the stages");
+    auto kernel = gemm_f32_tc_kernel<BM, VEC, PER>;
+    static_assert(gt_stages_bytes(BM) >= PER * BM * GT_BN * 4, "the parts' sums fit into the stages");
     static bool configured[VX_MAX_DEVICES];
     if (int rc = vx_configure_smem(kernel, gt_smem(BM) + 1024, configured)) return rc;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = gt_config<BM, VEC, SPLIT>(g, bm, parts, attr, stream);
+    const cudaLaunchConfig_t cfg = gt_config<BM>(g, bm, PER ? (parts + PER - 1) / (PER ? PER : 1) : 1, attr, stream);
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, g, bm, parts, len);
     if (e != cudaSuccess) return (int)e;
     VX_LAUNCH_CHECK();
     return VX_OK;
 }
 
-// Clusters of `parts` blocks that run at once (a block fills an SM; clusters lie within a group of SMs: 33 of four, 15 of eight).
-static int gt_clusters(int parts, int sms) {
+// Clusters of `blocks` blocks that run at once (a block fills an SM; clusters lie within a group of SMs: 33 of four, 15 of eight).
+static int gt_clusters(int blocks, int sms) {
     static int cache[VX_MAX_DEVICES][GT_MAX_PARTS + 1];
     const int dev = vx_current_device();
-    if (dev < 0) return sms / parts;
-    if (!cache[dev][parts]) {
+    if (dev < 0) return sms / blocks;
+    if (!cache[dev][blocks]) {
         static bool configured[VX_MAX_DEVICES];
-        auto kernel = gemm_f32_tc_kernel<128, true, true>;
+        auto kernel = gemm_f32_tc_kernel<128, true, 1>;
         GtCall g = {};
         g.M = g.N = g.K = g.batch = 1;
         cudaLaunchAttribute attr[2];
-        cudaLaunchConfig_t cfg = gt_config<128, true, true>(g, 16, parts, attr, nullptr);
+        cudaLaunchConfig_t cfg = gt_config<128>(g, 16, blocks, attr, nullptr);
         cfg.numAttrs = 1;   // (the cluster's size alone)
         int n = 0;
         if (vx_configure_smem(kernel, gt_smem(128) + 1024, configured) != VX_OK ||
             cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
-            n = sms / parts;
+            n = sms / blocks;
         }
-        cache[dev][parts] = n;
+        cache[dev][blocks] = n;
     }
-    return cache[dev][parts];
+    return cache[dev][blocks];
 }
 
 template <int BM>
-static int gt_go(const GtCall& g, bool vec, bool split, int bm, int parts, int len, cudaStream_t stream) {
-    if (split) return vec ? gt_launch<BM, true, true>(g, bm, parts, len, stream) : gt_launch<BM, false, true>(g, bm, parts, len, stream);
-    return vec ? gt_launch<BM, true, false>(g, bm, parts, len, stream) : gt_launch<BM, false, false>(g, bm, parts, len, stream);
+static int gt_go(const GtCall& g, bool vec, int per, int bm, int parts, int len, cudaStream_t stream) {
+#define GT_GO(PER_) return vec ? gt_launch<BM, true, PER_>(g, bm, parts, len, stream) : gt_launch<BM, false, PER_>(g, bm, parts, len, stream)
+    if (per == 1) GT_GO(1);
+    if (per == 2) GT_GO(2);
+    if (per == 4) GT_GO((BM <= 32 ? 4 : 2));
+    GT_GO(0);
+#undef GT_GO
 }
 
-// Row tiles, and whether the parts of k go to the blocks of a cluster: what takes the least time by the rounds of the SMs (of the
-// clusters that run at once) and the time of a round, which was measured: a chunk takes 1.17 us and 4.5 ns a row up to 64 rows of A, 20 ns a
-// row above; a round 2 us besides, with a cluster's sums 4 us and 10 ns a row.
-// Measured, us, multiply-adds (gemm_f32.cu) and this (rows x N x K): 1 x 4096 x 1024 10.2, 8.6; 24 x 4096 x 1024 14.5, 9.9; 99 x 4096 x 1024 38.4, 14.3;
-// 99 x 1024 x 2048 21.1, 13.1; 99 x 6144 x 1024 56.4, 23.8; 99 x 1024 x 3072 29.5, 16.6; 158 x 1024 x 2048 28, 20.4; 300 x 4096 x 2048 170, 68.6;
-// 2000 x 4096 x 1024 428, 162; 8 x 6144 x 1024 14.5, 16.5; 8 x 2560 x 9728 47.9, 51.8 (a few rows on a wide W: the two places where multiply-adds are ahead).
+// Row tiles (`bm` rows each), and whether and how the parts of k go to the blocks of a cluster (`per` parts a block, 0: no cluster): what takes
+// the least time by the rounds of the SMs (of the clusters that run at once) and the time of a round, which was measured: a chunk takes 1.17 us
+// and 4.5 ns a row up to 64 rows of A, 20 ns a row above; a round 2 us besides, with a cluster's sums 4 us and 10 ns a row.  Returns that time.
+static double gt_plan(int M, int K, long long columns, int sms, int* best_bm, int* per) {
+    int parts, len;
+    gt_parts(K, &parts, &len);
+    double best = 0;
+    *best_bm = 0;
+    for (int t = (M + 127) / 128; t <= (M + 127) / 128 + 3; ++t) {
+        const int bm = ((M + t - 1) / t + 15) / 16 * 16;
+        const long long tiles = columns * ((M + bm - 1) / bm);
+        const double chunk = 1.17 + 0.0045 * bm + (bm > 64 ? 0.0155 * (bm - 64) : 0.0);
+        for (int p = 0; p < parts && p <= (bm <= 32 ? 4 : 2); p = p ? 2 * p : 1) {   // (a cluster has two blocks or more)
+            const int at_once = p ? gt_clusters((parts + p - 1) / p, sms) : sms, k = p ? p * len : K;
+            const double cost = (double)((tiles + at_once - 1) / at_once) * ((p ? 4.0 + 0.01 * bm : 2.0) + chunk * ((k + GT_BK - 1) / GT_BK));
+            if (!*best_bm || cost < best) { *best_bm = bm; *per = p; best = cost; }
+        }
+        if (bm <= 16) break;
+    }
+    return best;
+}
+
+// Whether a float32 product takes the tensor cores.  N and K alone say, because a row's result must not depend on how many rows the call has: a
+// product that one call has for a decoded token another has for a prompt.  So they are taken where they are not slower for a few rows either: by
+// estimates of both for eight rows, not by more than an eighth (the multiply-adds': a part's chain, 42 ns a k; 2.9 TB/s and 4.5 us).  Not for k
+// below 1,024, where multiply-adds have short parts, nor for more than 32,768 columns, a vocabulary's head, of which a step wants a few rows.
+// Measured, us, multiply-adds and tensor cores (N x K), 8 rows: 4096 x 1024 10.9, 9.8; 6144 x 1024 14.8, 14.4; 1024 x 3072 14.0, 11.9; 4096 x 4096
+// 28, 26.7; 4096 x 12288 74, 66; 12288 x 2048 40.9, 44.2; 24576 x 4096 122, 133; 2560 x 4096 22.2, 25; refused: 2048 x 2048 11.5, 14.2;
+// 19456 x 2560 67.6, 88; 3072 x 512 5.1, 7.9; 8192 x 768 13.3, 14.8.
+// 99 rows: 4096 x 1024 39, 17.6; 6144 x 1024 57, 26; 1024 x 3072 29.7, 21.7; 12288 x 2048 195, 87; 24576 x 4096 733, 284; 300 rows:
+// 6144 x 1024 127, 46; 1024 x 2048 54, 25; 4096 x 12288 929, 395; (refused) 19456 x 2560 835, 355; 3072 x 512 37, 16.
+extern "C" int vx_gemm_f32_takes_tc(int N, int K) {
+    if (K < 1024 || N <= 0 || N > 32768) return 0;
+    static int sms_cache[VX_MAX_DEVICES];
+    int parts, len, bm, per;
+    gt_parts(K, &parts, &len);
+    const double chain = (long long)N * K < (6 << 20) ? 0.034 * len : 0.0425 * len, bytes = 4.5 + 4.0 * N * K / 2.9e6;
+    return gt_plan(8, K, (N + GT_BN - 1) / GT_BN, vx_sm_count(sms_cache), &bm, &per) <= 1.125 * (chain > bytes ? chain : bytes);
+}
+
 int vx_gemm_f32_tc(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int lda, int ldw, int ldc, int batch,
                    long long sa, long long sw, long long sc, int w_ready, int* error, cudaStream_t stream) {
     const GtCall g = {A, W, bias, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready, error};
     // rows that begin on 16-byte addresses are fetched 16 bytes at a time, others four
     const bool vec = !((lda | ldw) & 3) && !((sa | sw) & 3) && !((((uintptr_t)A) | ((uintptr_t)W)) & 15);
     static int sms_cache[VX_MAX_DEVICES];
-    const int sms = vx_sm_count(sms_cache);
-    int parts, len;
+    int parts, len, bm, per;
     gt_parts(K, &parts, &len);
-    const long long columns = (long long)((N + GT_BN - 1) / GT_BN) * batch;
-    int best_bm = 0;
-    bool split = false;
-    double best = 0;
-    for (int t = (M + 127) / 128; t <= (M + 127) / 128 + 3; ++t) {
-        const int bm = ((M + t - 1) / t + 15) / 16 * 16;
-        const long long tiles = columns * ((M + bm - 1) / bm);
-        const double chunk = 1.17 + 0.0045 * bm + (bm > 64 ? 0.0155 * (bm - 64) : 0.0);
-        for (int s = 0; s < (parts > 1 ? 2 : 1); ++s) {
-            const int at_once = s ? gt_clusters(parts, sms) : sms;
-            const double cost = (double)((tiles + at_once - 1) / at_once) * ((s ? 4.0 + 0.01 * bm : 2.0) + chunk * (((s ? len : K) + GT_BK - 1) / GT_BK));
-            if (!best_bm || cost < best) { best_bm = bm; split = s; best = cost; }
-        }
-        if (bm <= 16) break;
-    }
-    if ((M + best_bm - 1) / best_bm > 65535) return VX_ERR_LIMIT;
-    if (best_bm <= 16) return gt_go<16>(g, vec, split, best_bm, parts, len, stream);
-    if (best_bm <= 32) return gt_go<32>(g, vec, split, best_bm, parts, len, stream);
-    if (best_bm <= 64) return gt_go<64>(g, vec, split, best_bm, parts, len, stream);
-    return gt_go<128>(g, vec, split, best_bm, parts, len, stream);
+    gt_plan(M, K, (long long)((N + GT_BN - 1) / GT_BN) * batch, vx_sm_count(sms_cache), &bm, &per);
+    if ((M + bm - 1) / bm > 65535) return VX_ERR_LIMIT;
+    if (bm <= 16) return gt_go<16>(g, vec, per, bm, parts, len, stream);
+    if (bm <= 32) return gt_go<32>(g, vec, per, bm, parts, len, stream);
+    if (bm <= 64) return gt_go<64>(g, vec, per, bm, parts, len, stream);
+    return gt_go<128>(g, vec, per, bm, parts, len, stream);
 }

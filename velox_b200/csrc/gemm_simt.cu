@@ -80,10 +80,7 @@ gemm_nt_simt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const fl
 // `w_ready`: W (a model's weights, say) is not something the kernel launched just before this one writes; the float32 product
 // then asks for its first chunks before it waits for that kernel.  `error` (may be null): a device int that the float32 product sets if it
 // gives up its wait for the tensor core; its results are NaN then.
-//
-// Which float32 product: N and K alone say (a row's result must not depend on how many rows the call has).  The tensor cores, except
-// for k up to 256, where they have no time to get going (1 x 1024 x 256: multiply-adds 3.5 us, tensor cores 6.6; 37 x 64 x 64 3.8, 3.5), and
-// for more than 32,768 columns, a vocabulary's head, of which a step wants a few rows (4 x 151936 x 1024: 144, 193).
+// Which float32 product: vx_gemm_f32_takes_tc, by N and K alone.
 extern "C" int vx_gemm_nt_simt_checked(const void* A, const void* W, const float* bias, void* C, int M, int N,
                                        int K, int lda, int ldw, int ldc, int batch, long long sa, long long sw,
                                        long long sc, int in_dtype, int out_dtype, int w_ready, int* error, cudaStream_t stream) {
@@ -93,7 +90,7 @@ extern "C" int vx_gemm_nt_simt_checked(const void* A, const void* W, const float
     if (grid.y > 65535 || batch > 65535) return VX_ERR_LIMIT;
     if (in_dtype == VX_F32 && out_dtype == VX_F32) {
         const float *a = (const float*)A, *w = (const float*)W;
-        if (K > 256 && N <= 32768)
+        if (vx_gemm_f32_takes_tc(N, K))
             return vx_gemm_f32_tc(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready, error, stream);
         return vx_gemm_f32(a, w, bias, (float*)C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, w_ready, stream);
     }

@@ -151,6 +151,7 @@ def _declare(lib) -> None:
         "vx_sample": [P, I, I, I, P, P, P, P, P],
         "vx_qk_norm_rope_kv_pairs": [P, I, P, P, F, P, I, P, P, P, P, I, I, I, I, I, I, I, I, P],
         "vx_paged_attention_generic_cap": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, P],
+        "vx_gemm_f32_takes_tc": [I, I],
         "vx_gemm_nt_simt_checked": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, I, P, P],
         "vx_gemm_nt_simt_batched": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, P],
         "vx_linear_attention_walk": [P, I, I, I, I, P, P, I, F, P, I, I, P, F, F, P, P, P, P, I, I, I, I, I, P],
@@ -1033,9 +1034,22 @@ def paged_prefill_attention_tc(q: torch.Tensor, q_row_stride: int, k_pool, v_poo
     return out
 
 
+_F32_TAKES_TC = {}
+
+
+def _f32_takes_tc(n: int, k: int) -> bool:
+    """Whether float32 products of these sizes run on the tensor cores (`vx_gemm_f32_takes_tc`)."""
+    takes = _F32_TAKES_TC.get((n, k))
+    if takes is None:
+        if len(_F32_TAKES_TC) >= 4096:
+            _F32_TAKES_TC.clear()
+        takes = _F32_TAKES_TC[n, k] = library().vx_gemm_f32_takes_tc(n, k) == 1
+    return takes
+
+
 def _simt(a, w, bias, out, m, n, k, lda, ldw, ldc, batch, sa, sw, sc, w_ready, what) -> None:
-    """(The float32 product's waits for the tensor core are bounded: it reports into the error word.)"""
-    exact = a.dtype == torch.float32
+    """(The float32 product's waits for the tensor core are bounded: where it takes them it reports into the error word.)"""
+    exact = a.dtype == torch.float32 and out.dtype == torch.float32 and _f32_takes_tc(n, k)
     _check(library().vx_gemm_nt_simt_checked(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, lda, ldw, ldc, batch, sa, sw, sc,
                                              dtype_code(a.dtype), dtype_code(out.dtype), 1 if w_ready else 0,
                                              _ptr(_error_word(a.device)) if exact else None, _stream()), what)
@@ -1045,8 +1059,8 @@ def _simt(a, w, bias, out, m, n, k, lda, ldw, ldc, batch, sa, sw, sc, w_ready, w
 
 def gemm_nt_simt(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[torch.dtype] = None,
                  w_ready: bool = False) -> torch.Tensor:
-    """a [M,K] times w [N,K] transposed: float32 multiply-adds on the CUDA cores, or (float32 operands, k above 256) the tensor cores
-    with every operand in three bfloat16 parts, which is no less exact.  `w_ready` says that `w` is not something the
+    """a [M,K] times w [N,K] transposed: float32 multiply-adds on the CUDA cores, or (float32 operands, where `vx_gemm_f32_takes_tc`
+    says so) the tensor cores with every operand in three bfloat16 parts, which is no less exact.  `w_ready` says that `w` is not something the
     kernel launched just before this one writes (a model's weights never are): its first tiles may then be fetched before the wait for
     that kernel."""
     _dev(a, w, bias)
