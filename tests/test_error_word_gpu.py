@@ -16,15 +16,13 @@ def ops():
 def clean():
     ops().check_device_errors()
     yield
-    word = ops()._error_word(torch.device(DEV))
     torch.cuda.synchronize()
-    word.zero_()
+    ops()._error_word(torch.device(DEV)).zero_()
     ops().check_device_errors()
 
 
 def set_word():
     ops()._error_word(torch.device(DEV)).fill_(8)
-    torch.cuda.synchronize()   # (a kernel's own report is there when the kernel has ended)
 
 
 def products():
@@ -51,6 +49,21 @@ def test_products_with_bounded_waits_are_checked(name):
     with pytest.raises(o.KernelError, match="gave up a wait"):
         o.check_pending_device_errors()
     o.check_pending_device_errors()   # (reported once)
+
+
+def test_a_kernel_writes_the_error_word_and_the_host_reads_it():
+    """The word lies in host memory: what a kernel stores there (the sampler its token id, 8) is there when the kernel has ended."""
+    o = ops()
+    logits = torch.zeros(1, 64, device=DEV)
+    logits[0, 8] = 1.0
+    word = o._error_word(torch.device(DEV))
+    assert int(word[0]) == 0 and word.data_ptr() == o._error_address(torch.device(DEV))
+    o._check(o.library().vx_sample(o._ptr(logits), 64, 1, 64, None, None, None, o._ptr(word), o._stream()), "sample")
+    torch.cuda.synchronize()
+    assert int(word[0]) == 8
+    with pytest.raises(o.KernelError, match="code 8"):
+        o.check_device_errors()
+    assert int(word[0]) == 0
 
 
 def engine(dtype, vocab=512):

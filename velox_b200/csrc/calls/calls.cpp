@@ -71,6 +71,14 @@ struct Scalars {
         if (overflow || v != (int)v) bad = true;
         return (int)v;
     }
+    void* p(PyObject* o) {   // (an address; none is 0)
+        void* v = PyLong_Check(o) ? PyLong_AsVoidPtr(o) : nullptr;
+        if (!v) {
+            PyErr_Clear();
+            bad = true;
+        }
+        return v;
+    }
     float f(PyObject* o) {
         if (PyFloat_Check(o)) return (float)PyFloat_AS_DOUBLE(o);
         return (float)i(o);
@@ -204,40 +212,42 @@ PyObject* gemm_bf16(PyObject*, PyObject* const* o, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// (a, w, bias, epilogue code, activation, columns of a tile or 0, pair, error word)
+// (a, w, bias, epilogue code, activation, columns of a tile or 0, pair, the error word's address)
 PyObject* gemm_tcgen05(PyObject*, PyObject* const* o, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 8) NOT_HERE;
-    Arg a(o[0]), w(o[1]), error(o[7]);
+    Arg a(o[0]), w(o[1]);
     Optional bias(o[2]);
     Scalars sc;
     const int code = sc.i(o[3]), act = sc.i(o[4]), columns = sc.i(o[5]), pair = sc.i(o[6]);
-    if (sc.bad || !a || !w || !is(error, at::kInt) || !bias.is(at::kFloat) || !tcgen05_takes(*a, *w)) NOT_HERE;
+    void* const error = sc.p(o[7]);
+    if (sc.bad || !a || !w || !bias.is(at::kFloat) || !tcgen05_takes(*a, *w)) NOT_HERE;
     const int64_t M = a->size(0), N = w->size(0), cols = code == 1 ? N / 2 : N;
     if ((bias && bias.a->numel() != N) || cols % 8) NOT_HERE;
     at::Tensor out = fresh(M, cols, at::kBFloat16, *a);
     LAUNCH(rc, pair ? entry.gemm_tcgen05_pair(a->data_ptr(), w->data_ptr(), bias.ptr(), out.data_ptr(), (int)M, (int)N, (int)a->size(1),
-                                              (int)a->stride(0), (int)w->stride(0), (int)cols, code, act, error->data_ptr(), s)
+                                              (int)a->stride(0), (int)w->stride(0), (int)cols, code, act, error, s)
                     : entry.gemm_tcgen05_columns(a->data_ptr(), w->data_ptr(), bias.ptr(), out.data_ptr(), (int)M, (int)N, (int)a->size(1),
-                                                 (int)a->stride(0), (int)w->stride(0), (int)cols, code, act, columns, error->data_ptr(), s));
+                                                 (int)a->stride(0), (int)w->stride(0), (int)cols, code, act, columns, error, s));
     return result(rc, std::move(out));
     END_HANDLE_TH_ERRORS
 }
 
-// (a, w, gated, activation, out dtype, w is ready, error word)
+// (a, w, gated, activation, out dtype, w is ready, the error word's address)
 PyObject* gemm_turned(PyObject*, PyObject* const* o, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 7) NOT_HERE;
-    Arg a(o[0]), w(o[1]), error(o[6]);
+    Arg a(o[0]), w(o[1]);
     Scalars sc;
     const int gated = sc.i(o[2]), act = sc.i(o[3]), ready = sc.i(o[5]);
-    if (sc.bad || !a || !w || !THPDtype_Check(o[4]) || !is(error, at::kInt) || !tcgen05_takes(*a, *w)) NOT_HERE;
+    void* const error = sc.p(o[6]);
+    if (sc.bad || !a || !w || !THPDtype_Check(o[4]) || !tcgen05_takes(*a, *w)) NOT_HERE;
     const at::ScalarType kind = ((THPDtype*)o[4])->scalar_type;
     const int64_t M = a->size(0), N = w->size(0), cols = gated ? N / 2 : N;
     if (code_of(kind) < 0 || cols % 8) NOT_HERE;
     at::Tensor out = fresh(M, cols, kind, *a);
     LAUNCH(rc, entry.gemm_turned(a->data_ptr(), w->data_ptr(), out.data_ptr(), (int)M, (int)N, (int)a->size(1), (int)a->stride(0),
-                                 (int)w->stride(0), (int)cols, gated, act, code_of(kind), ready, error->data_ptr(), s));
+                                 (int)w->stride(0), (int)cols, gated, act, code_of(kind), ready, error, s));
     return result(rc, std::move(out));
     END_HANDLE_TH_ERRORS
 }
@@ -264,22 +274,23 @@ struct Attention {
 };
 
 // (q, row stride, k_pool, v_pool, block table, cu_seqlens, kv_offsets, scale, window, heads, kv heads, head size, requests,
-//  max_new, tokens, seq_list, out, scratch, max_splits, error word)
+//  max_new, tokens, seq_list, out, scratch, max_splits, the error word's address)
 PyObject* prefill_attention(PyObject*, PyObject* const* o, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 20) NOT_HERE;
     Attention x(o[0], o[2], o[3], o[4], o[16]);
-    Arg cu(o[5]), offsets(o[6]), error(o[19]);
+    Arg cu(o[5]), offsets(o[6]);
     Optional list(o[15]), scratch(o[17]);
     Scalars sc;
     const int ld = sc.i(o[1]), window = sc.i(o[8]), H = sc.i(o[9]), Hk = sc.i(o[10]), D = sc.i(o[11]), requests = sc.i(o[12]),
               max_new = sc.i(o[13]), tokens = sc.i(o[14]), splits = sc.i(o[18]);
     const float scale = sc.f(o[7]);
-    if (sc.bad || !x.fine(D) || !cu || !offsets || !is(error, at::kInt) || !list.ok || !scratch.is(at::kFloat)) NOT_HERE;
+    void* const error = sc.p(o[19]);
+    if (sc.bad || !x.fine(D) || !cu || !offsets || !list.ok || !scratch.is(at::kFloat)) NOT_HERE;
     at::Tensor out = x.out ? *x.out.a : fresh(tokens, (int64_t)H * D, at::kBFloat16, *x.q);
     LAUNCH(rc, entry.prefill(x.q->data_ptr(), ld, tokens, x.k->data_ptr(), x.v->data_ptr(), (int)x.k->size(0), x.table->data_ptr(),
                              (int)x.table->size(1), cu->data_ptr(), offsets->data_ptr(), list.ptr(), out.data_ptr(), H * D, scale, window,
-                             requests, max_new, H, Hk, D, (int)x.k->size(2), scratch.ptr(), splits, error->data_ptr(), s));
+                             requests, max_new, H, Hk, D, (int)x.k->size(2), scratch.ptr(), splits, error, s));
     return result(rc, std::move(out));
     END_HANDLE_TH_ERRORS
 }

@@ -13,6 +13,7 @@ import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional, Tuple
 
+import numpy as np
 import torch
 
 from . import build as _build
@@ -202,6 +203,7 @@ def _declare(lib) -> None:
         "vx_latent_gather_window": [P, P, I, P, P, P, P, I, P, I, I, I, I, I, I, I, P],
     }
     lib.vx_set_pdl_mask.argtypes = [I]
+    lib.vx_host_word.argtypes, lib.vx_host_word.restype = [], c_void_p
     lib.vx_set_pdl_mask.restype = None
     lib.vx_set_pdl.argtypes = [I]
     lib.vx_set_pdl.restype = None
@@ -1006,7 +1008,7 @@ def paged_prefill_attention_tc(q: torch.Tensor, q_row_stride: int, k_pool, v_poo
     if not halves and sinks is None and gate_col < 0:
         done = (_CALLS or _calls()).prefill_attention(q, q_row_stride, k_pool, v_pool, block_table, cu_seqlens, kv_offsets, scale, window,
                                                       num_heads, num_kv_heads, head_dim, requests, max_new, tokens, seq_list, out,
-                                                      scratch, max_splits, _error_word(q.device))
+                                                      scratch, max_splits, _error_address(q.device))
         if done is not None:
             done = _called(done, "paged_prefill_attention_tc")
             note_bounded_wait()
@@ -1637,15 +1639,25 @@ def _sm_count(device) -> int:
     return count
 
 
-_ERROR_WORDS = {}
+_ERROR_WORDS = {}   # device: (the word, its address)
 
 
 def _error_word(device) -> torch.Tensor:
-    """The device int that kernels with bounded waits report into."""
-    word = _ERROR_WORDS.get(device)
-    if word is None:
-        word = _ERROR_WORDS[device] = torch.zeros(1, dtype=torch.int32, device=device)
-    return word
+    """The int that kernels with bounded waits report into, in host memory that the device writes: a host that has waited for a
+    kernel reads it without a copy."""
+    return (_ERROR_WORDS.get(device) or _new_error_word(device))[0]
+
+
+def _error_address(device) -> int:
+    return (_ERROR_WORDS.get(device) or _new_error_word(device))[1]
+
+
+def _new_error_word(device):
+    address = library().vx_host_word()
+    if not address:
+        raise KernelError("no host memory that the device can write")
+    word = torch.from_numpy(np.ctypeslib.as_array((ctypes.c_int32 * 1).from_address(address)))
+    return _ERROR_WORDS.setdefault(device, (word, address))
 
 
 _BOUNDED_WAIT_LAUNCHES = 0   # launches of kernels with bounded waits, ever
@@ -1684,7 +1696,6 @@ class EndOfWaits:
 
 
 _END_OF_WAITS = (-1, None)   # the latest end: (launches with bounded waits before it, its event)
-_READERS = {}                # device: the stream on which the error word is read without waiting for what runs
 
 
 def note_end_of_waits(end: EndOfWaits) -> None:
@@ -1704,7 +1715,7 @@ def check_pending_device_errors() -> None:
         launches, event = _END_OF_WAITS
         if launches == _BOUNDED_WAIT_LAUNCHES:
             event.synchronize()
-            _read_error_words(True)
+            _read_error_words()
         else:
             check_device_errors()
 
@@ -1712,22 +1723,17 @@ def check_pending_device_errors() -> None:
 def check_device_errors() -> None:
     """Raises if a kernel has reported that one of its bounded waits ran out since
     the last check (its results are then missing).  Synchronises the device."""
-    _read_error_words(False)
+    for key in _ERROR_WORDS:
+        torch.cuda.current_stream(key).synchronize()
+    _read_error_words()
 
 
-def _read_error_words(reached: bool) -> None:
-    """`reached`: the kernels in question have ended; the words are read beside what runs now, else behind it."""
+def _read_error_words() -> None:
+    """(The kernels in question have ended.)"""
     global _BOUNDED_WAIT_CHECKED
     _BOUNDED_WAIT_CHECKED = _BOUNDED_WAIT_LAUNCHES
-    for key, word in _ERROR_WORDS.items():
-        if reached:
-            reader = _READERS.get(key)
-            if reader is None:
-                reader = _READERS[key] = torch.cuda.Stream(word.device)
-            with torch.cuda.stream(reader):
-                code = int(word.item())
-        else:
-            code = int(word.item())
+    for key, (word, address) in _ERROR_WORDS.items():
+        code = ctypes.c_int32.from_address(address).value
         if code:
             word.zero_()
             raise KernelError("a kernel on %s gave up a wait on its asynchronous copies or tensor-core work "
@@ -1795,7 +1801,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
     _need(not (pair and activation), "gemm_tcgen05: a plain activation on tiles of single blocks")
     if gated_activation is None or gated_activation in ACTIVATIONS:
         out = (_CALLS or _calls()).gemm_tcgen05(a, w, bias, code, ACTIVATIONS.get(gated_activation, 0) if pair else act, columns or (256 if wide else 0),
-                                                1 if pair else 0, _error_word(a.device))
+                                                1 if pair else 0, _error_address(a.device))
         if out is not None:
             out = _called(out, "gemm_tcgen05_pair" if pair else "gemm_tcgen05")
             note_bounded_wait()
@@ -1848,7 +1854,7 @@ def gemm_turned(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtyp
     out_dtype = out_dtype or torch.bfloat16
     _need(gated_activation is None or gated_activation in ACTIVATIONS, "gemm_turned: unknown activation %r" % gated_activation)
     gated, act = (0, 0) if gated_activation is None else (1, ACTIVATIONS[gated_activation])
-    out = (_CALLS or _calls()).gemm_turned(a, w, gated, act, out_dtype, 1 if w_ready else 0, _error_word(a.device))
+    out = (_CALLS or _calls()).gemm_turned(a, w, gated, act, out_dtype, 1 if w_ready else 0, _error_address(a.device))
     if out is not None:
         out = _called(out, "gemm_turned")
     else:
