@@ -517,6 +517,26 @@ def test_gemm_turned(M, N, K):
     ops().check_device_errors()
 
 
+@pytest.mark.parametrize("M,N,K", [(24, 24576, 512), (24, 2560, 4096), (50, 12288, 512), (150, 6144, 1024), (312, 4096, 2048)])
+def test_gemm_turned_waits_for_a_w_that_was_just_written(M, N, K):
+    """W written by the kernel launched just before, in memory that holds NaN until then: without `w_ready` the product sees it whole, with every
+    kind of tile that is chosen; with `w_ready` and a W that is, the same bits."""
+    a = rnd((M, K), torch.bfloat16, 1)
+    for seed in range(4):
+        x = rnd((N, 2 * K), torch.float32, 10 + seed)
+        w = ops().gated_act(x, "silu", out_dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        want = [ops().gemm_turned(a, w, w_ready=True), ops().gemm_turned(a, w, gated_activation="silu", w_ready=True)]
+
+        def just_written():
+            torch.full((N, K), float("nan"), dtype=torch.bfloat16, device=DEV)   # (given back at once: the block that the next result of this size takes)
+            return ops().gated_act(x, "silu", out_dtype=torch.bfloat16)
+
+        assert torch.equal(ops().gemm_turned(a, just_written()), want[0])
+        assert torch.equal(ops().gemm_turned(a, just_written(), gated_activation="silu"), want[1])
+    ops().check_device_errors()
+
+
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("M,N,K", [(1, 53, 72), (37, 64, 16), (130, 136, 104), (64, 384, 96), (8, 4096, 4096)])
 def test_gemm_bf16(M, N, K, out_dtype):
