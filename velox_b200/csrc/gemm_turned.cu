@@ -483,13 +483,24 @@ extern "C" int vx_gemm_turned(const void* A, const void* W, void* C, int M, int 
 }
 
 // Whether a step's product of M rows with a model's weights is fastest this way, with its neighbours in the step: the kernels before and
-// after it overlap it (programmatic launch), which they don't with the library's product; that is worth 1.5 to 3 us.
-// Alone, us, library and this: 24 x 2560 x 9728 15.2, 12.3; 24 x 6144 x 2560 8.4, 8.5; 64 x 6144 x 4096 11.5, 13.0; 312 x 2560 x 9728 25.1, 19.9;
-// 230 x 6144 x 2560 10.6, 12.5; 512 x 2560 x 9728 23.5, 26.6.  Gated (the library's with the activation's kernel, or gemm_tcgen05's): 24 x 24576 x 4096
-// 39.0, 35.3; 150 x 19456 x 2560 29.9, 26.0; 312 x 19456 x 2560 39.3, 33.6; 777 x 24576 x 4096 137, 124; 777 x 12288 x 2048 41.7, 41.8;
-// 777 x 6144 x 1024 18.9, 21.0.
+// after it overlap it (programmatic launch), which they don't with the library's product.
+// Measured in steps of 12 layers (us a step: without it and with it, everything else the same; shapes of 0.6B, 1.7B, 4B and 8B, whose gated products
+// have N = 6,144, 12,288, 19,456 and 24,576 and whose deep ones 1,024 x 3072, 2,048 x 6144, 2,560 x 9728 and 4,096 x 12288):
+//   9 to 32 rows   all products: 9 rows 643, 527; 733, 734; 1,025, 955; 1,437, 1,361; 32 rows 741, 694; 863, 855; 1,118, 1,075; 1,539, 1,492.
+//   33 to 64 rows  wide gated and large deep ones.  For the others what they gain is less than what the host's wait for the step costs, which the
+//                  library's products do without: 64 rows, none at all 829, all 956 (0.6B); 1,042, 1,079 (1.7B); alone 64 x 6144 x 2560 9.2 us, 13.0.
+//   gated, above   up to 400 rows for N below 8,192 (150 rows 1,123, 1,041; 777 alone 18.9 us, 21.0), 640 below 16,384 (400 rows 1,369, 1,315; 512
+//                  1,430, 1,425; 720 1,610, 1,629), else 800 (4B 312 rows 1,667, 1,577; 760 2,543, 2,485; 850 2,752, 2,744).  Not 225 to 256 rows
+//                  of the middle ones, which are two whole tiles of gemm_tcgen05 (1,202, 1,240; 264 rows 1,240, 1,183).
+//   deep (K of 2 N and more), above   up to 320 rows: 70 rows 1,141, 1,108 (1.7B); 150 rows 1,395, 1,353 (4B); 200 rows 2,082, 1,964 (8B); 312 rows
+//                  1,664, 1,577 (4B); 328 1,676, 1,669; 360 1,682, 1,696.  Not 225 to 256 rows, whole tiles of the library's (1,481, 1,513; 1,990, 2,051),
+//                  nor, for N of 2,048, more than 192 (208 rows 1,162, 1,181; 312 1,204, 1,221); but of smaller ones, whose steps wait for the
+//                  host's launches (256 rows 1,139, 1,053).
+// Where more than 64 rows are there a step has a prompt's attention, whose waits the host waits for anyway.
 extern "C" int vx_gemm_turned_wins(int M, int N, int K, int gated) {
-    if (M <= 8 || N <= 0 || K <= 0 || (N & 15) || (K & 7)) return 0;
-    if (gated) return M <= (N >= 8192 ? 800 : 400);
-    return N <= 32768 && (M <= 64 || (M <= 320 && K >= 2 * N));
+    if (M <= 8 || N <= 0 || K <= 0 || (N & 15) || (K & 7) || (!gated && N > 32768)) return 0;
+    if (M <= 32) return 1;
+    const bool whole = M > 224 && M <= 256;
+    if (gated) return N >= 16384 ? M <= 800 : (M > 64 && (N >= 8192 ? M <= 640 && !whole : M <= 400));
+    return K >= 2 * N && (M <= 64 ? N >= 2560 : (N < 2048 ? M <= 320 : (N < 2560 ? M <= 192 : M <= 320 && !whole)));
 }

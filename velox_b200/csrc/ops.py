@@ -1829,7 +1829,7 @@ def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, bias=None, gated_activation: 
     return out
 
 
-TURNED_MAX_ROWS = 800   # from which on `turned_wins` never holds
+TURNED_MAX_ROWS, TURNED_GATED_MAX_ROWS = 320, 800   # above which `turned_wins` never holds
 _TURNED = {}
 
 

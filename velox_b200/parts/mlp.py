@@ -61,7 +61,7 @@ class GatedMLP(FeedForward):
         if fused and ops.skinny_supported(h.shape[0], h.shape[1], h, w):
             # a decode step: W streamed once, act(gate) * up taken on the accumulators
             a = ops.gemm_skinny(h, w, None, h.dtype, gated_activation=self.activation)
-        elif fused and ops.turned_wins(h.shape[0], w.shape[0], h.shape[1], True) and ops.tcgen05_supported(h, w):
+        elif fused and h.shape[0] <= ops.TURNED_GATED_MAX_ROWS and ops.turned_wins(h.shape[0], w.shape[0], h.shape[1], True) and ops.tcgen05_supported(h, w):
             # a wider decode step, a mixed step, a shorter prompt portion: the same epilogue on the turned product
             a = ops.gemm_turned(h, w, h.dtype, gated_activation=self.activation, w_ready=True)
         elif fused and h.shape[0] >= FUSED_TCGEN05_MIN_ROWS and ops.tcgen05_supported(h, w):
