@@ -563,50 +563,3 @@ extern "C" int vx_paged_attention_generic_requests(const void* q, int q_row_stri
     VX_LAUNCH_CHECK();
     return VX_OK;
 }
-
-extern "C" int vx_paged_attention_generic_chunk(const void* q, int q_row_stride, const void* k_pool,
-                                                 const void* v_pool, const int* block_table, int max_blocks,
-                                                 const int* seq_of_token, const int* positions, void* out,
-                                                 int out_row_stride, float scale, int window, int tokens,
-                                                 int H, int Hk, int D, int S, int dtype, int Dv, int keep_first,
-                                                 float bias_exp, const float* sinks, int gate_col, float softcap,
-                                                 int v_stride, int v_share, int out_f32, int chunk, cudaStream_t stream) {
-    return vx_paged_attention_generic_requests(q, q_row_stride, k_pool, v_pool, block_table, max_blocks, seq_of_token, positions, out,
-                                               out_row_stride, scale, window, tokens, H, Hk, D, S, dtype, Dv, keep_first, bias_exp, sinks,
-                                               gate_col, softcap, v_stride, v_share, out_f32, chunk, 0, stream);
-}
-
-extern "C" int vx_paged_attention_generic_shared(const void* q, int q_row_stride, const void* k_pool,
-                                                 const void* v_pool, const int* block_table, int max_blocks,
-                                                 const int* seq_of_token, const int* positions, void* out,
-                                                 int out_row_stride, float scale, int window, int tokens,
-                                                 int H, int Hk, int D, int S, int dtype, int Dv, int keep_first,
-                                                 float bias_exp, const float* sinks, int gate_col, float softcap,
-                                                 int v_stride, int v_share, int out_f32, cudaStream_t stream) {
-    return vx_paged_attention_generic_chunk(q, q_row_stride, k_pool, v_pool, block_table, max_blocks, seq_of_token, positions,
-                                            out, out_row_stride, scale, window, tokens, H, Hk, D, S, dtype, Dv, keep_first,
-                                            bias_exp, sinks, gate_col, softcap, v_stride, v_share, out_f32, 0, stream);
-}
-
-extern "C" int vx_paged_attention_generic_cap(const void* q, int q_row_stride, const void* k_pool,
-                                              const void* v_pool, const int* block_table, int max_blocks,
-                                              const int* seq_of_token, const int* positions, void* out,
-                                              int out_row_stride, float scale, int window, int tokens,
-                                              int H, int Hk, int D, int S, int dtype, int Dv, int keep_first,
-                                              float bias_exp, const float* sinks, int gate_col, float softcap,
-                                              int v_stride, cudaStream_t stream) {
-    return vx_paged_attention_generic_shared(q, q_row_stride, k_pool, v_pool, block_table, max_blocks, seq_of_token, positions,
-                                             out, out_row_stride, scale, window, tokens, H, Hk, D, S, dtype, Dv, keep_first,
-                                             bias_exp, sinks, gate_col, softcap, v_stride, 1, 0, stream);
-}
-
-extern "C" int vx_paged_attention_generic(const void* q, int q_row_stride, const void* k_pool,
-                                          const void* v_pool, const int* block_table, int max_blocks,
-                                          const int* seq_of_token, const int* positions, void* out,
-                                          int out_row_stride, float scale, int window, int tokens,
-                                          int H, int Hk, int D, int S, int dtype, int Dv, int keep_first,
-                                          float bias_exp, const float* sinks, int gate_col, cudaStream_t stream) {
-    return vx_paged_attention_generic_cap(q, q_row_stride, k_pool, v_pool, block_table, max_blocks, seq_of_token, positions,
-                                          out, out_row_stride, scale, window, tokens, H, Hk, D, S, dtype, Dv, keep_first,
-                                          bias_exp, sinks, gate_col, 0.f, 0, stream);
-}

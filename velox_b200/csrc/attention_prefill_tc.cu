@@ -32,7 +32,7 @@
 //               (warp 11).
 // Registers move from warps 8-11 to the softmax warps (setmaxnreg).  The two query tiles' softmaxes (a thread is busy for
 // 1,830 cycles a key tile) and the 32 products of 128 x 128 x 16 per key tile take turns; with the products issued by an elected
-// lane (tc_elect) 1,000 tokens on 15,000 keys take 261 us (274 under `lane == 0`), 8,192 tokens 666 (689).
+// lane (tc_elect) 1,000 tokens on 15,000 keys, 32 heads on 8, take 231 us (246 under `lane == 0`), 8,192 tokens 450 (470).
 //
 // Keys past the request's last key and below its window are masked; the values of a
 // tile that reaches past the last key are cleared in shared memory first, because a

@@ -497,11 +497,11 @@ static double gt_plan(int M, int K, long long columns, int sms, int* best_bm, in
 // product that one call has for a decoded token another has for a prompt.  So they are taken where they are not slower for a few rows either: by
 // estimates of both for eight rows, not by more than an eighth (the multiply-adds': a part's chain, 42 ns a k; 2.9 TB/s and 4.5 us).  Not for k
 // below 1,024, where multiply-adds have short parts, nor for more than 32,768 columns, a vocabulary's head, of which a step wants a few rows.
-// Measured, us, multiply-adds and tensor cores (N x K), 8 rows: 4096 x 1024 10.9, 9.8; 6144 x 1024 14.8, 14.4; 1024 x 3072 14.0, 11.9; 4096 x 4096
-// 28, 26.7; 4096 x 12288 74, 66; 12288 x 2048 40.9, 44.2; 24576 x 4096 122, 133; 2560 x 4096 22.2, 25; refused: 2048 x 2048 11.5, 14.2;
-// 19456 x 2560 67.6, 88; 3072 x 512 5.1, 7.9; 8192 x 768 13.3, 14.8.
-// 99 rows: 4096 x 1024 39, 17.6; 6144 x 1024 57, 26; 1024 x 3072 29.7, 21.7; 12288 x 2048 195, 87; 24576 x 4096 733, 284; 300 rows:
-// 6144 x 1024 127, 46; 1024 x 2048 54, 25; 4096 x 12288 929, 395; (refused) 19456 x 2560 835, 355; 3072 x 512 37, 16.
+// Measured, us, W from memory, multiply-adds and tensor cores (N x K), 8 rows: 4096 x 1024 10.9, 10.0; 6144 x 1024 14.8, 14.7; 1024 x 3072 14.0,
+// 12.1; 4096 x 4096 28, 27.3; 4096 x 12288 74, 68; 12288 x 2048 40.9, 45.6; 24576 x 4096 122, 137; 2560 x 4096 22.2, 25.4; refused: 2048 x 2048
+// 11.5, 14.2; 19456 x 2560 67.6, 88; 3072 x 512 5.1, 7.9; 8192 x 768 13.3, 14.8.
+// 99 rows: 4096 x 1024 39, 17.7; 6144 x 1024 57, 26.2; 1024 x 3072 29.7, 21.3; 12288 x 2048 195, 90; 24576 x 4096 733, 284; 300 rows:
+// 6144 x 1024 127, 43; 1024 x 2048 54, 25; 4096 x 12288 929, 390; (refused) 19456 x 2560 835, 355; 3072 x 512 37, 16.
 extern "C" int vx_gemm_f32_takes_tc(int N, int K) {
     if (K < 1024 || N <= 0 || N > 32768) return 0;
     static int sms_cache[VX_MAX_DEVICES];

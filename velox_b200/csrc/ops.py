@@ -118,7 +118,6 @@ def _declare(lib) -> None:
         "vx_gated_act": [P, P, I, I, I, I, I, I, P],
         "vx_add_bias": [P, P, P, I, I, I, F, P],
         "vx_qk_norm_rope_kv": [P, I, P, P, F, P, I, P, P, P, P, I, I, I, I, I, I, I, P],
-        "vx_paged_attention_generic": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, P],
         "vx_biased_attention": [P, I, P, P, P, I, P, P, P, P, P, I, F, F, I, I, I, I, I, I, I, I, I, P, I, P, I, P],
         "vx_latent_attention": [P, P, P, I, P, P, P, P, F, I, I, I, I, I, I, I, P],
         "vx_biased_attention_cap": [P, I, P, P, P, I, P, P, P, P, P, I, F, F, I, I, I, I, I, I, I, I, I, P, I, P, I, F, P],
@@ -135,8 +134,6 @@ def _declare(lib) -> None:
         "vx_moe_combine": [P, P, P, P, P, I, I, I, I, I, P, I, P, I, P, P],
         "vx_moe_gather_rows": [P, I, P, I, P, I, I, P],
         "vx_moe_gemm_tcgen05": [P, P, P, I, I, I, I, I, I, I, I, P, P, I, P, P],
-        "vx_gemm_nt_simt": [P, P, P, P, I, I, I, I, I, I, I, I, P],
-        "vx_gemm_nt_simt_ready": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, I, P],
         "vx_gemm_tcgen05": [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_tcgen05_columns": [P, P, P, P, I, I, I, I, I, I, I, I, I, P, P],
         "vx_gemm_turned": [P, P, P, I, I, I, I, I, I, I, I, I, I, P, P],
@@ -151,10 +148,8 @@ def _declare(lib) -> None:
         "vx_paged_decode_attention_shape": [P, I, P, P, P, I, P, P, P, P, I, P, I, F, I, I, I, I, I, I, I, I, I, P],
         "vx_sample": [P, I, I, I, P, P, P, P, P],
         "vx_qk_norm_rope_kv_pairs": [P, I, P, P, F, P, I, P, P, P, P, I, I, I, I, I, I, I, I, P],
-        "vx_paged_attention_generic_cap": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, P],
         "vx_gemm_f32_takes_tc": [I, I],
         "vx_gemm_nt_simt_checked": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, I, P, P],
-        "vx_gemm_nt_simt_batched": [P, P, P, P, I, I, I, I, I, I, I, c_longlong, c_longlong, c_longlong, I, I, P],
         "vx_linear_attention_walk": [P, I, I, I, I, P, P, I, F, P, I, I, P, F, F, P, P, P, P, I, I, I, I, I, P],
         "vx_linear_attention_walk_parts": [P, I, I, I, I, P, P, I, F, P, I, I, P, F, F, P, P, P, P, I, I, I, I, I, I, P],
         "vx_stretch_log_decay": [P, I, F, P, P, I, I, P],
@@ -168,7 +163,6 @@ def _declare(lib) -> None:
         "vx_sum_add_rmsnorm": [P, P, F, P, F, P, F, P, P, P, P, I, I, F, I, P],
         "vx_softcap_rows": [P, P, c_longlong, F, P],
         "vx_qk_norm_rope_kv_shared": [P, I, P, P, F, P, I, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P],
-        "vx_paged_attention_generic_shared": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, I, I, P],
         "vx_latent_attention_window": [P, P, P, I, P, P, P, P, F, I, I, I, I, I, I, I, I, P],
         "vx_stream_norm": [P, I, P, P, P, P, F, P, I, P, I, I, I, I, P],
         "vx_stream_update": [P, I, P, P, F, P, P, I, P, P, F, P, I, I, I, I, P],
@@ -185,7 +179,6 @@ def _declare(lib) -> None:
         "vx_linear_attention_walk_bonus": [P, I, I, I, I, P, P, I, F, P, I, I, P, F, F, P, P, P, P, I, I, I, I, I, P, I, I, P],
         "vx_stretch_log_decay_form": [P, I, F, P, P, I, I, I, P],
         "vx_head_norm_gate_heads": [P, P, I, P, I, P, I, I, I, F, I, I, I, P],
-        "vx_paged_attention_generic_chunk": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, I, I, I, P],
         "vx_paged_attention_generic_requests": [P, I, P, P, P, I, P, P, P, I, F, I, I, I, I, I, I, I, I, I, F, P, I, F, I, I, I, I, I, P],
         "vx_biased_attention_chunk": [P, I, P, P, P, I, P, P, P, P, P, I, F, F, I, I, I, I, I, I, I, I, I, P, I, P, I, F, I, I, I, P],
         "vx_gemm_skinny_act": [P, P, P, P, I, I, I, I, I, I, I, I, I, I, P],
@@ -1941,10 +1934,11 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, bias=None, out_dtype: Optional[t
               w_ready: bool = False) -> torch.Tensor:
     """a [M,K] times w [N,K] transposed on the tensor cores, float32 accumulation.  `w_ready`: see `gemm_nt_simt`; only then is
     the turned product taken where it is the fastest (part of what it gains are weights on their way before the wait)."""
-    if w_ready and bias is None and SKINNY_MAX_ROWS < a.shape[0] <= TURNED_MAX_ROWS and a.is_cuda and turned_wins(a.shape[0], w.shape[0], a.shape[1], False) and tcgen05_supported(a, w):
+    rows = a.shape[0]
+    if w_ready and bias is None and SKINNY_MAX_ROWS < rows <= TURNED_MAX_ROWS and a.is_cuda and turned_wins(rows, w.shape[0], a.shape[1], False) and tcgen05_supported(a, w):
         return gemm_turned(a, w, out_dtype, w_ready=True)
     if bias is None and _MATMUL_SET and a.is_cuda:
-        few = a.shape[0] <= SKINNY_MAX_ROWS
+        few = rows <= SKINNY_MAX_ROWS
         out = (_CALLS or _calls()).gemm_bf16(a, w, out_dtype or torch.bfloat16)
         if out is not None:
             return _called(out, "gemm_skinny") if few and skinny_supported(a.shape[0], a.shape[1], a, w) else out

@@ -56,7 +56,8 @@ __device__ __forceinline__ unsigned tc_desc_lo(unsigned addr) { return ((addr >>
 // One lane of the warp, the same every time.  A role that one thread has (loads, products) is run by its whole warp, and the
 // elected lane issues: its operands then stay in the warp's uniform registers.  Under `if (lane == 0)` every operand of every
 // instruction is moved there first: gated products with short tiles took up to 1.3 times as long (777 x 6144 x 1024 on tiles of 160
-// columns 21.2 us, 18.9 so; 2048 x 19456 x 2560 by pairs 154, 141; 2048 x 24576 x 4096 by pairs 288, 273).
+// columns 21.1 us, 19.3 so; 2048 x 19456 x 2560 by pairs 155, 146; 2048 x 24576 x 4096 by pairs 294, 277; the votes of tc_warp_wait among that,
+// 1 to 3 %).
 __device__ __forceinline__ bool tc_elect() {
     unsigned p;
     asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));

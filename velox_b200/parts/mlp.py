@@ -58,16 +58,17 @@ class GatedMLP(FeedForward):
     def forward(self, h: torch.Tensor, ctx=None) -> torch.Tensor:
         w = self.gate_up.weight
         fused = self.tile and h.dtype == torch.bfloat16
-        if fused and ops.skinny_supported(h.shape[0], h.shape[1], h, w):
+        rows = h.shape[0]
+        if fused and ops.skinny_supported(rows, h.shape[1], h, w):
             # a decode step: W streamed once, act(gate) * up taken on the accumulators
             a = ops.gemm_skinny(h, w, None, h.dtype, gated_activation=self.activation)
-        elif fused and h.shape[0] <= ops.TURNED_GATED_MAX_ROWS and ops.turned_wins(h.shape[0], w.shape[0], h.shape[1], True) and ops.tcgen05_supported(h, w):
+        elif fused and rows <= ops.TURNED_GATED_MAX_ROWS and ops.turned_wins(rows, w.shape[0], h.shape[1], True) and ops.tcgen05_supported(h, w):
             # a wider decode step, a mixed step, a shorter prompt portion: the same epilogue on the turned product
             a = ops.gemm_turned(h, w, h.dtype, gated_activation=self.activation, w_ready=True)
-        elif fused and h.shape[0] >= FUSED_TCGEN05_MIN_ROWS and ops.tcgen05_supported(h, w):
+        elif fused and rows >= FUSED_TCGEN05_MIN_ROWS and ops.tcgen05_supported(h, w):
             # a prompt portion: tcgen05 product with the same epilogue (measured no slower than
             # the library product followed by the activation kernel from 128 rows, faster from 512)
-            pair, columns = ops.tcgen05_tile(h.shape[0], w.shape[0], h.shape[1], h.device)
+            pair, columns = ops.tcgen05_tile(rows, w.shape[0], h.shape[1], h.device)
             a = ops.gemm_tcgen05(h, w, None, gated_activation=self.activation, pair=pair, columns=columns)
         elif h.dtype == torch.bfloat16:
             # the library product hands over its float32 sums: gate and up are not rounded
