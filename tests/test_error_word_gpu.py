@@ -156,3 +156,40 @@ def test_a_captured_step_is_checked_at_its_end_of_waits():
             assert o._END_OF_WAITS[1] is g.end_of_waits.event
         e.runner.check_errors()
         assert not e.runner.pending_error_check
+
+
+def test_a_captured_step_without_bounded_waits_records_no_end():
+    from velox_b200.engine import StepEntry
+    o, e = ops(), engine("bfloat16", vocab=32784)
+    for i in range(2):
+        e.cache.add_request(i)
+    for _ in range(3):
+        e.runner.step([StepEntry(i, [3 + i], [0]) for i in range(2)])
+        assert not e.runner.pending_error_check
+    g = next(iter(e.runner.graphs.graphs.values()))
+    assert g.graph is not None and g.bounded_wait_launches == 0 and g.end_of_waits.launches == -1
+
+
+def test_a_step_that_the_caller_captures_notes_no_end_of_waits():
+    """Checks afterwards wait for the stream, as they do for any
+    kernel with bounded waits behind which no end was noted."""
+    from velox_b200.engine import StepEntry
+    from velox_b200.engine.batch import build_step_context
+    o, e = ops(), engine("bfloat16", vocab=32784)
+    for i in range(12):
+        e.cache.add_request(i)
+    entries = [StepEntry(i, [3 + i], [0]) for i in range(12)]
+    for i in range(12):
+        e.cache.reserve(i, 1)
+    ctx = build_step_context(entries, e.cache, e.device, 32784, e.runner.short_max)
+    e.runner.run(ctx)
+    e.runner.check_errors()
+    noted = o._END_OF_WAITS
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        e.runner.run(ctx)
+    assert o._END_OF_WAITS is noted and e.runner.pending_error_check
+    graph.replay()
+    set_word()
+    with pytest.raises(o.KernelError, match="gave up a wait"):
+        e.runner.check_errors()

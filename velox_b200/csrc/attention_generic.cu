@@ -236,7 +236,8 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, PARTS == 0 ? 9 : (PARTS <= 4 ?
 // into shared memory once for all of them: four chunks a round, sixteen warps: warp w works on chunk 4 round + w mod 4 for every fourth
 // query (token and head) of the block, from w / 4 on.  The next round's keys come while this one's values are used, and the other way round.
 // A token's chunks go to the same four running sums in the same order, and are merged alike, whatever tokens are in its block.
-// What bounds it: a round's chain (loads, products, sums over eight lanes, softmax, values; about 5 us a round).  16 heads of 128, 8 kv heads, us, a
+// What bounds it: a round's chain (loads, products, sums over eight lanes, softmax, values; about 5 us a round; with four queries a warp
+// it spills 148 bytes at its 128 registers).  16 heads of 128, 8 kv heads, us, a
 // block per token and head and this: 96 prompt tokens beside 3 on 200 to 400 keys 54, 23; 96 prompt tokens alone 26, 16; one token on 400 keys 42,
 // 22; four on 800 79, 39; 150 prompt tokens 52, 35.
 #define ATS_TOKENS 8

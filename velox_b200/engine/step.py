@@ -134,10 +134,12 @@ class ModelRunner:
 
     def run(self, ctx: StepContext, end_of_waits=None) -> Optional[torch.Tensor]:
         """`end_of_waits`: a captured step's own (`ops.EndOfWaits`)."""
+        before = ops.bounded_wait_launches()
         residual, delta = self.model.forward_hidden(ctx, self.cache)
         if end_of_waits is not None:
-            end_of_waits.record()
-        elif ops.bounded_wait_pending():
+            if ops.bounded_wait_launches() != before:   # (a step without any is not cut in two: 3 us a replay)
+                end_of_waits.record()
+        elif ops.bounded_wait_pending() and not torch.cuda.is_current_stream_capturing():   # (a capture of the caller's records no place in time)
             self.end_of_waits.record()
             ops.note_end_of_waits(self.end_of_waits)
         if ctx.wanted_rows.numel() == 0:
